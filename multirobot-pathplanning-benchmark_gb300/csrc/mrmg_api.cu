@@ -307,28 +307,38 @@ void box_tables(const ArmSrc& a, std::vector<int> boxes, ArmTables* t) {
 }
 
 // penetration-cost tables: the set's spheres in slot order (robot, then
-// frame), tasks of two consecutive spheres of one robot, boxes in the given order
+// frame; an even number per robot), tasks of two consecutive spheres of one
+// robot, boxes in the given order
 void pen_tables(const ArmSrc& a, int R, const std::vector<char>& on, const std::vector<int>& boxes, ArmTables* t) {
   PenDev& pd = t->pd;
-  int cnt[kMaxRobots][kMaxLinks + 1] = {};
   t->pen_sph.clear();
   t->pen_task.clear();
-  for (int sl = 0; sl < a.G * a.SPG; sl++) {
-    const int i = a.slot_sphere[sl];
-    if (i < 0 || !on[i]) continue;
-    const int r = a.grp[sl / a.SPG] & 0xff, k = a.grp[sl / a.SPG] >> 8;
-    cnt[r][k]++;
-    t->pen_sph.push_back(make_float4((float)a.local[3 * i], (float)a.local[3 * i + 1], (float)a.local[3 * i + 2],
-                                     (float)a.radius[i]));
-  }
-  int acc = 0;
+  int real = 0;
   for (int r = 0; r < kMaxRobots; r++) {
-    for (int k = 0; k <= kMaxLinks; k++) { pd.lk[r][k] = acc; acc += cnt[r][k]; }
+    // this robot's spheres; an odd count is made even by a sphere of radius
+    // -1e30 at the last one's place, which adds nothing to any pair
+    const int s0 = (int)t->pen_sph.size();
+    int cnt[kMaxLinks + 1] = {}, last = -1;
+    for (int sl = 0; r < R && sl < a.G * a.SPG; sl++) {
+      const int i = a.slot_sphere[sl];
+      if (i < 0 || !on[i] || (a.grp[sl / a.SPG] & 0xff) != r) continue;
+      last = a.grp[sl / a.SPG] >> 8;
+      cnt[last]++;
+      t->pen_sph.push_back(make_float4((float)a.local[3 * i], (float)a.local[3 * i + 1], (float)a.local[3 * i + 2],
+                                       (float)a.radius[i]));
+    }
+    real += (int)t->pen_sph.size() - s0;
+    if ((t->pen_sph.size() - s0) & 1) {
+      float4 none = t->pen_sph.back();
+      none.w = -1e30f;
+      t->pen_sph.push_back(none);
+      cnt[last]++;
+    }
+    const int s1 = (int)t->pen_sph.size();
+    int acc = s0;
+    for (int k = 0; k <= kMaxLinks; k++) { pd.lk[r][k] = acc; acc += cnt[k]; }
     pd.lk[r][kMaxLinks + 1] = acc;
-  }
-  for (int r = 0; r < R; r++) {
-    const int s0 = pd.lk[r][0], s1 = pd.lk[r][kMaxLinks + 1];
-    for (int i = s0; i < s1; i += 2) t->pen_task.push_back(make_int4(i, i + 1 < s1 ? i + 1 : -1, s0, s1));
+    for (int i = s0; i < s1; i += 2) t->pen_task.push_back(make_int4(i, i + 1, s0, s1));
   }
   t->pen_box.assign(2 * boxes.size(), make_float4(0.f, 0.f, 0.f, 0.f));
   for (size_t j = 0; j < boxes.size(); j++) {
@@ -339,7 +349,15 @@ void pen_tables(const ArmSrc& a, int R, const std::vector<char>& on, const std::
     t->pen_box[2 * j + 1] = make_float4((float)(0.5 * (hi[0] - lo[0])), (float)(0.5 * (hi[1] - lo[1])),
                                         (float)(0.5 * (hi[2] - lo[2])), 0.f);
   }
+  float r_max = 0.f, deep = 0.f;
+  for (const float4& c : t->pen_sph) r_max = std::max(r_max, c.w);
+  for (size_t j = 0; j < boxes.size(); j++) {
+    const float4 h = t->pen_box[2 * j + 1];
+    deep = std::max(deep, std::min(h.x, std::min(h.y, h.z)));
+  }
+  pd.reach = r_max + std::max(r_max, deep);
   pd.S = (int)t->pen_sph.size();
+  pd.real = real;
   pd.B = (int)boxes.size();
   pd.NTK = (int)t->pen_task.size();
 }
@@ -1580,13 +1598,14 @@ int mrmg_path_penetration(mrmg_scene* sc, const float* d_paths, int64_t P, int32
   if (!std::isfinite(margin) || !(scale > 0.0) || !std::isfinite(scale) || !(beta > 0.0) || !std::isfinite(beta) ||
       !(smooth >= 0.0) || !std::isfinite(smooth))
     return fail(MRMG_ERR_ARG, "params: finite margin, scale > 0, beta > 0, smooth weight >= 0");
-  const long long nseg = (T + 31) / 32;
-  if (P * nseg >= (1ll << 31)) return fail(MRMG_ERR_ARG, "too many path segments for one call");
+  const long long nseg = pen_segments(T, kPenMinSeg);   // at most; sizes the scratch
+  if (P * ((T + 31ll) / 32) >= (1ll << 31)) return fail(MRMG_ERR_ARG, "too many path segments for one call");
   int warps = warps_per_cta > 0 ? warps_per_cta : 16;
   if (warps < sc->arm.R) warps = sc->arm.R;
   if (warps > 16) return fail(MRMG_ERR_UNSUPPORTED, "warps per CTA must be <= 16 (and >= robots)");
-  int smem_max = 0;
+  int smem_max = 0, smem_sm = 0;
   cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, sc->device);
+  cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, sc->device);
   const size_t smem = pen_smem_bytes(sc->arm, sc->pen, 0, warps, 0, sc->arm.R);
   if (smem > (size_t)smem_max)
     return fail(MRMG_ERR_UNSUPPORTED, "scene too large for the penetration kernel (%zu B shared memory > %d)", smem,
@@ -1622,7 +1641,7 @@ int mrmg_path_penetration(mrmg_scene* sc, const float* d_paths, int64_t P, int32
   pp.inv_beta = (float)(1.0 / beta);
   pp.smooth_w = (float)smooth;
   cudaError_t e = pen_launch(sc->arm, sc->pen, pp, d_paths, P, T, d_grad_cost, sc->d_pen_seg, d_cost, d_wp_cost,
-                             d_grad, warps, n_groups, bounds, st);
+                             d_grad, warps, n_groups, bounds, sc->num_sms, (size_t)smem_sm, st);
   if (e != cudaSuccess) return cuda_fail(e, "launch penetration cost");
   if (flags & MRMG_FLAG_ASYNC) return MRMG_OK;
   e = cudaStreamSynchronize(st);
@@ -1632,7 +1651,7 @@ int mrmg_path_penetration(mrmg_scene* sc, const float* d_paths, int64_t P, int32
 
 int mrmg_penetration_info(const mrmg_scene* sc, int64_t* out4) {
   if (!sc || sc->kind != 1 || !out4) return fail(MRMG_ERR_ARG, "arm scene and out4 required");
-  out4[0] = sc->pen.S;
+  out4[0] = sc->pen.real;
   out4[1] = sc->pen.B;
   out4[2] = (int64_t)pen_smem_bytes(sc->arm, sc->pen, 0, 16, 0, sc->arm.R);
   out4[3] = (int64_t)pen_smem_bytes(sc->arm, sc->pen, 1, 16, 0, sc->arm.R);

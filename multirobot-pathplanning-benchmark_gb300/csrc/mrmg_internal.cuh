@@ -108,15 +108,16 @@ __host__ __device__ inline void arm_table_layout(const ArmDev& s, size_t off[9])
 }
 
 // ---------------------------------------------------------------------------
-// Path-penetration cost tables of an arm scene: the real spheres (padding
-// dropped) grouped by robot, then by frame, so the spheres of other robots
+// Path-penetration cost tables of an arm scene: the real spheres (empty slots
+// dropped, each robot's count made even) grouped by robot, then by frame, so the spheres of other robots
 // are [0, first of robot) and [first of next robot, S); boxes in input order.
 // ---------------------------------------------------------------------------
 struct PenDev {
-  int S, B, NTK;
+  int S, B, NTK;         // spheres (with the padding), boxes, tasks
+  int real;              // spheres without the padding
+  float reach;           // largest -d of any pair: two radii, or a radius and half a box's smallest extent
   const float4* sph;     // [S]  local xyz, radius
-  const int4* task;      // [NTK] sphere, second sphere of the same robot (-1: none),
-                         //       the robot's first sphere, the next robot's first sphere
+  const int4* task;      // [NTK] first sphere, second sphere, the robot's first sphere, the next robot's first
   const float4* box;     // [2B] centre xyz, half extents xyz
   int lk[kMaxRobots][kMaxLinks + 2];   // spheres of (robot r, frame k): [lk[r][k], lk[r][k+1])
 };
@@ -274,6 +275,10 @@ int arm_prepare(const ArmDev& s, int warps);
 int arm_supported_spg(int idx);   // list of compiled SPG values, -1 at end
 int arm_gpl_for_spg(int spg);
 
+// penetration kernels: waypoints per CTA (32, or 16 for the gradient), and the
+// most warps of a 16-waypoint gradient CTA
+constexpr int kPenMinSeg = 16, kPenGradWarps = 12;
+__host__ __device__ inline int pen_segments(int T, int seg) { return (int)(((long long)T + seg - 1) / seg); }
 // shared memory of a penetration launch whose gradient covers robots [gr0, gr1)
 size_t pen_smem_bytes(const ArmDev& a, const PenDev& pd, int grad, int warps, int gr0, int gr1);
 // splits the robots into the fewest groups of consecutive robots whose
@@ -282,7 +287,7 @@ size_t pen_smem_bytes(const ArmDev& a, const PenDev& pd, int grad, int warps, in
 int pen_grad_groups(const ArmDev& a, const PenDev& pd, int warps, size_t smem_max, int* bounds);
 cudaError_t pen_launch(const ArmDev& a, const PenDev& pd, const PenParams& pp, const float* paths, long long P, int T,
                        const float* gout, double* seg, double* cost, float* wp_cost, float* grad, int warps,
-                       int n_groups, const int* bounds, cudaStream_t st);
+                       int n_groups, const int* bounds, int num_sms, size_t smem_sm, cudaStream_t st);
 
 cudaError_t binary_indices(long long N, long long* out, cudaStream_t st, int chunked);
 

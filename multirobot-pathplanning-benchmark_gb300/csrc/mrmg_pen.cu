@@ -12,10 +12,11 @@
 // radius) and every pair of spheres on different robots (d = centre distance
 // minus both radii).  With beta = 1 this is softplus(margin - d) / scale.
 //
-// One CTA per segment of 32 consecutive waypoints of one path, one waypoint per
-// lane: forward kinematics runs per segment (warp r walks robot r's chain for
-// its 32 waypoints) and is recomputed, not stored, when the gradient is asked
-// for.  The gradient of a joint angle theta_k follows the geometric Jacobian:
+// One CTA per segment of 32 (cost) or 16 (gradient, where two CTAs then fit an
+// SM) consecutive waypoints of one path, one waypoint per lane or per pair of
+// half-warp lanes: forward kinematics runs per segment (a warp or half warp
+// walks one robot's chain for its waypoints) and is recomputed, not stored, when
+// the gradient is asked for.  Few segments: a cluster of CTAs shares each.  The gradient of a joint angle theta_k follows the geometric Jacobian:
 // with o, z the origin and z axis of frame k-1 and g_s = dcost/dc_s,
 //   dcost/dtheta_k = z . sum_{s beyond joint k} (c_s - o) x g_s
 //                  = z . (M - o x G),  M = sum c_s x g_s,  G = sum g_s,
@@ -30,7 +31,8 @@
 namespace mrmg {
 namespace {
 
-constexpr int kSeg = 32;   // waypoints per CTA
+constexpr int kMaxSplit = 8;              // CTAs that share a segment, at most (a portable cluster)
+constexpr double kFixedShare = 0.1;       // a CTA's fixed work over a whole segment's pair work
 
 __host__ __device__ inline size_t al4(size_t n) { return (n + 3) & ~(size_t)3; }
 
@@ -38,25 +40,53 @@ __host__ __device__ inline size_t al4(size_t n) { return (n + 3) & ~(size_t)3; }
 // The gradient regions cover the Sg spheres and Rg robots whose gradients
 // the launch computes (all of them, or one group of robots of a scene too
 // large for one CTA's shared memory).
+template <int SEG>
 struct PenLayout {
-  size_t C, G, OZ, W, QG, sph, box, task, br, part, total;
+  size_t C, G, OZ, W, QG, sph, box, br, part, total;
   __host__ __device__ PenLayout(int S, int B, int D, bool grad, int warps, int Sg, int Rg) {
     size_t o = 0;
-    C = o;   o += (size_t)S * 3 * kSeg;                          // sphere centres [S*3][32]
-    G = o;   o += grad ? (size_t)Sg * 3 * kSeg : 0;              // dcost/dcentre  [Sg*3][32]
-    OZ = o;  o += grad ? (size_t)Rg * kMaxLinks * 6 * kSeg : 0;  // frame origin, z axis [Rg][L][6][32]
-    W = o;   o += al4((size_t)(kSeg + 2) * D);                   // waypoints t0-1 .. t0+32
-    QG = o;  o += grad ? al4((size_t)kSeg * D) : 0;              // obstacle gradient [32][D]
+    C = o;   o += (size_t)S * 3 * SEG;                          // sphere centres [S/2][3][SEG][2]
+    G = o;   o += grad ? (size_t)Sg * 3 * SEG : 0;              // dcost/dcentre  [Sg*3][SEG]
+    OZ = o;  o += grad ? (size_t)Rg * kMaxLinks * 6 * SEG : 0;  // frame origin, z axis [Rg][L][6][SEG]
+    W = o;   o += al4((size_t)(SEG + 2) * D);                   // waypoints t0-1 .. t0+SEG
+    QG = o;  o += grad ? al4((size_t)SEG * D) : 0;              // obstacle gradient [SEG][D]
     sph = o; o += (size_t)S * 4;
-    box = o; o += (size_t)B * 8;
-    task = o; o += (size_t)S * 4;                               // at most S tasks (int4)
+    box = o; o += (size_t)((B + 1) / 2) * 12;                    // pairs of boxes [(B+1)/2][6][2]
     br = o;  o += al4((size_t)S);                               // beta log2(e) radius
-    part = o; o += (size_t)warps * kSeg * 2;
+    part = o; o += (size_t)warps * 64;
     total = o;
   }
 };
 
+// place of coordinate i of sphere s, waypoint `wl`, among the centres:
+// spheres 2j and 2j + 1 side by side, read as one packed pair
+template <int SEG>
+__device__ __forceinline__ int cen(int s, int i, int wl) { return (((s >> 1) * 3 + i) * SEG + wl) * 2 + (s & 1); }
+
 __host__ __device__ inline int pen_first_sphere(const PenDev& pd, int R, int r) { return r < R ? pd.lk[r][0] : pd.S; }
+
+// the CTAs of a cluster: size, this CTA's rank, barrier, and loads from the
+// same shared-memory place of CTA `rank`
+__device__ __forceinline__ int cluster_size() { int v; asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(v)); return v; }
+__device__ __forceinline__ int cluster_rank() { int v; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(v)); return v; }
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float cluster_ld(const float* p, int rank) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ double cluster_ld64(const double* p, int rank) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(cluster_addr(p, rank)) : "memory");
+  return v;
+}
 
 // MUFU approximations (PTX): 2^x, log2, sqrt, 1/sqrt, 1/x
 __device__ __forceinline__ float ex2a(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
@@ -70,88 +100,198 @@ __device__ __forceinline__ float rcpa(float x) { float y; asm("rcp.approx.ftz.f3
 // and sigmoid(beta (margin - d)) = 1 / (1 + e) for x2 >= 0, e / (1 + e) else.
 // K folds the constant part: x2 = K - beta log2(e) * (distance).
 //
-// A task's two spheres are evaluated together in packed FP32x2 arithmetic
-// (.x = first sphere, .y = second): one add / multiply / FMA instruction does
-// both; min/max, abs and the special functions stay per component.
+// One sphere is evaluated against two partners (boxes or spheres, .x and .y) in
+// packed FP32x2 arithmetic: one add / multiply / FMA instruction does both, and
+// the partners' data are read as pairs (broadcasting a scalar into a packed
+// operand would cost moves); min/max, abs and the special functions stay per
+// component.
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
 
-struct PairAcc2 {
-  float2 ps;           // sums of max(x2, 0) + log2(1 + e)
-  float2 gx, gy, gz;   // dcost / dcentre
+// one sphere of a task: minus its centre, the constant of x2 and its sums
+struct Side {
+  float2 nx, ny, nz;   // minus the centre, broadcast
+  float2 K;            // beta log2(e) (margin + radius), broadcast
+  float2 ps;           // sums of log2(1 + 2^x2) (without DIRECT: of max(x2, 0) + log2(1 + e))
+  float2 pr;           // product of the 1 + e not yet in ps, less 1
+  float2 gx, gy, gz;   // scale * dcost / dcentre
 };
 
-// softplus (base 2) of x2 into ps; sigmoid-based dterm/d(distance) into w
-template <bool COST, bool GRAD>
-__device__ __forceinline__ void term2(float2 x2, float inv_scale, float2& ps, float2& w) {
-  const float2 e = make_float2(ex2a(-fabsf(x2.x)), ex2a(-fabsf(x2.y)));
-  const float2 ope = add2(e, bc2(1.f));
-  if (COST)
-    ps = add2(ps, add2(make_float2(fmaxf(x2.x, 0.f), fmaxf(x2.y, 0.f)), make_float2(lg2a(ope.x), lg2a(ope.y))));
+// Floor of the squared distances whose reciprocal root is taken: added to the
+// last product of the sum, it leaves every square above 1e-22 m^2 unchanged.
+constexpr float kTiny2 = 1e-30f;
+// x2 of a partner that is not there: e = 0
+constexpr float kNone = -1e30f;
+
+// Pairs whose 1 + e are multiplied before one log2 is taken of the product:
+// log2 is an eighth of an FMA on this part (measured 16 against 128 per clock
+// and SM) and the sum of log2(1 + e) is the log2 of the product.  The product is
+// kept less 1, so pairs far apart (e below half an ulp of 1) still count.  With
+// DIRECT every factor is at most 1 + 2^kDirectMax, so kProd of them stay below
+// 2^113; without, at most 2.
+constexpr int kProd = 16;
+constexpr float kDirectMax = 7.f;
+
+// softplus (base 2) of x2 into the product; e and 1 + e for the sigmoid.
+// DIRECT (every x2 of the scene is at most kDirectMax): e = 2^x2, no |x2|, no max.
+template <bool COST, bool DIRECT>
+__device__ __forceinline__ void soft2(Side& a, float2 x2, float2* e, float2* ope) {
+  *e = DIRECT ? make_float2(ex2a(x2.x), ex2a(x2.y)) : make_float2(ex2a(-fabsf(x2.x)), ex2a(-fabsf(x2.y)));
+  *ope = add2(*e, bc2(1.f));
+  if (COST) {
+    a.pr = fma2(a.pr, *ope, *e);   // (1 + p)(1 + e) - 1
+    if (!DIRECT) a.ps = add2(a.ps, make_float2(fmaxf(x2.x, 0.f), fmaxf(x2.y, 0.f)));
+  }
+}
+
+// sigmoids of the four pairs of a step from two reciprocals:
+// 1/a = b * (1 / (a b)), 1/b = a * (1 / (a b))
+template <bool DIRECT>
+__device__ __forceinline__ void sigmoid4(float2 x0, float2 e0, float2 o0, float2 x1, float2 e1, float2 o1, float2* w0,
+                                         float2* w1) {
+  const float2 m = mul2(o0, o1);
+  const float2 r = make_float2(rcpa(m.x), rcpa(m.y));
+  const float2 i0 = mul2(r, o1), i1 = mul2(r, o0);
+  *w0 = mul2(e0, i0);
+  *w1 = mul2(e1, i1);
+  if (!DIRECT) {
+    *w0 = make_float2(x0.x >= 0.f ? i0.x : w0->x, x0.y >= 0.f ? i0.y : w0->y);
+    *w1 = make_float2(x1.x >= 0.f ? i1.x : w1->x, x1.y >= 0.f ? i1.y : w1->y);
+  }
+}
+
+// log2(1 + p): the series of the logarithm below 1/64 (its first left-out term
+// is p^4 / 5 < 1.2e-8 of the value)
+template <bool COST>
+__device__ __forceinline__ void flush_product(Side& a) {
+  if (COST) {
+    const float2 p = a.pr;
+    const float2 t = fma2(fma2(fma2(p, bc2(-0.25f), bc2(0.33333333f)), p, bc2(-0.5f)), p, bc2(1.f));
+    const float2 s = mul2(mul2(p, bc2(1.44269504f)), t);
+    const float2 l = make_float2(lg2a(1.f + p.x), lg2a(1.f + p.y));
+    a.ps = add2(a.ps, make_float2(p.x < 0.015625f ? s.x : l.x, p.y < 0.015625f ? s.y : l.y));
+    a.pr = bc2(0.f);
+  }
+}
+
+// a sphere whose centre lies inside a box (every max(|d| - h, 0) zero): its
+// signed distance max_k(|d_k| - h_k), and the unit vector along that axis
+__device__ __forceinline__ float inside_box(float dx, float dy, float dz, float hx, float hy, float hz, float* gx,
+                                            float* gy, float* gz) {
+  const float ax = fabsf(dx) - hx, ay = fabsf(dy) - hy, az = fabsf(dz) - hz;
+  const bool bx = ax >= ay && ax >= az, by = !bx && ay >= az;
+  *gx = bx ? copysignf(1.f, dx) : 0.f;
+  *gy = by ? copysignf(1.f, dy) : 0.f;
+  *gz = (!bx && !by) ? copysignf(1.f, dz) : 0.f;
+  return fmaxf(ax, fmaxf(ay, az));
+}
+
+__device__ __forceinline__ float2 beyond2(float2 d, float2 h) {   // max(|d| - h, 0)
+  return make_float2(fmaxf(fabsf(d.x) - h.x, 0.f), fmaxf(fabsf(d.y) - h.y, 0.f));
+}
+__device__ __forceinline__ float2 sign2(float2 m, float2 d) { return make_float2(copysignf(m.x, d.x), copysignf(m.y, d.y)); }
+
+template <bool V>
+struct Flag { static constexpr bool value = V; };
+
+// two boxes: centres and half extents
+struct Box2 {
+  float2 cx, cy, cz, hx, hy, hz;
+};
+
+// x2 of a sphere against two boxes; with GRAD also u, inv: the gradient of the
+// distance is -u * inv (the vector from the centre to the box over its length)
+template <bool GRAD>
+__device__ __forceinline__ float2 box_x2(const Side& a, const Box2& b, float2 nbl, float2 K, float2* ux, float2* uy,
+                                         float2* uz, float2* inv) {
+  const float2 dx = add2(b.cx, a.nx), dy = add2(b.cy, a.ny), dz = add2(b.cz, a.nz);
+  *ux = beyond2(dx, b.hx);
+  *uy = beyond2(dy, b.hy);
+  *uz = beyond2(dz, b.hz);
+  float2 sdf;
+  if (!GRAD) {
+    const float2 u2 = fma2(*ux, *ux, fma2(*uy, *uy, mul2(*uz, *uz)));
+    sdf = make_float2(sqrta(u2.x), sqrta(u2.y));
+    if (__builtin_expect(fminf(u2.x, u2.y) == 0.f, 0)) {   // a centre inside a box (seldom): the negative part
+      float gx, gy, gz;
+      if (u2.x == 0.f) sdf.x = fminf(inside_box(dx.x, dy.x, dz.x, b.hx.x, b.hy.x, b.hz.x, &gx, &gy, &gz), 0.f);
+      if (u2.y == 0.f) sdf.y = fminf(inside_box(dx.y, dy.y, dz.y, b.hx.y, b.hy.y, b.hz.y, &gx, &gy, &gz), 0.f);
+    }
+  } else {
+    const float2 u2 = fma2(*ux, *ux, fma2(*uy, *uy, fma2(*uz, *uz, bc2(kTiny2))));
+    *inv = make_float2(rsqa(u2.x), rsqa(u2.y));
+    sdf = mul2(u2, *inv);
+    *ux = sign2(*ux, dx);
+    *uy = sign2(*uy, dy);
+    *uz = sign2(*uz, dz);
+    if (__builtin_expect(fminf(u2.x, u2.y) <= kTiny2, 0)) {   // a centre inside a box (seldom)
+      if (u2.x <= kTiny2) {
+        sdf.x = inside_box(dx.x, dy.x, dz.x, b.hx.x, b.hy.x, b.hz.x, &ux->x, &uy->x, &uz->x);
+        inv->x = 1.f;
+      }
+      if (u2.y <= kTiny2) {
+        sdf.y = inside_box(dx.y, dy.y, dz.y, b.hx.y, b.hy.y, b.hz.y, &ux->y, &uy->y, &uz->y);
+        inv->y = 1.f;
+      }
+    }
+  }
+  return fma2(nbl, sdf, K);
+}
+
+// x2 of a sphere against two spheres (centres x, y, z); v: from the centre to theirs
+template <bool GRAD>
+__device__ __forceinline__ float2 sphere_x2(const Side& a, float2 x, float2 y, float2 z, float2 nbl, float2 K, float2* vx,
+                                            float2* vy, float2* vz, float2* inv) {
+  *vx = add2(x, a.nx);
+  *vy = add2(y, a.ny);
+  *vz = add2(z, a.nz);
+  if (!GRAD) {
+    const float2 d2 = fma2(*vx, *vx, fma2(*vy, *vy, mul2(*vz, *vz)));
+    return fma2(nbl, make_float2(sqrta(d2.x), sqrta(d2.y)), K);
+  }
+  const float2 d2 = fma2(*vx, *vx, fma2(*vy, *vy, fma2(*vz, *vz, bc2(kTiny2))));
+  *inv = make_float2(rsqa(d2.x), rsqa(d2.y));
+  return fma2(nbl, mul2(d2, *inv), K);
+}
+
+__device__ __forceinline__ void pull(Side& a, float2 w, float2 inv, float2 ux, float2 uy, float2 uz) {
+  const float2 f = mul2(w, inv);
+  a.gx = fma2(f, ux, a.gx);
+  a.gy = fma2(f, uy, a.gy);
+  a.gz = fma2(f, uz, a.gz);
+}
+
+// both spheres of a task against two boxes
+template <bool COST, bool GRAD, bool DIRECT>
+__device__ __forceinline__ void box_step(Side& a, Side& b, const Box2& bx, float2 nbl, float2 Ka, float2 Kb) {
+  float2 ax, ay, az, ai, cx, cy, cz, ci, ea, oa, ec, oc;
+  const float2 xa = box_x2<GRAD>(a, bx, nbl, Ka, &ax, &ay, &az, &ai);
+  const float2 xc = box_x2<GRAD>(b, bx, nbl, Kb, &cx, &cy, &cz, &ci);
+  soft2<COST, DIRECT>(a, xa, &ea, &oa);
+  soft2<COST, DIRECT>(b, xc, &ec, &oc);
   if (GRAD) {
-    const float2 r = make_float2(rcpa(ope.x), rcpa(ope.y));
-    const float2 er = mul2(e, r);
-    w = mul2(make_float2(x2.x >= 0.f ? r.x : er.x, x2.y >= 0.f ? r.y : er.y), bc2(-inv_scale));
+    float2 wa, wc;
+    sigmoid4<DIRECT>(xa, ea, oa, xc, ec, oc, &wa, &wc);
+    pull(a, wa, ai, ax, ay, az);
+    pull(b, wc, ci, cx, cy, cz);
   }
 }
 
-template <bool COST, bool GRAD>
-__device__ __forceinline__ void box_pair2(float2 cx, float2 cy, float2 cz, const float4& bc, const float4& bh,
-                                          float2 nbl, float2 K, float inv_scale, PairAcc2& acc) {
-  const float2 dx = add2(cx, bc2(-bc.x)), dy = add2(cy, bc2(-bc.y)), dz = add2(cz, bc2(-bc.z));
-  const float2 ax = make_float2(fabsf(dx.x) - bh.x, fabsf(dx.y) - bh.x);
-  const float2 ay = make_float2(fabsf(dy.x) - bh.y, fabsf(dy.y) - bh.y);
-  const float2 az = make_float2(fabsf(dz.x) - bh.z, fabsf(dz.y) - bh.z);
-  const float2 ux = make_float2(fmaxf(ax.x, 0.f), fmaxf(ax.y, 0.f));
-  const float2 uy = make_float2(fmaxf(ay.x, 0.f), fmaxf(ay.y, 0.f));
-  const float2 uz = make_float2(fmaxf(az.x, 0.f), fmaxf(az.y, 0.f));
-  const float2 u2 = fma2(ux, ux, fma2(uy, uy, mul2(uz, uz)));
-  const float2 mx = make_float2(fmaxf(ax.x, fmaxf(ay.x, az.x)), fmaxf(ax.y, fmaxf(ay.y, az.y)));
-  float2 w;
-  if (!GRAD) {
-    // signed distance of the box: |max(q, 0)| + min(max_k q_k, 0)
-    const float2 sdf = add2(make_float2(sqrta(u2.x), sqrta(u2.y)), make_float2(fminf(mx.x, 0.f), fminf(mx.y, 0.f)));
-    term2<COST, false>(fma2(nbl, sdf, K), inv_scale, acc.ps, w);
-  } else {
-    const float2 inv = make_float2(rsqa(fmaxf(u2.x, 1e-30f)), rsqa(fmaxf(u2.y, 1e-30f)));
-    const float2 ui = mul2(u2, inv);
-    const bool ox = mx.x > 0.f, oy = mx.y > 0.f;
-    const float2 sdf = make_float2(ox ? ui.x : mx.x, oy ? ui.y : mx.y);
-    term2<COST, true>(fma2(nbl, sdf, K), inv_scale, acc.ps, w);
-    // d(distance)/dc: the unit vector of max(q, 0) outside, the axis of the
-    // largest q inside; both with the signs of c - centre
-    float2 sx = mul2(ux, inv), sy = mul2(uy, inv), sz = mul2(uz, inv);
-    if (!ox) {
-      const bool bx = ax.x >= ay.x && ax.x >= az.x, by = !bx && ay.x >= az.x;
-      sx.x = bx ? 1.f : 0.f; sy.x = by ? 1.f : 0.f; sz.x = (!bx && !by) ? 1.f : 0.f;
-    }
-    if (!oy) {
-      const bool bx = ax.y >= ay.y && ax.y >= az.y, by = !bx && ay.y >= az.y;
-      sx.y = bx ? 1.f : 0.f; sy.y = by ? 1.f : 0.f; sz.y = (!bx && !by) ? 1.f : 0.f;
-    }
-    acc.gx = fma2(w, make_float2(copysignf(sx.x, dx.x), copysignf(sx.y, dx.y)), acc.gx);
-    acc.gy = fma2(w, make_float2(copysignf(sy.x, dy.x), copysignf(sy.y, dy.y)), acc.gy);
-    acc.gz = fma2(w, make_float2(copysignf(sz.x, dz.x), copysignf(sz.y, dz.y)), acc.gz);
-  }
-}
-
-template <bool COST, bool GRAD>
-__device__ __forceinline__ void sphere_pair2(float2 cx, float2 cy, float2 cz, float jx, float jy, float jz, float2 nbl,
-                                             float2 K, float inv_scale, PairAcc2& acc) {
-  const float2 vx = add2(cx, bc2(-jx)), vy = add2(cy, bc2(-jy)), vz = add2(cz, bc2(-jz));
-  const float2 d2 = fma2(vx, vx, fma2(vy, vy, mul2(vz, vz)));
-  float2 w;
-  if (!GRAD) {
-    term2<COST, false>(fma2(nbl, make_float2(sqrta(d2.x), sqrta(d2.y)), K), inv_scale, acc.ps, w);
-  } else {
-    const float2 inv = make_float2(rsqa(fmaxf(d2.x, 1e-30f)), rsqa(fmaxf(d2.y, 1e-30f)));
-    term2<COST, true>(fma2(nbl, mul2(d2, inv), K), inv_scale, acc.ps, w);
-    const float2 f = mul2(w, inv);
-    acc.gx = fma2(f, vx, acc.gx);
-    acc.gy = fma2(f, vy, acc.gy);
-    acc.gz = fma2(f, vz, acc.gz);
+// both spheres of a task against two spheres of another robot
+template <bool COST, bool GRAD, bool DIRECT>
+__device__ __forceinline__ void sphere_step(Side& a, Side& b, float2 x, float2 y, float2 z, float2 br, float2 nbl) {
+  float2 ax, ay, az, ai, cx, cy, cz, ci, ea, oa, ec, oc;
+  const float2 xa = sphere_x2<GRAD>(a, x, y, z, nbl, add2(a.K, br), &ax, &ay, &az, &ai);
+  const float2 xc = sphere_x2<GRAD>(b, x, y, z, nbl, add2(b.K, br), &cx, &cy, &cz, &ci);
+  soft2<COST, DIRECT>(a, xa, &ea, &oa);
+  soft2<COST, DIRECT>(b, xc, &ec, &oc);
+  if (GRAD) {
+    float2 wa, wc;
+    sigmoid4<DIRECT>(xa, ea, oa, xc, ec, oc, &wa, &wc);
+    pull(a, wa, ai, ax, ay, az);
+    pull(b, wc, ci, cx, cy, cz);
   }
 }
 
@@ -162,59 +302,79 @@ __device__ __forceinline__ void acc2(float& h, float& l, float v) {
   l += e;
 }
 
-// the cost kernel fits two 16-warp CTAs per SM (shared memory allows it when
-// the registers stay at 64); the gradient kernel holds twice the tables
-template <bool COST, bool GRAD>
-__global__ void __launch_bounds__(512, GRAD ? 1 : 2)
+// Bound: issue slots (cost: 15 warp instructions per 32 pairs, 83 % of them
+// used) and, with the gradient, the FMA and special-function pipes together
+// (18 instructions; 17 and 16 of 27 cycles per 32 pairs).  512 paths of 256
+// waypoints, four arms, 50 boxes: cost 1.55 -> 1.27 ms, gradient 3.63 -> 2.81
+// ms, both 4.03 -> 3.19 ms, against one log2 and one reciprocal per pair, two
+// spheres per packed instruction and 32-waypoint gradient CTAs (one per SM).
+// Unrolling the sphere loop by 1, 2, 4 or 8: cost 1.31, 1.31, 1.24, 1.23 ms, the
+// gradient unchanged.  12 paths of 45 waypoints: cost 117 -> 80 us, gradient 185
+// -> 80 us, from the clusters.
+template <int SEG, bool COST, bool GRAD, bool DIRECT>
+__global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 32 ? 1 : 2)
     pen_kernel(ArmDev a, PenDev pd, PenParams pp, const float* __restrict__ paths, int T, int nseg,
                const float* __restrict__ gout, double* __restrict__ seg_cost, float* __restrict__ wp_cost,
                float* __restrict__ grad, int gr0, int gr1) {
   extern __shared__ __align__(16) float smf[];
   const int S = pd.S, B = pd.B, R = a.R, D = a.D;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, NW = blockDim.x >> 5;
-  const long long p = blockIdx.x / nseg;
-  const int seg = blockIdx.x - (int)(p * nseg);
-  const int t0 = seg * kSeg;
+  // HV half warps (or whole ones) hold the same SEG waypoints: this lane's
+  // waypoint, and its share of a warp's partners and robots
+  constexpr int HV = 32 / SEG;
+  const int wl = lane & (SEG - 1), half = HV > 1 ? lane / SEG : 0;
+  // the CTAs of a cluster share one segment: each runs its kinematics and a
+  // share of the pair tasks
+  const int split = cluster_size(), rank = cluster_rank();
+  const long long sidx = blockIdx.x / split;
+  const long long p = sidx / nseg;
+  const int seg = (int)(sidx - p * nseg);
+  const int t0 = seg * SEG;
   // the gradient of this launch: robots [gr0, gr1), their spheres [s_lo, s_hi)
   // and joints [j_lo, j_hi) (robots' joints are contiguous in robot order)
   const int s_lo = pen_first_sphere(pd, R, gr0), s_hi = pen_first_sphere(pd, R, gr1);
   const int j_lo = a.q_off[gr0], j_hi = gr1 < R ? a.q_off[gr1] : D;
-  const PenLayout L(S, B, D, GRAD, NW, s_hi - s_lo, gr1 - gr0);
+  const PenLayout<SEG> L(S, B, D, GRAD, NW, s_hi - s_lo, gr1 - gr0);
   float* C = smf + L.C;
   float* Gs = smf + L.G;
   float* OZ = smf + L.OZ;
   float* W = smf + L.W;
   float* QG = smf + L.QG;
   float4* sph = (float4*)(smf + L.sph);
-  float4* box = (float4*)(smf + L.box);
-  int4* tasks = (int4*)(smf + L.task);
+  float2* box = (float2*)(smf + L.box);
   float* br = smf + L.br;
   const int NTK = pd.NTK;
   float* part = smf + L.part;
 
-  // ---- stage tables and the segment's waypoints (rows t0-1 .. t0+32)
+  // ---- stage tables and the segment's waypoints (rows t0-1 .. t0+SEG)
   for (int i = tid; i < S; i += blockDim.x) {
     sph[i] = pd.sph[i];
     br[i] = pp.beta * 1.4426950408889634f * pd.sph[i].w;
   }
-  for (int i = tid; i < NTK; i += blockDim.x) tasks[i] = pd.task[i];
-  for (int i = tid; i < 2 * B; i += blockDim.x) box[i] = pd.box[i];
+  for (int i = tid; i < 6 * ((B + 1) / 2); i += blockDim.x) {   // pair i / 6: centre x, y, z, half extent x, y, z
+    const int b = 2 * (i / 6), k = i % 6, c = b + 1 < B ? b + 1 : b;
+    const float* f = (const float*)pd.box;
+    box[i] = make_float2(f[8 * b + (k < 3 ? k : k + 1)], f[8 * c + (k < 3 ? k : k + 1)]);
+  }
   {
     const float* src = paths + (size_t)p * T * D;
-    const int n = (kSeg + 2) * D;
+    const int n = (SEG + 2) * D;
     for (int i = tid; i < n; i += blockDim.x) {
       const int t = t0 - 1 + i / D;
       W[i] = (t >= 0 && t < T) ? src[(long long)(t0 - 1) * D + i] : 0.f;
     }
   }
-  if (GRAD)
-    for (int i = tid; i < kSeg * D; i += blockDim.x) QG[i] = 0.f;
+  if (GRAD) {
+    for (int i = tid; i < SEG * D; i += blockDim.x) QG[i] = 0.f;
+    if (split > 1)   // spheres of the other CTAs' tasks add nothing to this CTA's joint gradients
+      for (int i = tid; i < (s_hi - s_lo) * 3 * SEG; i += blockDim.x) Gs[i] = 0.f;
+  }
   __syncthreads();
 
-  // ---- forward kinematics: warp r walks robot r's chain, lane = waypoint
-  if (warp < R) {
-    const int r = warp;
-    const float* q = W + (lane + 1) * D;
+  // ---- forward kinematics: (half) warp r walks robot r's chain, lane = waypoint
+  if (HV * warp + half < R) {
+    const int r = HV * warp + half;
+    const float* q = W + (wl + 1) * D;
     int jo = a.q_off[r];
     float m[9], o[3];
     {
@@ -239,9 +399,9 @@ __global__ void __launch_bounds__(512, GRAD ? 1 : 2)
     for (int k = 0; k <= nl; k++) {
       if (k > 0) {
         if (GRAD && r >= gr0 && r < gr1) {
-          float* oz = OZ + (size_t)(((r - gr0) * kMaxLinks + (k - 1)) * 6) * kSeg + lane;
-          oz[0] = o[0]; oz[kSeg] = o[1]; oz[2 * kSeg] = o[2];
-          oz[3 * kSeg] = m[2]; oz[4 * kSeg] = m[5]; oz[5 * kSeg] = m[8];
+          float* oz = OZ + (size_t)(((r - gr0) * kMaxLinks + (k - 1)) * 6) * SEG + wl;
+          oz[0] = o[0]; oz[SEG] = o[1]; oz[2 * SEG] = o[2];
+          oz[3 * SEG] = m[2]; oz[4 * SEG] = m[5]; oz[5 * SEG] = m[8];
         }
         const float4 h = a.dh32[r * kMaxLinks + k - 1];   // a, d, cos(alpha), sin(alpha)
         float sn, cs;
@@ -261,72 +421,161 @@ __global__ void __launch_bounds__(512, GRAD ? 1 : 2)
         const float4 l = sph[s];
 #pragma unroll
         for (int i = 0; i < 3; i++)
-          C[(3 * s + i) * kSeg + lane] = o[i] + ((m[3 * i] * l.x + m[3 * i + 1] * l.y) + m[3 * i + 2] * l.z);
+          C[cen<SEG>(s, i, wl)] = o[i] + ((m[3 * i] * l.x + m[3 * i + 1] * l.y) + m[3 * i + 2] * l.z);
       }
     }
   }
   __syncthreads();
 
-  // ---- pair terms.  A task is one or two spheres of one robot, lane =
-  // waypoint; its warp evaluates them against every box and every sphere of
-  // the other robots.  With the gradient, each inter-robot pair is evaluated
-  // from both sides, so a task owns its spheres' gradients outright (no
-  // atomics, a fixed summation order); the cost counts each pair once (the
-  // partners on later robots).  Tasks are dealt zig-zag over the warps.
+  // ---- pair terms.  A task is two spheres of one robot against every box and
+  // every sphere of the other robots, by one warp (SEG 16: its halves take every
+  // other pair of partners).  With the gradient, each
+  // inter-robot pair is evaluated from both sides, so a task owns its spheres'
+  // gradients outright (no atomics, a fixed summation order); the cost counts
+  // each pair once (the partners on later robots).  Tasks are dealt zig-zag
+  // over the warps.
   const float bl = pp.beta * 1.4426950408889634f;   // beta log2(e)
   const float blm = bl * pp.margin;
   float acc_h = 0.f, acc_l = 0.f;
-  for (int base = 0; base < NTK; base += NW) {
-    const int tk = ((base / NW) & 1) ? base + NW - 1 - warp : base + warp;
+  const int VW = NW * split, vw = warp * split + rank;   // the cluster's warps, dealt over its CTAs
+  for (int base = 0, turn = 0; base < NTK; base += VW, turn ^= 1) {
+    const int tk = turn ? base + VW - 1 - vw : base + vw;
     if (tk >= NTK) continue;
-    const int4 task = tasks[tk];   // sphere, second sphere (-1: none), robot's first sphere, next robot's first
+    const int4 task = __ldg(&pd.task[tk]);   // first sphere, -, robot's first sphere, next robot's first
     if (GRAD && !COST && (task.x < s_lo || task.x >= s_hi)) continue;   // another group's robot
-    const bool two = task.y >= 0;
-    const int i0 = task.x, i1 = two ? task.y : task.x;
-    const float2 cx = make_float2(C[(3 * i0) * kSeg + lane], C[(3 * i1) * kSeg + lane]);
-    const float2 cy = make_float2(C[(3 * i0 + 1) * kSeg + lane], C[(3 * i1 + 1) * kSeg + lane]);
-    const float2 cz = make_float2(C[(3 * i0 + 2) * kSeg + lane], C[(3 * i1 + 2) * kSeg + lane]);
-    const float2 K = make_float2(fmaf(bl, sph[i0].w, blm), fmaf(bl, sph[i1].w, blm));
+    const int i0 = task.x, i1 = i0 + 1;
+    auto side = [&](int i) {
+      Side d;
+      d.nx = bc2(-C[cen<SEG>(i, 0, wl)]);
+      d.ny = bc2(-C[cen<SEG>(i, 1, wl)]);
+      d.nz = bc2(-C[cen<SEG>(i, 2, wl)]);
+      d.K = bc2(fmaf(bl, sph[i].w, blm));
+      d.ps = d.pr = d.gx = d.gy = d.gz = bc2(0.f);
+      return d;
+    };
+    Side a = side(i0), b = side(i1);
     const float2 nbl = bc2(-bl);
-    PairAcc2 a{bc2(0.f), bc2(0.f), bc2(0.f), bc2(0.f)};
-#pragma unroll 2
-    for (int b = 0; b < B; b++)
-      box_pair2<COST, GRAD>(cx, cy, cz, box[2 * b], box[2 * b + 1], nbl, K, pp.inv_scale, a);
-#pragma unroll 2
-    for (int j = task.w; j < S; j++)
-      sphere_pair2<COST, GRAD>(cx, cy, cz, C[(3 * j) * kSeg + lane], C[(3 * j + 1) * kSeg + lane],
-                               C[(3 * j + 2) * kSeg + lane], nbl, add2(K, bc2(br[j])), pp.inv_scale, a);
-    if (GRAD) {
-#pragma unroll 2
-      for (int j = 0; j < task.z; j++)
-        sphere_pair2<false, true>(cx, cy, cz, C[(3 * j) * kSeg + lane], C[(3 * j + 1) * kSeg + lane],
-                                  C[(3 * j + 2) * kSeg + lane], nbl, add2(K, bc2(br[j])), pp.inv_scale, a);
-      const int g0 = i0 - s_lo, g1 = i1 - s_lo;
-      Gs[(3 * g0) * kSeg + lane] = a.gx.x;
-      Gs[(3 * g0 + 1) * kSeg + lane] = a.gy.x;
-      Gs[(3 * g0 + 2) * kSeg + lane] = a.gz.x;
-      if (two) {
-        Gs[(3 * g1) * kSeg + lane] = a.gx.y;
-        Gs[(3 * g1 + 1) * kSeg + lane] = a.gy.y;
-        Gs[(3 * g1 + 2) * kSeg + lane] = a.gz.y;
+    const float4* b4 = (const float4*)box;
+    auto boxes = [&](int k, float2 Ka, float2 Kb) {
+      const float4 u = b4[3 * k], v = b4[3 * k + 1], w = b4[3 * k + 2];
+      const Box2 bx{make_float2(u.x, u.y), make_float2(u.z, u.w), make_float2(v.x, v.y),
+                    make_float2(v.z, v.w), make_float2(w.x, w.y), make_float2(w.z, w.w)};
+      box_step<COST, GRAD, DIRECT>(a, b, bx, nbl, Ka, Kb);
+    };
+    const int nb2 = B / 2, even = nb2 & ~(HV - 1);
+    for (int k = 0; k < even; k += HV) {
+      boxes(k + half, a.K, b.K);
+      if (COST && (k / HV) % kProd == kProd - 1) {
+        flush_product<COST>(a);
+        flush_product<COST>(b);
       }
     }
-    if (COST) acc2(acc_h, acc_l, two ? a.ps.x + a.ps.y : a.ps.x);
+    if (B > 2 * even) {   // the boxes left: a place without a box adds nothing
+      const int k = even + half, left = B - 2 * k;   // of this half's pair: both there when 2 or more, the first when 1
+      const float kx = left > 0 ? 0.f : kNone, ky = left > 1 ? 0.f : kNone;
+      boxes(left > 0 ? k : even, add2(a.K, make_float2(kx, ky)), add2(b.K, make_float2(kx, ky)));
+    }
+    flush_product<COST>(a);
+    flush_product<COST>(b);
+    const float2* C2 = (const float2*)C + wl;
+    const float2* br2 = (const float2*)br;
+    auto spheres = [&](auto with_cost, int j, float2 r) {
+      sphere_step<decltype(with_cost)::value, GRAD, DIRECT>(a, b, C2[(3 * j) * SEG], C2[(3 * j + 1) * SEG],
+                                                            C2[(3 * j + 2) * SEG], r, nbl);
+    };
+    const float2 none = bc2(kNone);
+    {   // the later robots' spheres
+      const int j0 = task.w / 2, j1 = S / 2, je = j0 + ((j1 - j0) & ~(HV - 1));
+#pragma unroll 4
+      for (int j = j0; j < je; j += HV) {
+        spheres(Flag<COST>(), j + half, br2[j + half]);
+        if (COST && ((j - j0) / HV) % kProd == kProd - 1) {
+          flush_product<COST>(a);
+          flush_product<COST>(b);
+        }
+      }
+      if (HV > 1 && je < j1) spheres(Flag<COST>(), je, half ? none : br2[je]);
+      flush_product<COST>(a);
+      flush_product<COST>(b);
+    }
+    if (GRAD) {   // the earlier robots' (the cost has counted them)
+      const int z = task.z / 2, ze = z & ~(HV - 1);
+#pragma unroll 4
+      for (int j = 0; j < ze; j += HV) spheres(Flag<false>(), j + half, br2[j + half]);
+      if (HV > 1 && ze < z) spheres(Flag<false>(), ze, half ? none : br2[ze]);
+      const float is = pp.inv_scale;
+      const float g[3] = {a.gx.x + a.gx.y, a.gy.x + a.gy.y, a.gz.x + a.gz.y};
+      const float h[3] = {b.gx.x + b.gx.y, b.gy.x + b.gy.y, b.gz.x + b.gz.y};
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        if (HV == 1) {
+          Gs[(3 * (i0 - s_lo) + i) * SEG + wl] = is * g[i];
+          Gs[(3 * (i1 - s_lo) + i) * SEG + wl] = is * h[i];
+        } else {   // both halves' sums: half 0 stores the first sphere's, half 1 the second's
+          const float mine = half ? h[i] : g[i], other = half ? g[i] : h[i];
+          Gs[(3 * (i0 + half - s_lo) + i) * SEG + wl] = is * (mine + __shfl_xor_sync(MRMG_FULL, other, SEG & 31));
+        }
+      }
+    }
+    if (COST) acc2(acc_h, acc_l, (a.ps.x + a.ps.y) + (b.ps.x + b.ps.y));
   }
   if (COST) {
-    part[warp * kSeg + lane] = acc_h;
-    part[(NW + warp) * kSeg + lane] = acc_l;
+    part[warp * 32 + lane] = acc_h;
+    part[(NW + warp) * 32 + lane] = acc_l;
   }
   __syncthreads();
 
-  const int t = t0 + lane;
+  double csum = 0.0;   // warp 0: this CTA's pair terms of waypoint t0 + wl
   if (COST && warp == 0) {
-    double c = 0.0;
-    for (int w = 0; w < NW; w++) c += (double)part[w * kSeg + lane] + (double)part[(NW + w) * kSeg + lane];
+    for (int w = 0; w < NW; w++) csum += (double)part[w * 32 + lane] + (double)part[(NW + w) * 32 + lane];
+    if (HV > 1) csum += __shfl_xor_sync(MRMG_FULL, csum, SEG & 31);
+    __syncwarp();
+    ((double*)part)[lane] = csum;
+  }
+  if (GRAD) {
+    // ---- joint gradients from the sphere gradients, tip to base
+    if (gr0 + HV * warp + half < gr1) {
+      const int r = gr0 + HV * warp + half;
+      const int nl = a.nl[r];
+      int jo = a.q_off[r] + (a.base_kind[r] == 1 ? 3 : 0);
+      float G0 = 0.f, G1 = 0.f, G2 = 0.f, M0 = 0.f, M1 = 0.f, M2 = 0.f;
+      float* qg = QG + wl * D;
+      for (int k = nl; k >= 0; k--) {
+        for (int s = pd.lk[r][k]; s < pd.lk[r][k + 1]; s++) {
+          const float c0 = C[cen<SEG>(s, 0, wl)], c1 = C[cen<SEG>(s, 1, wl)], c2 = C[cen<SEG>(s, 2, wl)];
+          const int sg = s - s_lo;
+          const float g0 = Gs[(3 * sg) * SEG + wl], g1 = Gs[(3 * sg + 1) * SEG + wl], g2 = Gs[(3 * sg + 2) * SEG + wl];
+          G0 += g0; G1 += g1; G2 += g2;
+          M0 += c1 * g2 - c2 * g1;
+          M1 += c2 * g0 - c0 * g2;
+          M2 += c0 * g1 - c1 * g0;
+        }
+        if (k == 0) break;
+        const float* oz = OZ + (size_t)(((r - gr0) * kMaxLinks + (k - 1)) * 6) * SEG + wl;
+        const float o0 = oz[0], o1 = oz[SEG], o2 = oz[2 * SEG];
+        const float z0 = oz[3 * SEG], z1 = oz[4 * SEG], z2 = oz[5 * SEG];
+        const float v0 = M0 - (o1 * G2 - o2 * G1), v1 = M1 - (o2 * G0 - o0 * G2), v2 = M2 - (o0 * G1 - o1 * G0);
+        qg[jo + k - 1] = z0 * v0 + z1 * v1 + z2 * v2;
+      }
+      if (a.base_kind[r] == 1) {
+        const int b0 = a.q_off[r];
+        const float x = W[(wl + 1) * D + b0], y = W[(wl + 1) * D + b0 + 1];
+        qg[b0] = G0;
+        qg[b0 + 1] = G1;
+        qg[b0 + 2] = M2 - (x * G1 - y * G0);
+      }
+    }
+  }
+  if (split > 1) cluster_sync();   // every CTA's sums are in place
+
+  const int t = t0 + wl;
+  if (COST && warp == 0 && rank == 0) {
+    double c = csum;
+    for (int r = 1; r < split; r++) c += cluster_ld64((double*)part + lane, r);
     c *= 0.69314718055994531 * (double)pp.inv_beta * (double)pp.inv_scale;   // ln 2 / (beta scale)
     if (t + 1 < T) {
-      const float* w0 = W + (lane + 1) * D;
-      const float* w1 = W + (lane + 2) * D;
+      const float* w0 = W + (wl + 1) * D;
+      const float* w1 = W + (wl + 2) * D;
       float sh = 0.f, sl = 0.f;
       for (int k = 0; k < D; k++) {
         const float dv = w1[k] - w0[k];
@@ -334,53 +583,21 @@ __global__ void __launch_bounds__(512, GRAD ? 1 : 2)
       }
       c += (double)pp.smooth_w * ((double)sh + (double)sl);
     }
-    if (t >= T) c = 0.0;
-    if (wp_cost && t < T) wp_cost[(size_t)p * T + t] = (float)c;
+    if (t >= T || half) c = 0.0;   // the second half holds copies
+    if (wp_cost && t < T && !half) wp_cost[(size_t)p * T + t] = (float)c;
 #pragma unroll
     for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(MRMG_FULL, c, o);
     if (lane == 0 && seg_cost) seg_cost[(size_t)p * nseg + seg] = c;
   }
 
   if (GRAD) {
-    // ---- joint gradients from the sphere gradients, tip to base
-    if (warp >= gr0 && warp < gr1) {
-      const int r = warp;
-      const int nl = a.nl[r];
-      int jo = a.q_off[r] + (a.base_kind[r] == 1 ? 3 : 0);
-      float G0 = 0.f, G1 = 0.f, G2 = 0.f, M0 = 0.f, M1 = 0.f, M2 = 0.f;
-      float* qg = QG + lane * D;
-      for (int k = nl; k >= 0; k--) {
-        for (int s = pd.lk[r][k]; s < pd.lk[r][k + 1]; s++) {
-          const float c0 = C[(3 * s) * kSeg + lane], c1 = C[(3 * s + 1) * kSeg + lane], c2 = C[(3 * s + 2) * kSeg + lane];
-          const int sg = s - s_lo;
-          const float g0 = Gs[(3 * sg) * kSeg + lane], g1 = Gs[(3 * sg + 1) * kSeg + lane], g2 = Gs[(3 * sg + 2) * kSeg + lane];
-          G0 += g0; G1 += g1; G2 += g2;
-          M0 += c1 * g2 - c2 * g1;
-          M1 += c2 * g0 - c0 * g2;
-          M2 += c0 * g1 - c1 * g0;
-        }
-        if (k == 0) break;
-        const float* oz = OZ + (size_t)(((r - gr0) * kMaxLinks + (k - 1)) * 6) * kSeg + lane;
-        const float o0 = oz[0], o1 = oz[kSeg], o2 = oz[2 * kSeg];
-        const float z0 = oz[3 * kSeg], z1 = oz[4 * kSeg], z2 = oz[5 * kSeg];
-        const float v0 = M0 - (o1 * G2 - o2 * G1), v1 = M1 - (o2 * G0 - o0 * G2), v2 = M2 - (o0 * G1 - o1 * G0);
-        qg[jo + k - 1] = z0 * v0 + z1 * v1 + z2 * v2;
-      }
-      if (a.base_kind[r] == 1) {
-        const int b0 = a.q_off[r];
-        const float x = W[(lane + 1) * D + b0], y = W[(lane + 1) * D + b0 + 1];
-        qg[b0] = G0;
-        qg[b0 + 1] = G1;
-        qg[b0 + 2] = M2 - (x * G1 - y * G0);
-      }
-    }
     __syncthreads();
     // ---- add the smoothness gradient, scale by dL/dcost, write coalesced
     const float go = gout ? gout[p] : 1.f;
     const float sw2 = 2.f * pp.smooth_w;
-    const int n = kSeg * D;
+    const int n = SEG * D, share = (n + split - 1) / split;   // each CTA writes a share of the rows
     float* dst = grad + ((size_t)p * T + t0) * D;
-    for (int i = tid; i < n; i += blockDim.x) {
+    for (int i = rank * share + tid; i < min(n, (rank + 1) * share); i += blockDim.x) {
       const int tt = t0 + i / D;
       if (tt >= T) break;
       const int j = i - (i / D) * D;
@@ -389,9 +606,15 @@ __global__ void __launch_bounds__(512, GRAD ? 1 : 2)
       float gsm = 0.f;
       if (tt > 0) gsm += sw2 * (wc - W[i]);
       if (tt + 1 < T) gsm -= sw2 * (W[i + 2 * D] - wc);
-      dst[i] = go * (QG[i] + gsm);
+      float qg = QG[i];
+      if (split > 1) {
+        qg = cluster_ld(QG + i, 0);
+        for (int r = 1; r < split; r++) qg += cluster_ld(QG + i, r);
+      }
+      dst[i] = go * (qg + gsm);
     }
   }
+  if (split > 1) cluster_sync();   // no CTA leaves while another reads its shared memory
 }
 
 __global__ void pen_sum_kernel(const double* __restrict__ seg, long long P, int nseg, double* __restrict__ cost) {
@@ -402,25 +625,86 @@ __global__ void pen_sum_kernel(const double* __restrict__ seg, long long P, int 
   }
 }
 
-template <bool COST, bool GRAD>
+// CTAs per segment: a segment's pair tasks go to a cluster of `s` CTAs where the
+// segments alone leave SMs idle.  Modelled time: waves of CTAs, each paying the
+// fixed part (tables, kinematics, joint gradients: about a tenth of a segment's
+// time by clock stamps) and its share of the pairs.  24 segments on 152 SMs: one
+// CTA each 117 us, clusters of 8 80 us (cost kernel).
+int pen_split(long long segs, int slots) {
+  int best = 1;
+  double best_t = 0.0;
+  for (int s = 1; s <= kMaxSplit; s *= 2) {
+    const double t = (double)((segs * s + slots - 1) / slots) * (kFixedShare + 1.0 / s);
+    if (s == 1 || t < best_t) {
+      best = s;
+      best_t = t;
+    }
+  }
+  return best;
+}
+
+template <int SEG, bool COST, bool GRAD, bool DIRECT>
 cudaError_t launch_one(const ArmDev& a, const PenDev& pd, const PenParams& pp, const float* paths, long long P, int T,
-                       int nseg, const float* gout, double* seg, float* wp, float* grad, int warps, int gr0, int gr1,
+                       const float* gout, double* seg, float* wp, float* grad, int warps, int split, int gr0, int gr1,
                        cudaStream_t st) {
-  const PenLayout L(pd.S, pd.B, a.D, GRAD, warps, pen_first_sphere(pd, a.R, gr1) - pen_first_sphere(pd, a.R, gr0),
-                    gr1 - gr0);
+  const PenLayout<SEG> L(pd.S, pd.B, a.D, GRAD, warps, pen_first_sphere(pd, a.R, gr1) - pen_first_sphere(pd, a.R, gr0),
+                         gr1 - gr0);
   const size_t smem = L.total * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(pen_kernel<COST, GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto kernel = pen_kernel<SEG, COST, GRAD, DIRECT>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  pen_kernel<COST, GRAD><<<(unsigned)(P * nseg), warps * 32, smem, st>>>(a, pd, pp, paths, T, nseg, gout, seg, wp, grad,
-                                                                          gr0, gr1);
-  return cudaGetLastError();
+  const int nseg = pen_segments(T, SEG);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(P * nseg * split));
+  cfg.blockDim = dim3(warps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = split;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = split > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, a, pd, pp, paths, T, nseg, gout, seg, wp, grad, gr0, gr1);
+}
+
+// One launch covers every path unless its grid would pass the limit of
+// 2^31 - 1 CTAs.
+template <int SEG, bool COST, bool GRAD>
+cudaError_t launch_form(const ArmDev& a, const PenDev& pd, const PenParams& pp, const float* paths, long long P, int T,
+                        const float* gout, double* seg, float* wp, float* grad, int warps, int gr0, int gr1,
+                        int num_sms, cudaStream_t st) {
+  // the largest x2 of any pair: centres coincide, or lie deepest in a box
+  const bool direct = pp.beta * 1.4426951f * (pp.margin + pd.reach) <= kDirectMax;
+  const int nseg = pen_segments(T, SEG);
+  const int split = pen_split(P * nseg, num_sms * (GRAD && SEG == 32 ? 1 : 2));
+  const long long step = std::max(1ll, 0x7fffffffll / ((long long)nseg * split));
+  cudaError_t e = cudaSuccess;
+  for (long long p0 = 0; p0 < P && e == cudaSuccess; p0 += step) {
+    const long long n = std::min(step, P - p0);
+    const size_t wp0 = (size_t)p0 * T;
+    const float* w = paths + wp0 * a.D;
+    const float* go = gout ? gout + p0 : nullptr;
+    double* sg = seg ? seg + p0 * nseg : nullptr;
+    float* wc = wp ? wp + wp0 : nullptr;
+    float* g = grad ? grad + wp0 * a.D : nullptr;
+    if (direct) e = launch_one<SEG, COST, GRAD, true>(a, pd, pp, w, n, T, go, sg, wc, g, warps, split, gr0, gr1, st);
+    else e = launch_one<SEG, COST, GRAD, false>(a, pd, pp, w, n, T, go, sg, wc, g, warps, split, gr0, gr1, st);
+  }
+  return e;
+}
+
+template <int SEG>
+size_t smem_bytes(const ArmDev& a, const PenDev& pd, int grad, int warps, int gr0, int gr1) {
+  return PenLayout<SEG>(pd.S, pd.B, a.D, grad != 0, warps,
+                        pen_first_sphere(pd, a.R, gr1) - pen_first_sphere(pd, a.R, gr0), gr1 - gr0)
+             .total * sizeof(float);
 }
 
 }  // namespace
 
 size_t pen_smem_bytes(const ArmDev& a, const PenDev& pd, int grad, int warps, int gr0, int gr1) {
-  return PenLayout(pd.S, pd.B, a.D, grad != 0, warps, pen_first_sphere(pd, a.R, gr1) - pen_first_sphere(pd, a.R, gr0),
-                   gr1 - gr0).total * sizeof(float);
+  return smem_bytes<32>(a, pd, grad, warps, gr0, gr1);
 }
 
 int pen_grad_groups(const ArmDev& a, const PenDev& pd, int warps, size_t smem_max, int* bounds) {
@@ -443,20 +727,31 @@ int pen_grad_groups(const ArmDev& a, const PenDev& pd, int warps, size_t smem_ma
 
 cudaError_t pen_launch(const ArmDev& a, const PenDev& pd, const PenParams& pp, const float* paths, long long P, int T,
                        const float* gout, double* seg, double* cost, float* wp_cost, float* grad, int warps,
-                       int n_groups, const int* bounds, cudaStream_t st) {
+                       int n_groups, const int* bounds, int num_sms, size_t smem_sm, cudaStream_t st) {
   if (P <= 0) return cudaSuccess;
-  const int nseg = (T + kSeg - 1) / kSeg;
   const bool want_cost = cost || wp_cost;
+  // gradient form: half-warp segments where two of their CTAs fit an SM
+  const int gw = std::min(warps, kPenGradWarps);
+  const bool halves = grad && n_groups <= 1 && 2 * (smem_bytes<16>(a, pd, 1, gw, 0, a.R) + 1024) <= smem_sm;
   cudaError_t e = cudaSuccess;
-  if (grad && n_groups <= 1) {
-    if (want_cost) e = launch_one<true, true>(a, pd, pp, paths, P, T, nseg, gout, seg, wp_cost, grad, warps, 0, a.R, st);
-    else e = launch_one<false, true>(a, pd, pp, paths, P, T, nseg, gout, nullptr, nullptr, grad, warps, 0, a.R, st);
+  int nseg = pen_segments(T, 32);   // segments whose costs are summed
+  if (grad && n_groups <= 1 && halves) {
+    nseg = pen_segments(T, 16);
+    if (want_cost)
+      e = launch_form<16, true, true>(a, pd, pp, paths, P, T, gout, seg, wp_cost, grad, gw, 0, a.R, num_sms, st);
+    else
+      e = launch_form<16, false, true>(a, pd, pp, paths, P, T, gout, nullptr, nullptr, grad, gw, 0, a.R, num_sms, st);
+  } else if (grad && n_groups <= 1) {
+    if (want_cost)
+      e = launch_form<32, true, true>(a, pd, pp, paths, P, T, gout, seg, wp_cost, grad, warps, 0, a.R, num_sms, st);
+    else
+      e = launch_form<32, false, true>(a, pd, pp, paths, P, T, gout, nullptr, nullptr, grad, warps, 0, a.R, num_sms, st);
   } else {
     if (want_cost || !grad)
-      e = launch_one<true, false>(a, pd, pp, paths, P, T, nseg, gout, seg, wp_cost, nullptr, warps, 0, a.R, st);
+      e = launch_form<32, true, false>(a, pd, pp, paths, P, T, gout, seg, wp_cost, nullptr, warps, 0, a.R, num_sms, st);
     for (int g = 0; grad && g < n_groups && e == cudaSuccess; g++)
-      e = launch_one<false, true>(a, pd, pp, paths, P, T, nseg, gout, nullptr, nullptr, grad, warps, bounds[g],
-                                  bounds[g + 1], st);
+      e = launch_form<32, false, true>(a, pd, pp, paths, P, T, gout, nullptr, nullptr, grad, warps, bounds[g],
+                                       bounds[g + 1], num_sms, st);
   }
   if (e != cudaSuccess || !cost) return e;
   const int blocks = (int)std::min<long long>((P + 255) / 256, 4096);
