@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/mrmg_gb300.h"
+#include "mrmg_exact.cuh"
 
 #define MRMG_FULL 0xffffffffu
 

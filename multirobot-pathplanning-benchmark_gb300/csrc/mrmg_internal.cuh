@@ -216,26 +216,31 @@ struct SliceTab {
 
 // FP64 distance of one difference row d(k) = a[k] - b[k] with the reference's
 // operation order (NpConfiguration._batch_dist, core/configuration.py:303-329:
-// sequential unfused sums of d*d, IEEE sqrt, strict '>' maxima)
+// sequential unfused sums of d*d, IEEE sqrt, strict '>' maxima).  The squares,
+// the root and the maxima run on the integer pipes with the same bits
+// (mrmg_exact.cuh), a sum starts with its first square (0 + x = x): per
+// coordinate two FP64 operations are left, a subtraction and an addition.
+template <class Diff>
+__device__ __forceinline__ double square_sum(int s, int e, Diff d) {
+  if (s >= e) return 0.0;
+  double acc = square_rn(d(s));
+  for (int k = s + 1; k < e; k++) acc = __dadd_rn(acc, square_rn(d(k)));
+  return acc;
+}
 template <class Diff>
 __device__ __forceinline__ double dist_of(const SliceTab& t, int metric, Diff d) {
-  if (metric == MRMG_METRIC_EUCLIDEAN) {
-    double acc = 0.0;
-    for (int k = 0; k < t.end_all; k++) { double v = d(k); acc = __dadd_rn(acc, __dmul_rn(v, v)); }
-    return sqrt(acc);
-  }
+  if (metric == MRMG_METRIC_EUCLIDEAN) return sqrt_rn(square_sum(0, t.end_all, d));
   if (metric == MRMG_METRIC_MAX) {
-    double m = fabs(d(0));
-    for (int k = 1; k < t.D; k++) { double v = fabs(d(k)); if (v > m) m = v; }
+    double m = abs64(d(0));
+    for (int k = 1; k < t.D; k++) { const double v = abs64(d(k)); if (above(v, m)) m = v; }
     return m;
   }
   double red = 0.0;
   for (int i = 0; i < t.A; i++) {
-    double acc = 0.0;
-    for (int k = t.s[i]; k < t.e[i]; k++) { double v = d(k); acc = __dadd_rn(acc, __dmul_rn(v, v)); }
-    const double r = sqrt(acc);
-    if (metric == MRMG_METRIC_SUM_EUCLIDEAN) red = __dadd_rn(red, r);
-    else if (i == 0 || r > red) red = r;
+    const double r = sqrt_rn(square_sum(t.s[i], t.e[i], d));
+    if (i == 0) red = r;
+    else if (metric == MRMG_METRIC_SUM_EUCLIDEAN) red = __dadd_rn(red, r);
+    else if (above(r, red)) red = r;
   }
   return red;
 }
