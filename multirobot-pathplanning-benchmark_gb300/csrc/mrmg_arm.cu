@@ -793,7 +793,8 @@ __device__ __forceinline__ void warp_areas(const ArmDev& s, unsigned char* smem_
 template <int GPL, int SPG, bool RESOLVE>
 __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ? 2 : 1))) arm_configs_kernel(ArmDev s, const void* q, int dtype, long long n,
                                                           uint8_t* out, int* ctr, long long* pend, int full) {
-  if (RESOLVE && ctr[kCtrPending] == 0) return;   // nothing was left undecided
+  // pass 2: as many CTAs stay as there are undecided items for their warps
+  if (RESOLVE && (long long)blockIdx.x * (blockDim.x >> 5) >= ctr[kCtrPending]) return;
   extern __shared__ __align__(16) unsigned char smem_arm[];
   ArmSmem t;
   stage_tables(s, smem_arm, &t);
@@ -836,10 +837,19 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
 //            warp in blocks of 32; a collision marks the edge dead and its
 //            remaining positions are skipped.  Long free edges no longer run on
 //            one warp.
-//   finalize survivors' verdicts (last CTA of the last phase-B launch);
-//            undecided ones join the FP64 pending list.
-//   pass 2   (RESOLVE) warp per pending edge, the reference's order, exact.
+//   finalize survivors' verdicts (last CTA of the last phase-B launch)
+//   pass 2   (RESOLVE) warp per undecided position, exact (the verdict does not
+//            depend on the order: an edge that no decided position collides
+//            with is free unless one of these collides).  Entries that name no
+//            position walk the whole edge in the reference's order; walking
+//            every undecided edge took 320 of the 1,960 us of 60,000 mostly free
+//            edges (15 of them undecided, each 15 positions of 20 us one after
+//            another on one warp).
 // ---------------------------------------------------------------------------
+// An entry of the pending list: the edge, and an undecided position + 1 (with
+// kPendBfs: its place in the BFS order; 0: the whole edge)
+constexpr int kPendBfs = 1 << 30;
+__device__ __forceinline__ long long pend_entry(long long e, int code) { return e | ((long long)code << 32); }
 
 // this lane's joints of edge e as double-floats: a = q1, d = q2 - q1
 __device__ __forceinline__ void load_edge(const void* q1, const void* q2, int dtype, long long e, int D, int lane,
@@ -908,8 +918,9 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
                                                         long long n, double res, int incl,
                                                         const long long* Np, long long N_start,
                                                         long long N_max, uint8_t* out, int* ctr,
-                                                        long long* pend, SurvivorEdge* surv, int full) {
-  if (RESOLVE && ctr[kCtrPending] == 0) return;   // nothing was left undecided
+                                                        long long* pend, long long pend_cap, SurvivorEdge* surv, int full) {
+  // pass 2: as many CTAs stay as there are undecided items for their warps
+  if (RESOLVE && (long long)blockIdx.x * (blockDim.x >> 5) >= ctr[kCtrPending]) return;
   extern __shared__ __align__(16) unsigned char smem_arm[];
   ArmSmem t;
   stage_tables(s, smem_arm, &t);
@@ -929,9 +940,19 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
     if (lane == 0) k = atomicAdd(&ctr[RESOLVE ? kCtrQueue2 : kCtrQueue], 1);
     k = __shfl_sync(MRMG_FULL, k, 0);
     long long e;
+    int code = 0;
     if (RESOLVE) {
-      if (k >= ctr[kCtrPending]) break;
-      e = pend[k];
+      const int listed = min(ctr[kCtrPending], (int)min(pend_cap, 0x7fffffffll));
+      if (k >= (long long)listed + (ctr[kCtrPendLost] ? ctr[kCtrL1] : 0)) break;
+      if (k < listed) {
+        e = pend[k] & 0xffffffffll;
+        code = (int)(pend[k] >> 32);
+        if (code && out[e] == V_COLLIDE) continue;      // another position of the edge collides
+      } else {                                          // the list overflowed: survivors with a lost entry
+        const SurvivorEdge& sv = surv[k - listed];
+        if (!sv.pend || sv.dead) continue;
+        e = sv.e;
+      }
     } else {
       if (k >= n) break;
       e = k;
@@ -941,7 +962,7 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
     bool nanf;
     load_edge(q1, q2, dtype, e, D, lane, &sdf, &mloc, &nanf);
     long long N = 0;
-    const bool good = edge_N(q1, q2, dtype, e, D, lane, res, res32, Np, mloc, nanf, !RESOLVE, &N);
+    const bool good = edge_N(q1, q2, dtype, e, D, lane, res, res32, Np, mloc, nanf, true, &N);
     if (!good || N_start > N) {
       if (lane == 0) { atomicOr(&ctr[kCtrErr], !good ? E_BAD_INPUT : E_N_START); out[e] = 0; }
       __syncwarp();
@@ -976,14 +997,16 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
               const int slot = atomicAdd(&ctr[kCtrL1], 1);
               SurvivorEdge sv;
               sv.e = e; sv.N = (int)N; sv.p_next = (int)(p + 1); sv.nmax = (int)nmax;
-              sv.dead = code == V_COLLIDE; sv.pend = code == V_PENDING; sv.pad = 0;
+              sv.dead = code == V_COLLIDE; sv.pend = 0; sv.pad = 0;
               surv[slot] = sv;
+              // phase A adds at most one entry per edge: the list has room
+              if (code == V_PENDING) pend[atomicAdd(&ctr[kCtrPending], 1)] = pend_entry(e, kPendBfs | (int)(p + 1));
               atomicMax(&ctr[kCtrMaxJ], (int)(nmax - p - 1));
             }
             __syncwarp();
             continue;                       // phase B decides (its last launch finalizes)
           } else {
-            r = code;
+            r = code;   // (pending: pass 2 walks the edge, which has this position only)
           }
         }
       }
@@ -991,12 +1014,13 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
         out[e] = r;
         if (r == V_PENDING) {
           const int slot = atomicAdd(&ctr[kCtrPending], 1);
-          pend[slot] = e;
+          pend[slot] = pend_entry(e, 0);
         }
       }
       __syncwarp();
     } else {
-      // ---- pass 2: the reference's order, one configuration at a time, FP64 where pending
+      // ---- pass 2: the undecided position, or the reference's order, one
+      // configuration at a time, FP64 where pending
       EdgeSource64 s64;
       const double denom = (double)(N - 1);
 #pragma unroll
@@ -1011,15 +1035,19 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
       }
       BfsChunker ch;
       ch.init(N);
-      long long v;
+      long long v = (code & kPendBfs) ? bfs_at(N, (code & ~kPendBfs) - 1) : (long long)code - 1;   // the position, or -1
+      const bool one = code != 0;
       unsigned m;
       long long pos0;
       bool coll = false;
-      while (!coll && ch.next(lane, &v, &m, &pos0)) {
-        if (pos0 >= nmax) break;
-        const long long my_pos = pos0 + __popc(m & lt_mask);
-        const bool active = v >= 0 && my_pos >= N_start && my_pos < nmax && (incl || (v != 0 && v != N - 1));
-        unsigned act = __ballot_sync(MRMG_FULL, active);
+      while (!coll && (one || ch.next(lane, &v, &m, &pos0))) {
+        unsigned act = 1u;
+        if (!one) {
+          if (pos0 >= nmax) break;
+          const long long my_pos = pos0 + __popc(m & lt_mask);
+          const bool active = v >= 0 && my_pos >= N_start && my_pos < nmax && (incl || (v != 0 && v != N - 1));
+          act = __ballot_sync(MRMG_FULL, active);
+        }
         while (act) {
           const int srcl = __ffs(act) - 1;
           act &= act - 1;
@@ -1029,27 +1057,24 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
             break;
           }
         }
+        if (one) break;
       }
-      if (lane == 0) out[e] = coll ? V_COLLIDE : V_FREE;
+      // a position's edge is free already unless one of its positions collides
+      if (lane == 0 && (coll || !one)) out[e] = coll ? V_COLLIDE : V_FREE;
       __syncwarp();
     }
   }
   if (lane == 0 && !RESOLVE) atomicAdd((unsigned long long*)&ctr[kCtrStat0], (unsigned long long)stat_cfg);
 }
 
-// survivors' verdicts; undecided ones join the FP64 pending list.  Run by
+// survivors' verdicts from the positions decided in FP32.  Run by
 // one CTA (thread stride) after every phase-B configuration has finished.
-__device__ void finalize_survivors(int* ctr, const SurvivorEdge* surv, uint8_t* out, long long* pend) {
+__device__ void finalize_survivors(int* ctr, const SurvivorEdge* surv, uint8_t* out) {
   const int nsv = *(volatile int*)&ctr[kCtrL1];
   const volatile SurvivorEdge* vs = surv;
   for (int l = threadIdx.x; l < nsv; l += blockDim.x) {
     const long long e = vs[l].e;
-    const uint8_t r = vs[l].dead ? V_COLLIDE : (vs[l].pend ? V_PENDING : V_FREE);
-    out[e] = r;
-    if (r == V_PENDING) {
-      const int slot = atomicAdd(&ctr[kCtrPending], 1);
-      pend[slot] = e;
-    }
+    out[e] = vs[l].dead ? V_COLLIDE : V_FREE;   // (undecided positions: pass 2 may still find a collision)
   }
 }
 
@@ -1057,7 +1082,8 @@ __device__ void finalize_survivors(int* ctr, const SurvivorEdge* surv, uint8_t* 
 template <int GPL, int SPG>
 __global__ void __launch_bounds__(256, GPL == 1 ? 3 : (GPL == 2 ? 2 : 1)) arm_edges_phase_b(ArmDev s, const void* q1, const void* q2, int dtype,
                                                          int incl, int* ctr, SurvivorEdge* surv, int full,
-                                                         int j_lo, int j_hi, uint8_t* out, long long* pend) {
+                                                         int j_lo, int j_hi, uint8_t* out, long long* pend,
+                                                         long long pend_cap) {
   // the last launch (j_hi < 0) also finalizes: its last CTA to finish sets the
   // survivors' verdicts (or CTA 0, when the launch has no positions left)
   const bool fin = j_hi < 0;
@@ -1066,7 +1092,7 @@ __global__ void __launch_bounds__(256, GPL == 1 ? 3 : (GPL == 2 ? 2 : 1)) arm_ed
   const long long first = (long long)nsv * j_lo;
   const long long total = (long long)nsv * maxj;
   if (total <= first) {
-    if (fin && blockIdx.x == 0) finalize_survivors(ctr, surv, out, pend);
+    if (fin && blockIdx.x == 0) finalize_survivors(ctr, surv, out);
     return;
   }
   extern __shared__ __align__(16) unsigned char smem_arm[];
@@ -1121,7 +1147,11 @@ __global__ void __launch_bounds__(256, GPL == 1 ? 3 : (GPL == 2 ? 2 : 1)) arm_ed
                                                                     full != 0 || j_lo > 0);
       if (lane == 0) {
         if (code == V_COLLIDE) vsurv[ls].dead = 1;
-        else if (code == V_PENDING) vsurv[ls].pend = 1;
+        else if (code == V_PENDING) {
+          const int slot = atomicAdd(&ctr[kCtrPending], 1);
+          if (slot < pend_cap) pend[slot] = pend_entry(e, (int)is + 1);
+          else vsurv[ls].pend = ctr[kCtrPendLost] = 1;
+        }
       }
     }
   }
@@ -1136,7 +1166,7 @@ __global__ void __launch_bounds__(256, GPL == 1 ? 3 : (GPL == 2 ? 2 : 1)) arm_ed
     __syncthreads();
     if (s_last) {
       __threadfence();
-      finalize_survivors(ctr, surv, out, pend);
+      finalize_survivors(ctr, surv, out);
     }
   }
 }
@@ -1471,7 +1501,7 @@ cudaError_t launch_edges(const ArmDev& s, int gpl, const void* q1, const void* q
   if (gpl == G_ && s.SPG == S_) {                                                                  \
     auto k = arm_edges_kernel<G_, S_, RESOLVE>;                                                    \
     k<<<grid, warps * 32, smem, st>>>(s, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out,     \
-                                      sc.ctr, sc.pend, sc.surv, full);                             \
+                                      sc.ctr, sc.pend, sc.pend_cap, sc.surv, full);                             \
     return cudaGetLastError();                                                                     \
   }
   MRMG_ARM_EDGE(1, 6)
@@ -1507,7 +1537,7 @@ cudaError_t launch_phase_b(const ArmDev& s, int gpl, const void* q1, const void*
   if (gpl == G_ && s.SPG == S_) {                                                                  \
     grid = std::min(grid, num_sms * phase_b_occupancy<G_, S_>(warps, smem));                       \
     arm_edges_phase_b<G_, S_><<<grid, warps * 32, smem, st>>>(s, q1, q2, dtype, incl, sc.ctr, sc.surv, full, \
-                                                              j_lo, j_hi, out, sc.pend);           \
+                                                              j_lo, j_hi, out, sc.pend, sc.pend_cap); \
     return cudaGetLastError();                                                                     \
   }
   MRMG_ARM_PB(1, 6)
@@ -1525,6 +1555,11 @@ int arm_supported_spg(int idx) {
 }
 
 int arm_gpl_for_spg(int spg) { return spg == 6 ? 1 : spg == 5 ? 2 : spg == 8 ? 4 : 0; }
+
+// Launch shape of the FP64 pass.  An undecided configuration is some 40 us of
+// latency on one warp (a 7-link FP64 chain, cold instructions), so thousands of
+// them need many warps: 2,000 of 660,000 positions took 315 us on two warps per SM.
+constexpr int kResolveWarps = 2, kResolveCtas = 6;
 
 static size_t smem_pass(const ArmDev& s, int warps, bool with64) {
   return table_bytes(s) + (size_t)warps * (warp32_bytes(s) + (with64 ? warp64_bytes(s) : 0));
@@ -1576,8 +1611,8 @@ cudaError_t arm_configs(const ArmDev& s, const void* q, int dtype, long long n, 
   int grid = (int)std::max(1ll, std::min(want, (long long)ls.ctas));
   cudaError_t e = launch_configs<false>(s, gpl, q, dtype, n, out, sc, grid, ls.warps, smem1, full, st);
   if (e != cudaSuccess) return e;
-  const int w2 = 2;
-  return launch_configs<true>(s, gpl, q, dtype, n, out, sc, ls.num_sms, w2, smem_pass(s, w2, true), 0, st);
+  return launch_configs<true>(s, gpl, q, dtype, n, out, sc, ls.num_sms * kResolveCtas, kResolveWarps,
+                              smem_pass(s, kResolveWarps, true), 0, st);
 }
 
 cudaError_t arm_edges(const ArmDev& s, const void* q1, const void* q2, int dtype, long long n,
@@ -1600,9 +1635,8 @@ cudaError_t arm_edges(const ArmDev& s, const void* q1, const void* q2, int dtype
   e = launch_phase_b(s, gpl, q1, q2, dtype, incl, sc, ls.ctas, ls.warps, smem1, full, s.phase_b1, -1, out, ls.num_sms,
                      st);
   if (e != cudaSuccess) return e;
-  const int w2 = 2;
-  return launch_edges<true>(s, gpl, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, sc, ls.num_sms,
-                            w2, smem_pass(s, w2, true), 0, st);
+  return launch_edges<true>(s, gpl, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, sc,
+                            ls.num_sms * kResolveCtas, kResolveWarps, smem_pass(s, kResolveWarps, true), 0, st);
 }
 
 bool arm_small_ok(const ArmDev& s) {

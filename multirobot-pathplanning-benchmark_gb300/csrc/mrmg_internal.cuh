@@ -133,6 +133,7 @@ struct PenParams {
 // queue (64-bit), [10] finished CTAs of the last phase-B launch
 constexpr int kCtrQueue = 0, kCtrPending = 1, kCtrErr = 2, kCtrQueue2 = 3, kCtrStat0 = 4;
 constexpr int kCtrL1 = 6, kCtrMaxJ = 7, kCtrQueueB = 8;
+constexpr int kCtrPendLost = 11;   // pending positions did not fit the list
 constexpr int kCtrDoneB = 10;   // CTAs of the last phase-B launch that have finished
 constexpr int kNumCtr = 16;
 
@@ -142,7 +143,7 @@ struct SurvivorEdge {
   long long e;
   int N, p_next, nmax;
   int dead;      // a remaining configuration collides
-  int pend;      // a configuration needs the exact FP64 pass
+  int pend;      // an undecided position did not fit the pending list: pass 2 walks the edge
   int pad;
 };
 
