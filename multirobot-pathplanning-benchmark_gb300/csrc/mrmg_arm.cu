@@ -792,7 +792,8 @@ __device__ __forceinline__ void warp_areas(const ArmDev& s, unsigned char* smem_
 
 template <int GPL, int SPG, bool RESOLVE>
 __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ? 2 : 1))) arm_configs_kernel(ArmDev s, const void* q, int dtype, long long n,
-                                                          uint8_t* out, int* ctr, long long* pend, int full) {
+                                                          uint8_t* out, int* ctr, long long* pend, const SurvivorEdge* list,
+                                                          int full) {
   // pass 2: as many CTAs stay as there are undecided items for their warps
   if (RESOLVE && (long long)blockIdx.x * (blockDim.x >> 5) >= ctr[kCtrPending]) return;
   extern __shared__ __align__(16) unsigned char smem_arm[];
@@ -805,13 +806,15 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
   const int D = s.D;
   while (true) {
     long long k0 = 0;
-    if (lane == 0) k0 = atomicAdd(&ctr[RESOLVE ? kCtrQueue2 : kCtrQueue], RESOLVE ? 1 : s.cfg_chunk);
+    // what the scan left is few and mostly free: one at a time
+    const int take = RESOLVE || list ? 1 : s.cfg_chunk;
+    if (lane == 0) k0 = atomicAdd(&ctr[RESOLVE ? kCtrQueue2 : kCtrQueue], take);
     k0 = __shfl_sync(MRMG_FULL, k0, 0);
-    const long long lim = RESOLVE ? (long long)ctr[kCtrPending] : n;
+    const long long lim = RESOLVE ? (long long)ctr[kCtrPending] : (list ? (long long)ctr[kCtrListed] : n);
     if (k0 >= lim) break;
-    const int cnt = RESOLVE ? 1 : (int)min((long long)s.cfg_chunk, lim - k0);
+    const int cnt = (int)min((long long)take, lim - k0);
     for (int c = 0; c < cnt; c++) {
-      const long long i = RESOLVE ? pend[k0] : k0 + c;
+      const long long i = RESOLVE ? pend[k0] : (list ? (long long)list[k0 + c].pad : k0 + c);
       const CfgSource src{q, dtype, i, D};
       uint8_t v = eval_config<GPL, SPG, RESOLVE>(s, t, wcs, wqv, wsph, w64, lane, src, full != 0);
       if (lane == 0) {
@@ -918,7 +921,8 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
                                                         long long n, double res, int incl,
                                                         const long long* Np, long long N_start,
                                                         long long N_max, uint8_t* out, int* ctr,
-                                                        long long* pend, long long pend_cap, SurvivorEdge* surv, int full) {
+                                                        long long* pend, long long pend_cap, SurvivorEdge* surv, int listed,
+                                                        int full) {
   // pass 2: as many CTAs stay as there are undecided items for their warps
   if (RESOLVE && (long long)blockIdx.x * (blockDim.x >> 5) >= ctr[kCtrPending]) return;
   extern __shared__ __align__(16) unsigned char smem_arm[];
@@ -954,8 +958,8 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
         e = sv.e;
       }
     } else {
-      if (k >= n) break;
-      e = k;
+      if (k >= (listed ? (long long)ctr[kCtrListed] : n)) break;
+      e = listed ? (long long)surv[k].pad : k;
     }
     EdgeSourceDF sdf;
     float mloc;
@@ -995,10 +999,9 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
           } else if (p + 1 < nmax) {
             if (lane == 0) {
               const int slot = atomicAdd(&ctr[kCtrL1], 1);
-              SurvivorEdge sv;
-              sv.e = e; sv.N = (int)N; sv.p_next = (int)(p + 1); sv.nmax = (int)nmax;
-              sv.dead = code == V_COLLIDE; sv.pend = 0; sv.pad = 0;
-              surv[slot] = sv;
+              SurvivorEdge* sv = surv + slot;   // (pad holds a listed edge that may not be read yet)
+              sv->e = e; sv->N = (int)N; sv->p_next = (int)(p + 1); sv->nmax = (int)nmax;
+              sv->dead = code == V_COLLIDE; sv->pend = 0;
               // phase A adds at most one entry per edge: the list has room
               if (code == V_PENDING) pend[atomicAdd(&ctr[kCtrPending], 1)] = pend_entry(e, kPendBfs | (int)(p + 1));
               atomicMax(&ctr[kCtrMaxJ], (int)(nmax - p - 1));
@@ -1172,6 +1175,331 @@ __global__ void __launch_bounds__(256, GPL == 1 ? 3 : (GPL == 2 ? 2 : 1)) arm_ed
 }
 
 
+
+// ---------------------------------------------------------------------------
+// Scan: a first pass of large batches over stored configurations, or the first
+// checked position of edges, that finds the certain box collisions.  A lane per
+// (configuration, robot) walks its robot's chain group by group with the frame in
+// registers, tests each group's bound against every box the group can reach and
+// the spheres of near groups, and the configuration ends at the first collision
+// of any of its robots: in a cluttered scene after two or three links, where the
+// warp-per-configuration kernels place every sphere of every robot first.  What
+// does not collide (or the FP32 path cannot decide) is listed for those kernels,
+// which evaluate it from the start, so verdicts do not depend on this pass.
+//
+// The robots of a configuration sit in adjacent lanes (32 / R configurations per
+// warp); a warp takes new ones from the queue when half of its places are free,
+// which keeps the set-up (an edge's step count, base frames) to dense rounds.
+// ---------------------------------------------------------------------------
+constexpr int kScanThreads = 128;
+constexpr int kMaxScanMask = 16384;   // (group, box) reach tests per CTA, at most; beyond: every box is tested
+
+__host__ __device__ inline size_t scan_smem(const ArmDev& s) {
+  return table_bytes(s) + align16(sizeof(float4) * 3 * ((s.B + 1) / 2)) + align16(sizeof(uint32_t) * s.G * ((s.B + 31) / 32));
+}
+
+// one joint of an edge (or of a stored configuration) as a double-float
+template <bool EDGES>
+__device__ __forceinline__ void scan_joint(const void* q1, const void* q2, int dtype, long long at, float fi, float nm1,
+                                           float rn, float* h, float* l) {
+  if (!EDGES) {
+    if (dtype == MRMG_F32) {
+      *h = ((const float*)q1)[at];
+      *l = 0.f;
+    } else {
+      const double x = ((const double*)q1)[at];
+      *h = (float)x;
+      *l = (float)__dsub_rn(x, (double)*h);
+    }
+    return;
+  }
+  float ah, al = 0.f, dh, dl;
+  if (dtype == MRMG_F32) {
+    const float b = ((const float*)q2)[at];
+    ah = ((const float*)q1)[at];
+    two_sum(b, -ah, &dh, &dl);
+  } else {
+    const double a = ((const double*)q1)[at], b = ((const double*)q2)[at], d = __dsub_rn(b, a);
+    ah = (float)a;
+    al = (float)__dsub_rn(a, (double)ah);
+    dh = (float)d;
+    dl = (float)__dsub_rn(d, (double)dh);
+  }
+  interp_df(ah, al, dh, dl, fi, nm1, rn, h, l);
+}
+
+template <int SPG, bool EDGES>
+__global__ void __launch_bounds__(kScanThreads, 5) arm_scan_kernel(ArmDev s, const void* q1, const void* q2, int dtype,
+                                                                   long long n, float res32, int incl,
+                                                                   const long long* Np, long long N_start,
+                                                                   long long N_max, uint8_t* out, int* ctr,
+                                                                   SurvivorEdge* surv) {
+  extern __shared__ __align__(16) unsigned char smem_arm[];
+  __shared__ int s_gbeg[kMaxRobots + 1], s_joint[kMaxRobots];
+  ArmSmem t;
+  stage_tables(s, smem_arm, &t);
+  float4* bp = (float4*)(smem_arm + table_bytes(s));   // boxes in pairs: centre x x y y, z z / half x x, y y z z
+  const int nw = (s.B + 31) / 32, np2 = (s.B + 1) / 2;
+  uint32_t* reach = (uint32_t*)(bp + 3 * np2);         // [G][nw]: boxes within the group's reach
+  __syncthreads();
+  if (threadIdx.x <= s.R) {
+    int c = 0;
+    for (int g = 0; g < s.G; g++) c += (t.grp[g] & 0xff) < (int)threadIdx.x;
+    s_gbeg[threadIdx.x] = c;   // groups are in robot order
+    if (threadIdx.x < s.R) s_joint[threadIdx.x] = s.q_off[threadIdx.x] + (s.base_kind[threadIdx.x] == 1 ? 3 : 0);
+  }
+  for (int i = threadIdx.x; i < np2; i += kScanThreads) {
+    const int b1 = min(2 * i + 1, s.B - 1);
+    const float4 c0 = t.box[4 * i], h0 = t.box[4 * i + 1], c1 = t.box[2 * b1], h1 = t.box[2 * b1 + 1];
+    bp[3 * i] = make_float4(-c0.x, -c1.x, -c0.y, -c1.y);
+    bp[3 * i + 1] = make_float4(-c0.z, -c1.z, -h0.x, -h1.x);
+    bp[3 * i + 2] = make_float4(-h0.y, -h1.y, -h0.z, -h1.z);
+  }
+  const bool cull = s.G * s.B <= kMaxScanMask;
+  for (int i = threadIdx.x; i < s.G * nw; i += kScanThreads) {
+    const int g = i / nw, b0 = (i - g * nw) * 32, nb = min(32, s.B - b0);
+    const int r = t.grp[g] & 0xff, k = t.grp[g] >> 8;
+    uint32_t m = nb >= 32 ? 0xffffffffu : (1u << nb) - 1u;
+    if (cull && s.base_kind[r] == 0) {
+      // a fixed base: the group stays within this distance of it (FP32 rounding: the last factor)
+      const float4 lb = t.gbs[g];
+      float d = sqrtf(fmaf(lb.z, lb.z, fmaf(lb.y, lb.y, lb.x * lb.x))) + sqrtf(fmaxf(lb.w, 0.f));
+      for (int j = 0; j < k; j++) {
+        const float4 h = t.dh[r * kMaxLinks + j];
+        d += sqrtf(fmaf(h.x, h.x, h.y * h.y));
+      }
+      d *= 1.0001f;
+      const float px = t.base[3 * r].w, py = t.base[3 * r + 1].w, pz = t.base[3 * r + 2].w;
+      m = 0u;
+      for (int b = 0; b < nb; b++) {
+        const float4 bc = t.box[2 * (b0 + b)], bh = t.box[2 * (b0 + b) + 1];
+        const float ex = fmaxf(fabsf(px - bc.x) - bh.x, 0.f), ey = fmaxf(fabsf(py - bc.y) - bh.y, 0.f);
+        const float ez = fmaxf(fabsf(pz - bc.z) - bh.z, 0.f);
+        if (fmaf(ez, ez, fmaf(ey, ey, ex * ex)) <= d * d) m |= 1u << b;
+      }
+    }
+    reach[i] = m;
+  }
+  __syncthreads();
+
+  const int lane = threadIdx.x & 31, R = s.R, D = s.D;
+  const int places = 32 / R, place = lane / R, r = lane - place * R;   // configurations per warp; this lane's robot
+  const bool used = place < places;
+  const unsigned gmask = used ? ((1u << R) - 1u) << (place * R) : 0u;
+  const unsigned lead = used && r == 0 ? 1u : 0u;
+  long long idx = -1;         // this place's configuration or edge
+  int g = 0, gend = 0, kc = 0;
+  float fr[9], p[3], fi = 0.f, nm1 = 1.f, rn = 1.f;
+  bool bad = false, exhausted = false;
+  long long stat_cfg = 0;
+  while (true) {
+    // ---- new configurations for the free places
+    const unsigned idle = __ballot_sync(MRMG_FULL, used && idx < 0);
+    const int free_places = __popc(idle) / R;
+    if (!exhausted && 2 * free_places >= places) {
+      long long base = 0;
+      if (lane == 0) base = atomicAdd(&ctr[kCtrScan], free_places);
+      base = __shfl_sync(MRMG_FULL, base, 0);
+      exhausted = base + free_places >= n;
+      const bool fresh = used && idx < 0;
+      bool none = false;      // an edge with no checked position: free
+      if (fresh) {
+        const long long c = base + __popc(idle & ((1u << (place * R)) - 1u)) / R;
+        if (c < n) {
+          idx = c;
+          bad = false;
+          kc = 0;
+          g = s_gbeg[r];
+          gend = (s.robot_mask >> r) & 1u ? s_gbeg[r + 1] : g;
+        }
+      }
+      if (EDGES) {
+        float m = 0.f;
+        bool nanf = false;
+        if (fresh && idx >= 0 && !Np)
+          for (int j = r; j < D; j += R) {
+            float dh;
+            if (dtype == MRMG_F32) dh = __fsub_rn(((const float*)q2)[idx * D + j], ((const float*)q1)[idx * D + j]);
+            else dh = (float)__dsub_rn(((const double*)q2)[idx * D + j], ((const double*)q1)[idx * D + j]);
+            nanf |= dh != dh;
+            m = fmaxf(m, fabsf(dh));
+          }
+        float mg = m;
+        for (int o = 1; o < R; o++) {   // the place's largest step
+          int from = r + o;
+          from -= from >= R ? R : 0;
+          mg = fmaxf(mg, __shfl_sync(MRMG_FULL, m, used ? place * R + from : lane));
+        }
+        const bool anynan = (__ballot_sync(MRMG_FULL, nanf) & gmask) != 0u;
+        if (fresh && idx >= 0) {
+          long long N = 0;
+          bool ok = true;
+          if (Np) N = Np[idx];
+          else ok = steps_fp32(mg, anynan, res32, &N);
+          ok = ok && N >= 0 && N_start <= N && N <= (1ll << 24);
+          if (!ok) {
+            bad = true;   // the edge kernel counts the steps in FP64 or reports the error
+          } else {
+            const int nmax = (int)((N_max < 0 || N_max > N) ? N : N_max);
+            int iv = -1;
+            for (int q = (int)N_start; q < nmax; q++) {
+              const int c = bfs_at32((int)N, q);
+              if (incl || (c != 0 && c != (int)N - 1)) { iv = c; break; }
+            }
+            none = iv < 0;
+            nm1 = (float)((int)N - 1);
+            rn = __frcp_rn(nm1);
+            fi = (float)iv;
+          }
+        }
+      }
+      if (fresh && idx >= 0 && !bad && !none) {
+        const float4 b0 = t.base[r * 3 + 0], b1 = t.base[r * 3 + 1], b2 = t.base[r * 3 + 2];
+        if (s_joint[r] != s.q_off[r]) {   // planar base: T(x, y) Rz(theta) times the mount
+          float v[3], h, l, cs, sn;
+          const long long at = idx * D + s_joint[r] - 3;
+          for (int i = 0; i < 3; i++) {
+            scan_joint<EDGES>(q1, q2, dtype, at + i, fi, nm1, rn, &h, &l);
+            if (i < 2) {
+              v[i] = __fadd_rn(h, l);
+              bad |= !(fabsf(h) <= s.xy_max);
+            } else {
+              add_offset_df(s, s_joint[r] - 1, &h, &l);
+              bad |= !reduce_df(h, l, &v[2]);
+            }
+          }
+          sincosf(v[2], &sn, &cs);
+          fr[0] = cs * b0.x - sn * b1.x; fr[1] = cs * b0.y - sn * b1.y; fr[2] = cs * b0.z - sn * b1.z;
+          fr[3] = sn * b0.x + cs * b1.x; fr[4] = sn * b0.y + cs * b1.y; fr[5] = sn * b0.z + cs * b1.z;
+          fr[6] = b2.x; fr[7] = b2.y; fr[8] = b2.z;
+          p[0] = v[0] + (cs * b0.w - sn * b1.w);
+          p[1] = v[1] + (sn * b0.w + cs * b1.w);
+          p[2] = b2.w;
+        } else {
+          fr[0] = b0.x; fr[1] = b0.y; fr[2] = b0.z; p[0] = b0.w;
+          fr[3] = b1.x; fr[4] = b1.y; fr[5] = b1.z; p[1] = b1.w;
+          fr[6] = b2.x; fr[7] = b2.y; fr[8] = b2.z; p[2] = b2.w;
+        }
+      }
+      if (none) {
+        if (lead) out[idx] = V_FREE;
+        idx = -1;
+      }
+    }
+    const unsigned live = __ballot_sync(MRMG_FULL, used && idx >= 0);
+    if (!live) {
+      if (exhausted) break;
+      continue;
+    }
+
+    // ---- the next group of this lane's robot: advance the chain to its link
+    bool hit = false;
+    const bool go = idx >= 0 && !bad && g < gend;
+    const int link = go ? t.grp[g] >> 8 : 0;
+    while (__any_sync(MRMG_FULL, go && kc < link && !bad)) {
+      if (go && kc < link && !bad) {
+        const int j = s_joint[r] + kc;
+        float h, l, a, sn, c;
+        scan_joint<EDGES>(q1, q2, dtype, idx * D + j, fi, nm1, rn, &h, &l);
+        add_offset_df(s, j, &h, &l);
+        bad = !reduce_df(h, l, &a);
+        sincosf(a, &sn, &c);
+        const float4 hd = t.dh[r * kMaxLinks + kc];
+        const float sca = sn * hd.z, cca = c * hd.z, ssa = sn * hd.w, csa = c * hd.w;
+        const float ac = hd.x * c, as = hd.x * sn;
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          const float r0 = fr[3 * i], r1 = fr[3 * i + 1], r2 = fr[3 * i + 2];
+          fr[3 * i] = r0 * c + r1 * sn;
+          fr[3 * i + 1] = r1 * cca - r0 * sca + r2 * hd.w;
+          fr[3 * i + 2] = r0 * ssa - r1 * csa + r2 * hd.z;
+          p[i] = p[i] + (r0 * ac + r1 * as + r2 * hd.y);
+        }
+        kc++;
+      }
+    }
+    // ---- its bound against the boxes in reach, then the spheres against the near ones
+    const bool test = go && !bad;
+    float gx = 0.f, gy = 0.f, gz = 0.f, nr2 = 1.f;
+    if (test) {
+      const float4 lb = t.gbs[g];
+      gx = p[0] + (fr[0] * lb.x + fr[1] * lb.y + fr[2] * lb.z);
+      gy = p[1] + (fr[3] * lb.x + fr[4] * lb.y + fr[5] * lb.z);
+      gz = p[2] + (fr[6] * lb.x + fr[7] * lb.y + fr[8] * lb.z);
+      nr2 = -lb.w;   // (positive for a group without spheres: never near)
+    }
+    float cx[SPG], cy[SPG], cz[SPG], rl[SPG];
+    bool placed = false;
+    for (int w = 0; w < nw; w++) {
+      const uint32_t in = test ? reach[g * nw + w] : 0u;
+      const uint32_t any = __reduce_or_sync(MRMG_FULL, in);
+      uint32_t near = 0u;
+      const float2 x2 = make_float2(gx, gx), y2 = make_float2(gy, gy), z2 = make_float2(gz, gz);
+      for (uint32_t pr = (any | any >> 1) & 0x55555555u; pr; pr &= pr - 1) {
+        const int i = __ffs(pr) - 1;
+        const float4* f = bp + 3 * ((32 * w + i) >> 1);
+        const float4 u = f[0], v = f[1], h = f[2];
+        const float2 dx = __fadd2_rn(x2, make_float2(u.x, u.y)), dy = __fadd2_rn(y2, make_float2(u.z, u.w));
+        const float2 dz = __fadd2_rn(z2, make_float2(v.x, v.y));
+        const float2 ex = make_float2(fmaxf(fabsf(dx.x) + v.z, 0.f), fmaxf(fabsf(dx.y) + v.w, 0.f));
+        const float2 ey = make_float2(fmaxf(fabsf(dy.x) + h.x, 0.f), fmaxf(fabsf(dy.y) + h.y, 0.f));
+        const float2 ez = make_float2(fmaxf(fabsf(dz.x) + h.z, 0.f), fmaxf(fabsf(dz.y) + h.w, 0.f));
+        const float2 e2 = __ffma2_rn(ez, ez, __ffma2_rn(ey, ey, __ffma2_rn(ex, ex, make_float2(nr2, nr2))));
+        if (e2.x <= 0.f) near |= 1u << i;
+        if (e2.y <= 0.f) near |= 2u << i;
+      }
+      near &= in;
+      if (!__any_sync(MRMG_FULL, near != 0u && !hit)) continue;
+      if (!placed) {
+        placed = true;
+        if (test) {
+#pragma unroll
+          for (int v = 0; v < SPG; v++) {
+            const float4 l = t.sph[g * SPG + v];
+            cx[v] = p[0] + (fr[0] * l.x + fr[1] * l.y + fr[2] * l.z);
+            cy[v] = p[1] + (fr[3] * l.x + fr[4] * l.y + fr[5] * l.z);
+            cz[v] = p[2] + (fr[6] * l.x + fr[7] * l.y + fr[8] * l.z);
+            rl[v] = t.band[g * SPG + v].x;   // below: a certain collision (padding: -1)
+          }
+        }
+      }
+      while (__any_sync(MRMG_FULL, near != 0u && !hit)) {
+        if (near != 0u && !hit) {
+          const int b = 32 * w + __ffs(near) - 1;
+          near &= near - 1;
+          const float4 bc = t.box[2 * b], bh = t.box[2 * b + 1];
+#pragma unroll
+          for (int v = 0; v < SPG; v++) {
+            const float ex = fmaxf(fabsf(cx[v] - bc.x) - bh.x, 0.f);
+            const float ey = fmaxf(fabsf(cy[v] - bc.y) - bh.y, 0.f);
+            const float ez = fmaxf(fabsf(cz[v] - bc.z) - bh.z, 0.f);
+            hit |= fmaf(ez, ez, fmaf(ey, ey, ex * ex)) < rl[v];
+          }
+        }
+      }
+    }
+    if (go) g++;
+
+    // ---- a collision ends the configuration; one that has tested every group is listed
+    const unsigned hits = __ballot_sync(MRMG_FULL, hit), bads = __ballot_sync(MRMG_FULL, idx >= 0 && bad);
+    const unsigned more = __ballot_sync(MRMG_FULL, idx >= 0 && g < gend);
+    const bool dead = (hits & gmask) != 0u;
+    const bool list = idx >= 0 && !dead && ((bads & gmask) != 0u || (more & gmask) == 0u);
+    const unsigned lists = __ballot_sync(MRMG_FULL, list && lead);
+    if (dead && lead) {
+      out[idx] = V_COLLIDE;
+      stat_cfg++;
+    }
+    if (lists) {
+      int slot = 0;
+      if (lane == 0) slot = atomicAdd(&ctr[kCtrListed], __popc(lists));
+      slot = __shfl_sync(MRMG_FULL, slot, 0);
+      if (list && lead) surv[slot + __popc(lists & ((1u << lane) - 1u))].pad = (int)idx;
+    }
+    if (dead || list) idx = -1;
+  }
+  if (EDGES && stat_cfg) atomicAdd((unsigned long long*)&ctr[kCtrStat0], (unsigned long long)stat_cfg);
+}
 
 // ---------------------------------------------------------------------------
 // Small synchronous batches (a planner's single is_collision_free /
@@ -1478,11 +1806,12 @@ __global__ void arm_box_hits_kernel(ArmDev s, const void* q, int dtype, long lon
 // ---------------------------------------------------------------------------
 template <bool RESOLVE>
 cudaError_t launch_configs(const ArmDev& s, int gpl, const void* q, int dtype, long long n, uint8_t* out,
-                           const CallScratch& sc, int grid, int warps, size_t smem, int full, cudaStream_t st) {
+                           const CallScratch& sc, int grid, int warps, size_t smem, int full, int listed, cudaStream_t st) {
 #define MRMG_ARM_CFG(G_, S_)                                                                       \
   if (gpl == G_ && s.SPG == S_) {                                                                  \
     auto k = arm_configs_kernel<G_, S_, RESOLVE>;                                                  \
-    k<<<grid, warps * 32, smem, st>>>(s, q, dtype, n, out, sc.ctr, sc.pend, full);                 \
+    k<<<grid, warps * 32, smem, st>>>(s, q, dtype, n, out, sc.ctr, sc.pend,                         \
+                                      listed ? sc.surv : nullptr, full);                            \
     return cudaGetLastError();                                                                     \
   }
   MRMG_ARM_CFG(1, 6)
@@ -1495,13 +1824,13 @@ cudaError_t launch_configs(const ArmDev& s, int gpl, const void* q, int dtype, l
 template <bool RESOLVE>
 cudaError_t launch_edges(const ArmDev& s, int gpl, const void* q1, const void* q2, int dtype, long long n,
                          double res, int incl, const long long* Np, long long N_start, long long N_max,
-                         uint8_t* out, const CallScratch& sc, int grid, int warps, size_t smem, int full,
+                         uint8_t* out, const CallScratch& sc, int grid, int warps, size_t smem, int full, int listed,
                          cudaStream_t st) {
 #define MRMG_ARM_EDGE(G_, S_)                                                                      \
   if (gpl == G_ && s.SPG == S_) {                                                                  \
     auto k = arm_edges_kernel<G_, S_, RESOLVE>;                                                    \
     k<<<grid, warps * 32, smem, st>>>(s, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out,     \
-                                      sc.ctr, sc.pend, sc.pend_cap, sc.surv, full);                             \
+                                      sc.ctr, sc.pend, sc.pend_cap, sc.surv, listed, full);                             \
     return cudaGetLastError();                                                                     \
   }
   MRMG_ARM_EDGE(1, 6)
@@ -1589,6 +1918,8 @@ int arm_prepare(const ArmDev& s, int warps) {
     allow_max_smem(arm_configs_kernel<G_, S_, true>);                                              \
     allow_max_smem(arm_edges_phase_b<G_, S_>);                                                     \
     allow_max_smem(arm_small_kernel<G_, S_>);                                                      \
+    allow_max_smem(arm_scan_kernel<S_, false>);                                                    \
+    allow_max_smem(arm_scan_kernel<S_, true>);                                                     \
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, arm_edges_kernel<G_, S_, false>, warps * 32, \
                                                         smem_pass(s, warps, false));              \
   }
@@ -1603,16 +1934,52 @@ int arm_prepare(const ArmDev& s, int warps) {
   return blocks;
 }
 
+// The scan adds a pass of some 40 us of latency (seven links, one after another)
+// and pays where most configurations collide with a box and there are enough of
+// them for its lanes.  Measured, four arms, uniform configurations (before -> with
+// the scan): 200,000 among 50, 36, 22, 20 boxes 309 -> 197, 334 -> 230, 344 ->
+// 249, 378 -> 351 us, among 5 boxes 417 -> 499 us; 40,000 among 50, 36, 22 146 ->
+// 141, 146 -> 149, 157 -> 146 us; 10,000 among 50 89 -> 105 us.
+constexpr long long kScanMinLanes = 1ll << 18;
+constexpr int kScanMinBoxes = 16;
+static bool use_scan(const ArmDev& s, long long n, int full) {
+  return !full && s.B >= kScanMinBoxes && n * s.R >= kScanMinLanes && n < (1ll << 31) &&
+         scan_smem(s) <= (size_t)100 * 1024;
+}
+
+template <bool EDGES>
+static cudaError_t launch_scan(const ArmDev& s, const void* q1, const void* q2, int dtype, long long n, double res,
+                               int incl, const long long* Np, long long N_start, long long N_max, uint8_t* out,
+                               const CallScratch& sc, int num_sms, cudaStream_t st) {
+  const size_t smem = scan_smem(s);
+  const int per_cta = kScanThreads / 32 * (32 / s.R);
+  const int grid = (int)std::max(1ll, std::min((n + per_cta - 1) / per_cta, (long long)num_sms * 5));
+#define MRMG_ARM_SCAN(S_)                                                                          \
+  if (s.SPG == S_) {                                                                               \
+    arm_scan_kernel<S_, EDGES><<<grid, kScanThreads, smem, st>>>(s, q1, q2, dtype, n, (float)res, incl, Np, N_start, \
+                                                                 N_max, out, sc.ctr, sc.surv);     \
+    return cudaGetLastError();                                                                     \
+  }
+  MRMG_ARM_SCAN(6)
+  MRMG_ARM_SCAN(5)
+  MRMG_ARM_SCAN(8)
+#undef MRMG_ARM_SCAN
+  return cudaErrorInvalidValue;
+}
+
 cudaError_t arm_configs(const ArmDev& s, const void* q, int dtype, long long n, uint8_t* out,
                         const CallScratch& sc, const LaunchShape& ls, int full, cudaStream_t st) {
   const int gpl = arm_gpl_for_spg(s.SPG);
   const size_t smem1 = smem_pass(s, ls.warps, false);
   long long want = (n + (long long)ls.warps * s.cfg_chunk - 1) / ((long long)ls.warps * s.cfg_chunk);
   int grid = (int)std::max(1ll, std::min(want, (long long)ls.ctas));
-  cudaError_t e = launch_configs<false>(s, gpl, q, dtype, n, out, sc, grid, ls.warps, smem1, full, st);
+  const bool scan = use_scan(s, n, full);
+  cudaError_t e = cudaSuccess;
+  if (scan) e = launch_scan<false>(s, q, nullptr, dtype, n, 0.0, 0, nullptr, 0, -1, out, sc, ls.num_sms, st);
+  if (e == cudaSuccess) e = launch_configs<false>(s, gpl, q, dtype, n, out, sc, grid, ls.warps, smem1, full, scan, st);
   if (e != cudaSuccess) return e;
   return launch_configs<true>(s, gpl, q, dtype, n, out, sc, ls.num_sms * kResolveCtas, kResolveWarps,
-                              smem_pass(s, kResolveWarps, true), 0, st);
+                              smem_pass(s, kResolveWarps, true), 0, 0, st);
 }
 
 cudaError_t arm_edges(const ArmDev& s, const void* q1, const void* q2, int dtype, long long n,
@@ -1623,8 +1990,12 @@ cudaError_t arm_edges(const ArmDev& s, const void* q1, const void* q2, int dtype
   const size_t smem1 = smem_pass(s, ls.warps, false);
   long long want = (n + ls.warps - 1) / ls.warps;
   int grid = (int)std::max(1ll, std::min(want, (long long)ls.ctas));
-  cudaError_t e = launch_edges<false>(s, gpl, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, sc,
-                                      grid, ls.warps, smem1, full, st);
+  const bool scan = use_scan(s, n, full);
+  cudaError_t e = cudaSuccess;
+  if (scan) e = launch_scan<true>(s, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, sc, ls.num_sms, st);
+  if (e == cudaSuccess)
+    e = launch_edges<false>(s, gpl, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, sc, grid, ls.warps, smem1,
+                            full, scan, st);
   if (e != cudaSuccess) return e;
   // B1: the next s.phase_b1 positions of every survivor (kills most colliding
   // survivors); B2: everything left, spread over all warps
@@ -1636,7 +2007,7 @@ cudaError_t arm_edges(const ArmDev& s, const void* q1, const void* q2, int dtype
                      st);
   if (e != cudaSuccess) return e;
   return launch_edges<true>(s, gpl, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, sc,
-                            ls.num_sms * kResolveCtas, kResolveWarps, smem_pass(s, kResolveWarps, true), 0, st);
+                            ls.num_sms * kResolveCtas, kResolveWarps, smem_pass(s, kResolveWarps, true), 0, 0, st);
 }
 
 bool arm_small_ok(const ArmDev& s) {

@@ -133,6 +133,7 @@ struct PenParams {
 // queue (64-bit), [10] finished CTAs of the last phase-B launch
 constexpr int kCtrQueue = 0, kCtrPending = 1, kCtrErr = 2, kCtrQueue2 = 3, kCtrStat0 = 4;
 constexpr int kCtrL1 = 6, kCtrMaxJ = 7, kCtrQueueB = 8;
+constexpr int kCtrScan = 12, kCtrListed = 13;   // scan: its queue, and the items listed for the warp kernels
 constexpr int kCtrPendLost = 11;   // pending positions did not fit the list
 constexpr int kCtrDoneB = 10;   // CTAs of the last phase-B launch that have finished
 constexpr int kNumCtr = 16;
@@ -144,7 +145,7 @@ struct SurvivorEdge {
   int N, p_next, nmax;
   int dead;      // a remaining configuration collides
   int pend;      // an undecided position did not fit the pending list: pass 2 walks the edge
-  int pad;
+  int pad;       // (of entry k: the k-th item the scan listed)
 };
 
 struct CallScratch {
