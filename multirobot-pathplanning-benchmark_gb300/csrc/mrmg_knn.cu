@@ -148,14 +148,66 @@ __device__ __forceinline__ RadiusTest radius_test(double rp) {
   return r;
 }
 
+// FP32 rows of whole 16-byte words, up to 32 coordinates, whose agents' slices
+// follow one another from 0 to D: n4 words and the agents' last coordinates as
+// bits.  Such a row is loaded at once (eight independent 16-byte loads) instead of
+// coordinate by coordinate, each load of which waits some 300 ns for L2.
+struct RowPlan {
+  int n4;          // 0: rows are read coordinate by coordinate
+  unsigned ends;
+};
+inline RowPlan row_plan(const SliceTab& t, int metric) {
+  RowPlan p{0, 0u};
+  if (t.D > 32 || t.D % 4) return p;
+  if (metric == MRMG_METRIC_EUCLIDEAN) {
+    if (t.end_all != t.D) return p;
+    p.ends = 1u << (t.D - 1);
+  } else if (metric == MRMG_METRIC_MAX_EUCLIDEAN) {
+    int at = 0;
+    for (int a = 0; a < t.A; a++) {
+      if (t.s[a] != at || t.e[a] <= at) return RowPlan{0, 0u};
+      at = t.e[a];
+      p.ends |= 1u << (at - 1);
+    }
+    if (at != t.D) return RowPlan{0, 0u};
+  } else {
+    return p;
+  }
+  p.n4 = t.D / 4;
+  return p;
+}
+
 // q32 / x32: FP32 copies (rounded to nearest) of the FP64 rows qq / xx
 __device__ __forceinline__ bool within_radius(const float* __restrict__ q32, const float* __restrict__ x32,
                                               const double* __restrict__ qq, const double* __restrict__ xx,
-                                              const SliceTab& t, int metric, const RadiusTest& r) {
+                                              const SliceTab& t, int metric, const RadiusTest& r, RowPlan rows) {
   if (!(r.rp >= 0.0)) return false;   // distances are >= 0; NaN selects nothing
   if (metric == MRMG_METRIC_EUCLIDEAN || metric == MRMG_METRIC_MAX_EUCLIDEAN) {
     float qn = 0.f, xn = 0.f, m = 0.f;
-    if (metric == MRMG_METRIC_EUCLIDEAN) {
+    if (rows.n4) {
+      float4 x4[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        if (i < rows.n4) x4[i] = __ldg((const float4*)x32 + i);
+      float sa = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        if (i < rows.n4) {
+          const float4 q4 = __ldg((const float4*)q32 + i);
+          const float qv[4] = {q4.x, q4.y, q4.z, q4.w}, xv[4] = {x4[i].x, x4[i].y, x4[i].z, x4[i].w};
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            const float d = qv[k] - xv[k];
+            sa = fmaf(d, d, sa);
+            qn = fmaf(qv[k], qv[k], qn);
+            xn = fmaf(xv[k], xv[k], xn);
+            if ((rows.ends >> (4 * i + k)) & 1u) {
+              m = fmaxf(m, sa);
+              sa = 0.f;
+            }
+          }
+        }
+    } else if (metric == MRMG_METRIC_EUCLIDEAN) {
       for (int k = 0; k < t.end_all; k++) {
         const float qf = q32[k], xf = x32[k], d = qf - xf;
         m = fmaf(d, d, m);
@@ -563,7 +615,7 @@ __global__ void near_split_kernel(const double* __restrict__ qs, const float* __
                                   const float* __restrict__ nodes32, const long long* __restrict__ mode_beg,
                                   const long long* __restrict__ mode_end, SliceTab t, int metric,
                                   const double* __restrict__ rp, const long long* __restrict__ woff,
-                                  unsigned* __restrict__ bits, unsigned long long* __restrict__ counts) {
+                                  unsigned* __restrict__ bits, unsigned long long* __restrict__ counts, RowPlan rows) {
   const int lane = threadIdx.x & 31;
   const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
@@ -576,7 +628,7 @@ __global__ void near_split_kernel(const double* __restrict__ qs, const float* __
     if (id < mode_end[m] - mode_beg[m]) {
       const long long x = mode_beg[m] + id;
       in = within_radius(qs32 + q * t.D, nodes32 + x * t.D, qs + q * t.D, nodes + x * t.D, t, metric,
-                         radius_test(rp[q]));
+                         radius_test(rp[q]), rows);
     }
     const unsigned mk = __ballot_sync(MRMG_FULL, in);
     if (lane == 0) {
@@ -1309,85 +1361,77 @@ __global__ void __launch_bounds__(32 * kMergeWarps, 4) knn_merge_kernel(const do
 // ---------------------------------------------------------------------------
 constexpr int kNearWarps = 4;
 
-// Each warp takes a query and walks its bitmap 32 words (1024 nodes) at a
-// time: the set bits are listed in shared memory and spread over the lanes for
-// the FP64 distance, so a dense word does not serialise one lane.  Bits whose
-// exact distance exceeds the query's r' (or past the mode's nodes) are cleared.
-constexpr int kNearStage = 48;   // results per query staged in order by the exact pass
+// Exact check of the candidate bitmap.  A warp takes 32 consecutive words of all
+// queries' bitmaps (a lane each; most hold no bit), lists their set bits in
+// shared memory and spreads them over the lanes for the radius test, so neither a
+// long bitmap nor a dense word serialises one lane.  Bits that fail (or lie past
+// the mode's nodes) are cleared, the rest counted per query; a query's first
+// kNearStage results to arrive are staged, in any order, for the emit pass.
+// Bound: the candidates' rows from L2 (some 600 candidates per query lie within
+// the tile kernel's error bound of the radius).  2,001 queries on 150,000 nodes,
+// max over agents, 16 results each: 93 us with a warp per query walking its
+// bitmap, 56 us; 300 queries, whole call: 296 -> 228 us, with 11,600 results
+// each 4,910 -> 950 us.
+constexpr int kNearStage = 48;   // results staged per query
 
-__global__ void near_exact_kernel(const double* __restrict__ qs, const float* __restrict__ qs32, long long Q,
+__global__ void __launch_bounds__(32 * kNearWarps, 8) near_exact_kernel(const double* __restrict__ qs, const float* __restrict__ qs32, long long Q,
                                   const int* __restrict__ q_mode, const double* __restrict__ nodes,
                                   const float* __restrict__ nodes32, const long long* __restrict__ mode_beg,
                                   const long long* __restrict__ mode_end, SliceTab t,
                                   int metric, const double* __restrict__ rp, const long long* __restrict__ woff,
-                                  unsigned* __restrict__ bits, long long* __restrict__ counts,
-                                  int* __restrict__ stage) {
-  __shared__ int s_list[kNearWarps][1024];
+                                  unsigned* __restrict__ bits, unsigned long long* __restrict__ counts,
+                                  int* __restrict__ stage, RowPlan rows) {
+  __shared__ unsigned short s_list[kNearWarps][1024];   // word of the 32 and bit
   __shared__ unsigned s_res[kNearWarps][32];
+  __shared__ int s_q[kNearWarps][32];
+  __shared__ long long s_w[kNearWarps][32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const long long warp = (long long)blockIdx.x * kNearWarps + wib;
-  const long long nwarps = (long long)gridDim.x * kNearWarps;
-  int* list = s_list[wib];
-  for (long long q = warp; q < Q; q += nwarps) {
-    const int m = q_mode[q];
-    const long long M = mode_end[m] - mode_beg[m];
-    const double* xb = nodes + mode_beg[m] * t.D;
-    const float* xb32 = nodes32 + mode_beg[m] * t.D;
-    const double* qq = qs + q * t.D;
-    const float* qq32 = qs32 + q * t.D;
-    const long long w0 = woff[q], W = woff[q + 1] - w0;
-    const RadiusTest rt = radius_test(rp[q]);
-    long long cnt = 0;
-    for (long long base = 0; base < W; base += 32) {
-      const long long w = base + lane;
-      const unsigned mk = w < W ? bits[w0 + w] : 0u;
-      const int c = __popc(mk);
-      int incl = c;
+  const long long step = (long long)gridDim.x * kNearWarps * 32;
+  const long long total = woff[Q];
+  unsigned short* list = s_list[wib];
+  for (long long base = ((long long)blockIdx.x * kNearWarps + wib) * 32; base < total; base += step) {
+    const long long f = base + lane;
+    const unsigned mk = f < total ? bits[f] : 0u;
+    if (!__any_sync(MRMG_FULL, mk != 0u)) continue;
+    const int c = __popc(mk);
+    int incl = c;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(MRMG_FULL, incl, o);
-        if (lane >= o) incl += y;
-      }
-      const int n = __shfl_sync(MRMG_FULL, incl, 31);
-      if (n == 0) continue;
-      int pos = incl - c;
-      unsigned mm = mk;
-      while (mm) {
-        const int b = __ffs(mm) - 1;
-        mm &= mm - 1;
-        list[pos++] = lane * 32 + b;
-      }
-      s_res[wib][lane] = 0u;
-      __syncwarp();
-      for (int x = lane; x < n; x += 32) {
-        const int loc = list[x];
-        const long long id = base * 32 + loc;
-        if (id >= M) continue;
-        if (within_radius(qq32, xb32 + id * t.D, qq, xb + id * t.D, t, metric, rt))
-          atomicOr(&s_res[wib][loc >> 5], 1u << (loc & 31));
-      }
-      __syncwarp();
-      const unsigned res = s_res[wib][lane];
-      if (w < W) bits[w0 + w] = res;
-      // stage the first kNearStage results of the query in ascending order
-      const int rc = __popc(res);
-      int ri = rc;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(MRMG_FULL, ri, o);
-        if (lane >= o) ri += y;
-      }
-      long long sp = cnt + ri - rc;
-      unsigned rm = res;
-      while (rm && sp < kNearStage) {
-        const int b = __ffs(rm) - 1;
-        rm &= rm - 1;
-        stage[q * kNearStage + sp++] = (int)((base + lane) * 32 + b);
-      }
-      cnt += __shfl_sync(MRMG_FULL, ri, 31);
-      __syncwarp();
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(MRMG_FULL, incl, o);
+      if (lane >= o) incl += y;
     }
-    if (lane == 0) counts[q] = cnt;   // the same in every lane
+    const int n = __shfl_sync(MRMG_FULL, incl, 31);
+    int pos = incl - c;
+    // the words' queries: one search, then the next query while the word lies past this one
+    long long q = owner_of(woff, Q, base);
+    if (mk) {
+      while (f >= woff[q + 1]) q++;
+      s_q[wib][lane] = (int)q;
+      s_w[wib][lane] = f - woff[q];
+    }
+    for (unsigned mm = mk; mm; mm &= mm - 1) list[pos++] = (unsigned short)(lane * 32 + __ffs(mm) - 1);
+    s_res[wib][lane] = 0u;
+    __syncwarp();
+    for (int x = lane; x < n; x += 32) {
+      const int loc = list[x], w = loc >> 5;
+      const long long qx = s_q[wib][w];
+      const int m = q_mode[qx];
+      const long long id = s_w[wib][w] * 32 + (loc & 31);
+      if (id >= mode_end[m] - mode_beg[m]) continue;
+      const long long xr = (mode_beg[m] + id) * t.D;
+      if (within_radius(qs32 + qx * t.D, nodes32 + xr, qs + qx * t.D, nodes + xr, t, metric, radius_test(rp[qx]),
+                        rows))
+        atomicOr(&s_res[wib][w], 1u << (loc & 31));
+    }
+    __syncwarp();
+    unsigned res = s_res[wib][lane];
+    if (res != mk) bits[f] = res;
+    if (res) {
+      unsigned long long at = atomicAdd(counts + q, (unsigned long long)__popc(res));
+      for (; res && at < kNearStage; res &= res - 1)
+        stage[q * kNearStage + at++] = (int)((f - woff[q]) * 32 + __ffs(res) - 1);
+    }
+    __syncwarp();   // the next words reuse the lists
   }
 }
 
@@ -1436,8 +1480,16 @@ __global__ void near_emit_kernel(long long Q, const long long* __restrict__ woff
     long long o = offs[q];
     const long long nq = offs[q + 1] - o;
     if (o >= cap || nq == 0) continue;
-    if (stage && nq <= kNearStage) {   // staged by the exact pass
-      for (int x = lane; x < nq && o + x < cap; x += 32) out_idx[o + x] = stage[q * kNearStage + x];
+    if (stage && nq <= kNearStage) {   // staged by the exact pass: each result's place is its rank
+      for (int x = lane; x < nq; x += 32) list[x] = stage[q * kNearStage + x];
+      __syncwarp();
+      for (int x = lane; x < nq; x += 32) {
+        const int id = list[x];
+        int rank = 0;
+        for (int y = 0; y < nq; y++) rank += list[y] < id;
+        if (o + rank < cap) out_idx[o + rank] = id;
+      }
+      __syncwarp();
       continue;
     }
     const long long w0 = woff[q], W = woff[q + 1] - w0;
@@ -2293,13 +2345,13 @@ cudaError_t near_query(NearState* ns, KnnStore* s, const double* d_qs, long long
   double* d_rp = (double*)(p + b_order + b_qmode + b_items + b_woff);
   float* d_rad2 = (float*)(p + b_order + b_qmode + b_items + b_woff + b_rp);
   unsigned* d_bits = (unsigned*)(p + b_up);
-  long long* d_cnt = (long long*)(p + b_up + b_bits);
-  long long* d_offs = (long long*)(p + b_up + b_bits + b_cnt);
+  long long* d_offs = (long long*)(p + b_up + b_bits);
+  long long* d_cnt = (long long*)(p + b_up + b_bits + b_offs);
   long long* d_ctr = (long long*)(p + b_up + b_bits + b_cnt + b_offs);   // [0] total, [1] error bits
   float* d_q32 = (float*)(p + b_up + b_bits + b_cnt + b_offs + 256);
   int* d_stage = (int*)(p + b_up + b_bits + b_cnt + b_offs + 256 + b_q32);
   cudaError_t e = cudaMemcpyAsync(p, hp, b_up, cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_ctr, 0, 256, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_cnt, 0, b_cnt + 256, st);   // the counts, then the counters
   if (e == cudaSuccess) e = to_f32(d_qs, d_q32, Q * s->D, st);
   if (e != cudaSuccess) return e;
   if (tc && !pl.items.empty()) {
@@ -2320,16 +2372,18 @@ cudaError_t near_query(NearState* ns, KnnStore* s, const double* d_qs, long long
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   const int grid = near_grid(Q, num_sms);
+  const RowPlan rows = row_plan(t, metric);
   if (tc) {
-    near_exact_kernel<<<grid, 32 * kNearWarps, 0, st>>>(d_qs, d_q32, Q, d_qmode, nodes, s->nodes32, s->d_beg,
-                                                        s->d_end, t, metric, d_rp, d_woff, d_bits, d_cnt, d_stage);
+    const long long blocks = (Wtot + 32 * kNearWarps - 1) / (32 * kNearWarps);
+    if (blocks > 0)
+      near_exact_kernel<<<(int)std::min<long long>(blocks, (long long)num_sms * 12), 32 * kNearWarps, 0, st>>>(
+          d_qs, d_q32, Q, d_qmode, nodes, s->nodes32, s->d_beg, s->d_end, t, metric, d_rp, d_woff, d_bits,
+          (unsigned long long*)d_cnt, d_stage, rows);
   } else {
-    e = cudaMemsetAsync(d_cnt, 0, sizeof(long long) * Q, st);
-    if (e != cudaSuccess) return e;
     if (Wtot > 0) {
       const int g2 = (int)std::min<long long>((Wtot + 3) / 4, (long long)num_sms * 16);
       near_split_kernel<<<g2, 128, 0, st>>>(d_qs, d_q32, Q, d_qmode, nodes, s->nodes32, s->d_beg, s->d_end, t, metric,
-                                            d_rp, d_woff, d_bits, (unsigned long long*)d_cnt);
+                                            d_rp, d_woff, d_bits, (unsigned long long*)d_cnt, rows);
     }
   }
   near_scan_kernel<<<1, 1024, 0, st>>>(d_cnt, Q, d_offsets, d_offs, d_ctr);
