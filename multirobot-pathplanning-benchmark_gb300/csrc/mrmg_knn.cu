@@ -686,9 +686,10 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                : "memory");
 }
 
-// 32 lanes x 32 consecutive FP32 columns of TMEM (warp-wide)
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
+// 32 lanes x 32 consecutive FP32 columns of TMEM (warp-wide): the load, and the
+// wait for every load issued before (the registers hold nothing until then)
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%"
@@ -698,9 +699,21 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
         "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// The registers of a load whose wait has passed, as values: the empty asm keeps
+// every use below the wait.
+__device__ __forceinline__ void tmem_take(uint32_t (&r)[32], float (&v)[32]) {
 #pragma unroll
-  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+  for (int i = 0; i < 32; i++) {
+    asm volatile("" : "+r"(r[i]));
+    v[i] = __uint_as_float(r[i]);
+  }
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
+  uint32_t r[32];
+  tmem_ld32_issue(taddr, r);
+  tmem_ld_wait();
+  tmem_take(r, v);
 }
 
 // shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups
@@ -800,7 +813,7 @@ struct KnnItem {          // one CTA: a query tile of one mode against a chunk o
   int mode, q0, qn;       // queries qorder[q0 .. q0+qn)
   int tile0, tile1;       // node tiles [tile0, tile1) of the mode (mode-local tile index)
   int chunk;              // chunk slot of this item in the candidate lists
-  int pad;
+  int qtile;              // its query tile (packed once, by the item of chunk 0)
 };
 
 struct KnnStoreDev {
@@ -942,7 +955,7 @@ __device__ __forceinline__ unsigned mark32(const float (&v)[32], float t) {
 template <bool FROM_DOT>
 __device__ __forceinline__ void keep_marked(unsigned (&kk)[kKeep], const float (&v)[32], unsigned mk, float qn,
                                             float* cand, int lcol0, unsigned imask) {
-  const int nth = blockDim.x;
+  const int nth = blockDim.x - 32;   // the scanning threads
 #pragma unroll
   for (int i = 0; i < 32; i++) cand[i * nth] = v[i];
   while (mk) {
@@ -979,12 +992,103 @@ __device__ __forceinline__ void rad_chunk(const float (&v)[32], float qn, float 
 
 template <int FMT> struct TcSplit { static constexpr int S = FMT == KNN_FMT_EUCL ? 1 : 2; };
 
+// A packed query tile in global memory: the A1 and A2 operand tiles (SW128, as
+// they lie in shared memory), then per row |q|^2, |q_a|^2 of up to four agents
+// and, for radius queries, the threshold of the approximate squared distance.
+constexpr int kQTileBytes = 2 * kTileM * kRowBytes;
+constexpr int kQTileBlock = kQTileBytes + 6 * kTileM * 4;
+__device__ __forceinline__ const float* qtile_rows(const unsigned char* tile) { return (const float*)(tile + kQTileBytes); }
+
+// Packs the query tiles, a warp per row: A1 = [q_hi | -1/2 ... | q_hi], A2 =
+// [q_lo].  The conversions and norms are FP64 instructions (6 per coordinate), on
+// this part 6.6 us per tile of one SM: done once per tile over the whole GPU (10 us
+// for 39 tiles), not by every CTA that scans another chunk of nodes for it.
+constexpr int kPackRows = 16;   // rows per CTA, a warp each
+__global__ void __launch_bounds__(32 * kPackRows) knn_pack_queries_kernel(
+    KnnStoreDev st, const double* __restrict__ qs, const int* __restrict__ qorder, const KnnItem* __restrict__ tiles,
+    unsigned char* __restrict__ qtiles, float* __restrict__ q_eps, const float* __restrict__ rad2) {
+  const KnnItem it = tiles[blockIdx.x];
+  const int lane = threadIdx.x & 31, r = blockIdx.y * kPackRows + (threadIdx.x >> 5);
+  unsigned char* tile = qtiles + (size_t)it.qtile * kQTileBlock;
+  float* rows = (float*)(tile + kQTileBytes);
+  const int D = st.D;
+  const long long qid = r < it.qn ? qorder[it.q0 + r] : -1;
+  double x = 0.0;
+  if (qid >= 0 && lane < D) x = qs[qid * D + lane];
+  float hi, lo;
+  split2(x, &hi, &lo);
+  float a1[2], a2[2];
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int c = 2 * lane + i;
+    int src = -1;              // the coordinate whose hi part column c holds
+    bool low = false, half = false;
+    if (st.fmt == KNN_FMT_EUCL) {
+      low = c < D;
+      half = c >= D && c < D + 3;
+      src = c < D ? c : (c >= D + 3 && c < 2 * D + 3 ? c - D - 3 : -1);
+    } else if ((c >> 4) < st.A) {
+      const int s = st.agent_s[c >> 4], d = st.agent_e[c >> 4] - s, j = c & 15;
+      low = j < d;
+      half = j == 2 * d || j == 2 * d + 1;
+      src = j < d ? s + j : (j < 2 * d ? s + j - d : -1);
+    }
+    const float vh = __shfl_sync(MRMG_FULL, hi, src & 31), vl = __shfl_sync(MRMG_FULL, lo, src & 31);
+    a1[i] = qid < 0 ? 0.f : (half ? -0.5f : (src >= 0 ? vh : 0.f));
+    a2[i] = qid >= 0 && low ? vl : 0.f;
+  }
+  *(__nv_bfloat162*)(tile + sw128_off(r, 2 * lane)) = __floats2bfloat162_rn(a1[0], a1[1]);
+  *(__nv_bfloat162*)(tile + kTileM * kRowBytes + sw128_off(r, 2 * lane)) = __floats2bfloat162_rn(a2[0], a2[1]);
+  const double x2 = x * x;
+  float qn = 0.f;
+  if (st.fmt == KNN_FMT_EUCL) {
+    double n2 = x2;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) n2 += __shfl_xor_sync(MRMG_FULL, n2, o);
+    qn = (float)n2;
+  } else {
+    // lane a sums agent a's coordinates
+    const int s = lane < st.A ? st.agent_s[lane] : 0, d = lane < st.A ? st.agent_e[lane] - s : 0;
+    int dmax = 0;
+    for (int a = 0; a < st.A; a++) dmax = max(dmax, st.agent_e[a] - st.agent_s[a]);
+    double na = 0.0;
+    for (int j = 0; j < dmax; j++) {
+      const double v = __shfl_sync(MRMG_FULL, x2, (s + j) & 31);
+      if (j < d) na += v;
+    }
+    const float f = (float)na;
+    if (lane < 4) rows[(1 + lane) * kTileM + r] = lane < st.A ? f : 0.f;
+    for (int a = 0; a < st.A; a++) qn += __shfl_sync(MRMG_FULL, f, a);
+  }
+  if (lane == 0) {
+    rows[r] = qn;
+    if (qid >= 0) {
+      // error bound of the approximate squared distance (split-BF16 operands,
+      // FP32 accumulation), per query
+      const float es = sqrtf(qn) + st.mode_xmax[it.mode];
+      const float eps = 1.2e-4f * es * es + 1e-30f;
+      if (q_eps) q_eps[qid] = eps;
+      if (rad2) rows[5 * kTileM + r] = rad2[qid] < 0.f ? -__int_as_float(0x7f800000) : rad2[qid] + 1.0001f * eps;
+    }
+  }
+}
+
+// One CTA per item: 4 S warps scan the accumulators (a row per lane), one more
+// warp feeds them: a lane of it loads node tiles and issues the MMAs, up to two
+// tiles ahead, against barriers -- loaded tiles, finished accumulators, and
+// accumulators that the scanning warps have read.  With the tile's MMAs issued by
+// a scanning warp and a CTA barrier per tile, every tile waited for the slowest
+// warp and for the issue.  Tile kernel, with the packed query tiles: 2,001 radius
+// queries per agent on 150,000 nodes 111 -> 56 us; 4,096 nearest-neighbour queries
+// on 200,000 nodes 180 -> 154 us (their lists: 45 M warp instructions at 29 % issue,
+// four scanning warps per CTA and two CTAs per SM of tensor memory).
 template <int FMT, bool RAD>
-__global__ void __launch_bounds__(128 * TcSplit<FMT>::S, 1) knn_tc_kernel(KnnStoreDev st, const double* __restrict__ qs,
+__global__ void __launch_bounds__(128 * TcSplit<FMT>::S + 32, 1) knn_tc_kernel(KnnStoreDev st,
+                                                        const unsigned char* __restrict__ qtiles,
                                                         const int* __restrict__ qorder, const KnnItem* __restrict__ items,
                                                         int chunks_max, float* __restrict__ cand_d,
                                                         int* __restrict__ cand_i, float* __restrict__ cand_b,
-                                                        unsigned* __restrict__ g_thr, float* __restrict__ q_eps,
+                                                        unsigned* __restrict__ g_thr,
                                                         int* __restrict__ err, RadOut ro, unsigned imask) {
   constexpr int NT = FMT == KNN_FMT_EUCL ? kNtEucl : kNtAgent;
   constexpr uint32_t BT = NT * kRowBytes;   // bytes per node tile
@@ -999,14 +1103,11 @@ __global__ void __launch_bounds__(128 * TcSplit<FMT>::S, 1) knn_tc_kernel(KnnSto
   unsigned char* sA1 = base;
   unsigned char* sA2 = base + kTileM * kRowBytes;
   unsigned char* sB0 = base + 2 * kTileM * kRowBytes;   // kStagesB node-tile buffers
-  // per-thread candidate column: [32][blockDim] values after the operand buffers
+  // per-thread candidate column: [32][scanning threads] values after the operand buffers
   float* cand = (float*)(sB0 + kStagesB * (size_t)BT) + threadIdx.x;
-  __shared__ uint64_t bar_load[kStagesB], bar_mma[2];
+  __shared__ uint64_t bar_q, bar_load[kStagesB], bar_mma[2], bar_free[2];
   __shared__ uint32_t tbase;
   __shared__ int s_fail;
-  __shared__ float s_qn[kTileM], s_qna[4][kTileM];
-  __shared__ float s_tau[RAD ? kTileM : 1];
-  __shared__ long long s_qid[kTileM];
   __shared__ float s_bound[RAD ? 1 : kTileM];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row = tid & (kTileM - 1), slice = tid / kTileM;
@@ -1014,106 +1115,26 @@ __global__ void __launch_bounds__(128 * TcSplit<FMT>::S, 1) knn_tc_kernel(KnnSto
   const int D = st.D;
 
   if (tid == 0) {
+    mbar_init(&bar_q, 1);
     for (int b = 0; b < kStagesB; b++) mbar_init(&bar_load[b], 1);
-    mbar_init(&bar_mma[0], 1); mbar_init(&bar_mma[1], 1);
+    for (int b = 0; b < 2; b++) {
+      mbar_init(&bar_mma[b], 1);
+      mbar_init(&bar_free[b], 4 * S);
+    }
     s_fail = 0;
     fence_barrier_init();
   }
   if (warp == 0) tmem_alloc(&tbase, kTm);
-
-  // ---- the query tile: A1 = [q_hi | -1/2 ... | q_hi], A2 = [q_lo]; one thread per row
-  float qn = 0.f, qna[4] = {0.f, 0.f, 0.f, 0.f};
-  long long qid = -1;
-  if (tid < kTileM) {
-    const int r = tid;
-    for (int c = 0; c < 64; c++) {
-      *(__nv_bfloat16*)(sA1 + sw128_off(r, c)) = __float2bfloat16_rn(0.f);
-      *(__nv_bfloat16*)(sA2 + sw128_off(r, c)) = __float2bfloat16_rn(0.f);
-    }
-    if (r < it.qn) {
-      qid = qorder[it.q0 + r];
-      const double* q = qs + qid * D;
-      if (FMT == KNN_FMT_EUCL) {
-        double n2 = 0.0;
-        for (int j = 0; j < D; j++) {
-          float h, l;
-          split2(q[j], &h, &l);
-          *(__nv_bfloat16*)(sA1 + sw128_off(r, j)) = __float2bfloat16_rn(h);
-          *(__nv_bfloat16*)(sA1 + sw128_off(r, D + 3 + j)) = __float2bfloat16_rn(h);
-          *(__nv_bfloat16*)(sA2 + sw128_off(r, j)) = __float2bfloat16_rn(l);
-          n2 += q[j] * q[j];
-        }
-        for (int c = 0; c < 3; c++) *(__nv_bfloat16*)(sA1 + sw128_off(r, D + c)) = __float2bfloat16_rn(-0.5f);
-        qn = (float)n2;
-      } else {
-        for (int a = 0; a < st.A; a++) {
-          const int s = st.agent_s[a], d = st.agent_e[a] - s;
-          double na = 0.0;
-          for (int j = 0; j < d; j++) {
-            float h, l;
-            split2(q[s + j], &h, &l);
-            *(__nv_bfloat16*)(sA1 + sw128_off(r, 16 * a + j)) = __float2bfloat16_rn(h);
-            *(__nv_bfloat16*)(sA1 + sw128_off(r, 16 * a + d + j)) = __float2bfloat16_rn(h);
-            *(__nv_bfloat16*)(sA2 + sw128_off(r, 16 * a + j)) = __float2bfloat16_rn(l);
-            na += q[s + j] * q[s + j];
-          }
-          *(__nv_bfloat16*)(sA1 + sw128_off(r, 16 * a + 2 * d)) = __float2bfloat16_rn(-0.5f);
-          *(__nv_bfloat16*)(sA1 + sw128_off(r, 16 * a + 2 * d + 1)) = __float2bfloat16_rn(-0.5f);
-          qna[a] = (float)na;
-          qn += (float)na;
-        }
-      }
-      // error bound of the approximate squared distance (split-BF16 operands,
-      // FP32 accumulation), per query; stored once per query
-      const float es = sqrtf(qn) + st.mode_xmax[it.mode];
-      const float eps = 1.2e-4f * es * es + 1e-30f;
-      if (!RAD && it.chunk == 0) q_eps[qid] = eps;
-      if (RAD) s_tau[r] = ro.rad2[qid] < 0.f ? -__int_as_float(0x7f800000) : ro.rad2[qid] + 1.0001f * eps;
-    }
-    s_qid[r] = qid;
-    s_qn[r] = qn;
-    for (int a = 0; a < 4; a++) s_qna[a][r] = qna[a];
-  }
-  fence_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = tbase;
   const int T = it.tile1 - it.tile0;
-  qn = s_qn[row];
-  const unsigned char* gtiles = st.tiles + (long long)(st.mode_tile0[it.mode] + it.tile0) * BT;
-  const uint32_t idesc = idesc_bf16(kTileM, NT);
+  const unsigned char* qtile = qtiles + (size_t)it.qtile * kQTileBlock;
+  const long long qid = slice < S && row < it.qn ? (long long)qorder[it.q0 + row] : -1;
+  const float* qrows = qtile_rows(qtile);
+  const float qn = qrows[row];
 
-  auto issue_load = [&](int t) {
-    unsigned char* dst = sB0 + (t % kStagesB) * BT;
-    mbar_expect_tx(&bar_load[t % kStagesB], BT);
-    bulk_g2s(dst, gtiles + (long long)t * BT, BT, &bar_load[t % kStagesB]);
-  };
-  auto issue_mma = [&](int t) {
-    const uint32_t a1 = su32(sA1), a2 = su32(sA2), b = su32(sB0 + (t % kStagesB) * BT);
-    const uint32_t dcol = tm + (uint32_t)((t & 1) * (kTm / 2));
-    if (FMT == KNN_FMT_EUCL) {
-      for (int s = 0; s < 4; s++) umma_bf16(dcol, sw128_desc(a1 + 32 * s), sw128_desc(b + 32 * s), idesc, s > 0);
-      const int s2 = (D + 15) / 16;
-      for (int s = 0; s < s2; s++) umma_bf16(dcol, sw128_desc(a2 + 32 * s), sw128_desc(b + 32 * s), idesc, 1);
-    } else {
-      for (int a = 0; a < st.A; a++) {
-        umma_bf16(dcol + 64 * a, sw128_desc(a1 + 32 * a), sw128_desc(b + 32 * a), idesc, 0);
-        umma_bf16(dcol + 64 * a, sw128_desc(a2 + 32 * a), sw128_desc(b + 32 * a), idesc, 1);
-      }
-    }
-    umma_commit(&bar_mma[t & 1]);
-  };
-
-  if (tid == 0 && T > 0) {
-    for (int t = 0; t < kStagesB && t < T; t++) issue_load(t);
-    if (mbar_wait(&bar_load[0], 0)) issue_mma(0);
-    else s_fail = 1;
-  }
-
-  unsigned kk[kKeep];
-#pragma unroll
-  for (int i = 0; i < kKeep; i++) kk[i] = kKeyEmpty;
   // Threshold shared by the CTAs that scan other node chunks of the same
   // query: g_thr[q] holds the smallest 16th-kept value any of them has
   // published (FP32 bits of a non-negative value, so unsigned order is value
@@ -1124,84 +1145,188 @@ __global__ void __launch_bounds__(128 * TcSplit<FMT>::S, 1) knn_tc_kernel(KnnSto
   // `bound` is the smallest shared threshold this row has filtered with: every
   // node of the chunk left out of the list lies at or above min(bound, lower
   // end of the 16th key).
-  const long long qrow = RAD ? -1 : s_qid[row];
+  unsigned kk[kKeep];
+#pragma unroll
+  for (int i = 0; i < kKeep; i++) kk[i] = kKeyEmpty;
   float gcur = __int_as_float(0x7f800000), gnext = gcur, bound = gcur, published = gcur;
 
-  for (int t = 0; t < T; t++) {
-    if (tid == 0 && t + 1 < T && !s_fail) {
-      if (mbar_wait(&bar_load[(t + 1) % kStagesB], ((t + 1) / kStagesB) & 1)) issue_mma(t + 1);
-      else s_fail = 1;
-    }
-    const bool done = mbar_wait(&bar_mma[t & 1], (t >> 1) & 1);
-    if (!done) s_fail = 1;
-    tc_fence_after();
-    if (tid == 0 && t + kStagesB < T && done) issue_load(t + kStagesB);   // tile t's MMAs have read its buffer
-    if (!RAD && qrow >= 0) gnext = __uint_as_float(*(volatile const unsigned*)&g_thr[qrow]);
-    if (done) {
-      const int lcol = t * NT;   // chunk-local index of the tile's first node
-      const uint32_t lane_base = tm + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((t & 1) * (kTm / 2));
-      if (FMT == KNN_FMT_EUCL) {
-#pragma unroll 1
-        for (int c0 = slice * NCOL; c0 < slice * NCOL + NCOL; c0 += 32) {
-          float v[32];
-          tmem_ld32(lane_base + c0, v);
-          if (RAD) {
-            rad_chunk<true>(v, qn, s_tau[row], s_qid[row], (it.tile0 + t) * NT + c0, ro);
-          } else if (qrow >= 0) {   // a padding row of a partial query tile keeps no list
-            // marks: the dot products against the row's threshold in dot
-            // space, (qn - thr) / 2, lowered by a margin that covers the FP32
-            // rounding of both forms, so an unmarked column's distance
-            // qn - 2 v lies at or above thr
-            const float thr = fminf(key_lower(kk[kKeep - 1], imask), gcur);
-            const float thd = 0.5f * (qn - thr) - 1e-6f * (fabsf(qn) + fabsf(thr));
-            const unsigned mk = mark32<true>(v, thd);
-            if (mk) keep_marked<true>(kk, v, mk, qn, cand, lcol + c0, imask);
+  if (warp == 4 * S) {
+    // ---- the feeding warp
+    if (lane == 0 && T > 0) {
+      const unsigned char* gtiles = st.tiles + (long long)(st.mode_tile0[it.mode] + it.tile0) * BT;
+      const uint32_t idesc = idesc_bf16(kTileM, NT);
+      int loads = 0, mmas = 0;   // issued
+      auto issue_load = [&]() {
+        const int b = loads % kStagesB;
+        mbar_expect_tx(&bar_load[b], BT);
+        bulk_g2s(sB0 + b * BT, gtiles + (long long)loads * BT, BT, &bar_load[b]);
+        loads++;
+      };
+      auto issue_mma = [&](int t) {
+        const uint32_t a1 = su32(sA1), a2 = su32(sA2), b = su32(sB0 + (t % kStagesB) * BT);
+        const uint32_t dcol = tm + (uint32_t)((t & 1) * (kTm / 2));
+        if (FMT == KNN_FMT_EUCL) {
+          for (int s = 0; s < 4; s++) umma_bf16(dcol, sw128_desc(a1 + 32 * s), sw128_desc(b + 32 * s), idesc, s > 0);
+          const int s2 = (D + 15) / 16;
+          for (int s = 0; s < s2; s++) umma_bf16(dcol, sw128_desc(a2 + 32 * s), sw128_desc(b + 32 * s), idesc, 1);
+        } else {
+          for (int a = 0; a < st.A; a++) {
+            umma_bf16(dcol + 64 * a, sw128_desc(a1 + 32 * a), sw128_desc(b + 32 * a), idesc, 0);
+            umma_bf16(dcol + 64 * a, sw128_desc(a2 + 32 * a), sw128_desc(b + 32 * a), idesc, 1);
           }
+        }
+        umma_commit(&bar_mma[t & 1]);
+        mmas = t + 1;
+      };
+      mbar_expect_tx(&bar_q, kQTileBytes);
+      bulk_g2s(sA1, qtile, kQTileBytes, &bar_q);
+      while (loads < T && loads < kStagesB) issue_load();
+      bool ok = mbar_wait(&bar_q, 0);
+      for (int t = 0; ok && t < T; t++) {
+        ok = mbar_wait(&bar_load[t % kStagesB], (t / kStagesB) & 1);
+        if (ok && t >= 2) {
+          ok = mbar_wait(&bar_free[t & 1], ((t >> 1) - 1) & 1);   // tile t - 2 has been read
+          tc_fence_after();
+        }
+        if (ok) issue_mma(t);
+        if (ok && t >= 1 && loads < T) {   // tile t - 1's MMAs have read its buffer: the next load goes there
+          ok = mbar_wait(&bar_mma[(t - 1) & 1], ((t - 1) >> 1) & 1);
+          if (ok) issue_load();
+        }
+      }
+      if (!ok) {
+        // a wait ran out: report, then wait (bounded) for what is in flight
+        *(volatile int*)&s_fail = 1;
+        for (int u = max(0, loads - kStagesB); u < loads; u++) mbar_wait(&bar_load[u % kStagesB], (u / kStagesB) & 1);
+        if (mmas > 0) mbar_wait(&bar_mma[(mmas - 1) & 1], ((mmas - 1) >> 1) & 1);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ---- the scanning warps
+    const long long qrow = RAD ? -1 : qid;
+    const float tau = RAD ? qrows[5 * kTileM + row] : 0.f;
+    float qna[4] = {0.f, 0.f, 0.f, 0.f};
+    if (FMT == KNN_FMT_AGENT)
+#pragma unroll
+      for (int a = 0; a < 4; a++) qna[a] = qrows[(1 + a) * kTileM + row];
+    auto scan = [&](const float (&v)[32], int t, int c0) {
+      if (FMT == KNN_FMT_EUCL) {
+        if (RAD) {
+          rad_chunk<true>(v, qn, tau, qid, (it.tile0 + t) * NT + c0, ro);
+        } else if (qrow >= 0) {   // a padding row of a partial query tile keeps no list
+          // marks: the dot products against the row's threshold in dot
+          // space, (qn - thr) / 2, lowered by a margin that covers the FP32
+          // rounding of both forms, so an unmarked column's distance
+          // qn - 2 v lies at or above thr
+          const float thr = fminf(key_lower(kk[kKeep - 1], imask), gcur);
+          const float thd = 0.5f * (qn - thr) - 1e-6f * (fabsf(qn) + fabsf(thr));
+          const unsigned mk = mark32<true>(v, thd);
+          if (mk) keep_marked<true>(kk, v, mk, qn, cand, t * NT + c0, imask);
         }
       } else {
-#pragma unroll 1
-        for (int c0 = slice * NCOL; c0 < slice * NCOL + NCOL; c0 += 32) {
-          float m[32];
-#pragma unroll
-          for (int i = 0; i < 32; i++) m[i] = -__int_as_float(0x7f800000);
-          for (int a = 0; a < st.A; a++) {
-            float v[32];
-            tmem_ld32(lane_base + 64 * a + c0, v);
-            const float qa = s_qna[a][row];
-#pragma unroll
-            for (int i = 0; i < 32; i++) m[i] = fmaxf(m[i], fmaf(-2.f, v[i], qa));
-          }
-          if (RAD) {
-            rad_chunk<false>(m, 0.f, s_tau[row], s_qid[row], (it.tile0 + t) * NT + c0, ro);
-          } else if (qrow >= 0) {
-            const float thr = fminf(key_lower(kk[kKeep - 1], imask), gcur);
-            const unsigned mk = mark32<false>(m, thr);
-            if (mk) keep_marked<false>(kk, m, mk, 0.f, cand, lcol + c0, imask);
-          }
+        if (RAD) {
+          rad_chunk<false>(v, 0.f, tau, qid, (it.tile0 + t) * NT + c0, ro);
+        } else if (qrow >= 0) {
+          const float thr = fminf(key_lower(kk[kKeep - 1], imask), gcur);
+          const unsigned mk = mark32<false>(v, thr);
+          if (mk) keep_marked<false>(kk, v, mk, 0.f, cand, t * NT + c0, imask);
         }
       }
-    }
-    if (!RAD && qrow >= 0) {
-      bound = fminf(bound, gcur);
-      const float up = key_upper(kk[kKeep - 1], imask);
-      if (up < published) {   // publish a better 16th value
-        published = up;
-        atomicMin(&g_thr[qrow], __float_as_uint(fmaxf(published, 0.f)));
+    };
+    for (int t = 0; t < T; t++) {
+      if (!__all_sync(MRMG_FULL, mbar_wait(&bar_mma[t & 1], (t >> 1) & 1))) {
+        *(volatile int*)&s_fail = 1;
+        break;
       }
-      gcur = fminf(gcur, gnext);
+      tc_fence_after();
+      if (!RAD && qrow >= 0) gnext = __uint_as_float(*(volatile const unsigned*)&g_thr[qrow]);
+      const uint32_t lane_base = tm + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((t & 1) * (kTm / 2));
+      auto release = [&]() {   // this warp has read the tile's accumulator
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_free[t & 1]);
+      };
+      if (FMT == KNN_FMT_EUCL && !RAD) {
+        // one copy of the list code: four, with the next load under way, ran from
+        // the instruction cache no more (180 -> 232 us)
+#pragma unroll 1
+        for (int c0 = 0; c0 < NCOL; c0 += 32) {
+          float v[32];
+          tmem_ld32(lane_base + c0, v);
+          if (c0 + 32 == NCOL) release();
+          scan(v, t, c0);
+        }
+      } else if (FMT == KNN_FMT_EUCL) {
+        // the next 32 columns are on their way while these are scanned
+        // (straight-line code: a load's registers must not pass a branch, where
+        // the compiler could copy them before the wait)
+        static_assert(NCOL == 128 || FMT != KNN_FMT_EUCL, "four loads per tile");
+        uint32_t r0[32], r1[32], r2[32], r3[32];
+        float v[32];
+        tmem_ld32_issue(lane_base, r0);
+        tmem_ld_wait();
+        tmem_ld32_issue(lane_base + 32, r1);
+        tmem_take(r0, v);
+        scan(v, t, 0);
+        tmem_ld_wait();
+        tmem_ld32_issue(lane_base + 64, r2);
+        tmem_take(r1, v);
+        scan(v, t, 32);
+        tmem_ld_wait();
+        tmem_ld32_issue(lane_base + 96, r3);
+        tmem_take(r2, v);
+        scan(v, t, 64);
+        tmem_ld_wait();
+        release();
+        tmem_take(r3, v);
+        scan(v, t, 96);
+      } else {
+        // all four agents' columns (those past the last agent hold nothing that is used)
+        const int c0 = slice * NCOL;
+        float m[32];
+        uint32_t r0[32], r1[32], r2[32], r3[32];
+        tmem_ld32_issue(lane_base + c0, r0);
+        tmem_ld32_issue(lane_base + 64 + c0, r1);
+        tmem_ld_wait();
+        tmem_ld32_issue(lane_base + 128 + c0, r2);
+        tmem_ld32_issue(lane_base + 192 + c0, r3);
+#pragma unroll
+        for (int i = 0; i < 32; i++) m[i] = -__int_as_float(0x7f800000);
+        auto fold = [&](uint32_t (&r)[32], float qa) {
+          float v[32];
+          tmem_take(r, v);
+#pragma unroll
+          for (int i = 0; i < 32; i++) m[i] = fmaxf(m[i], fmaf(-2.f, v[i], qa));
+        };
+        fold(r0, qna[0]);
+        if (st.A > 1) fold(r1, qna[1]);
+        tmem_ld_wait();
+        release();
+        if (st.A > 2) fold(r2, qna[2]);
+        if (st.A > 3) fold(r3, qna[3]);
+        scan(m, t, c0);
+      }
+      if (!RAD && qrow >= 0) {
+        bound = fminf(bound, gcur);
+        const float up = key_upper(kk[kKeep - 1], imask);
+        if (up < published) {   // publish a better 16th value
+          published = up;
+          atomicMin(&g_thr[qrow], __float_as_uint(fmaxf(published, 0.f)));
+        }
+        gcur = fminf(gcur, gnext);
+      }
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (s_fail) break;
   }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
   if (s_fail && tid == 0) atomicOr(err, E_TIMEOUT);
-  (void)lane;
   // merge the slices' lists into slice 0's; every MMA has completed, so the
   // operand buffers are free (skipped after a timeout: copies may be in flight)
   if (!RAD && !s_fail) {
     unsigned* mk = (unsigned*)base;
-    if (slice > 0) {
+    if (slice > 0 && slice < S) {
 #pragma unroll
       for (int i = 0; i < kKeep; i++) mk[((size_t)(slice - 1) * kKeep + i) * kTileM + row] = kk[i];
       if (S > 1) s_bound[row] = bound;   // (S <= 2)
@@ -1219,7 +1344,7 @@ __global__ void __launch_bounds__(128 * TcSplit<FMT>::S, 1) knn_tc_kernel(KnnSto
   }
   // the lists leave as (lower end of the distance, mode-local node index),
   // an empty slot as (inf, -1)
-  if (!RAD && qid >= 0) {
+  if (!RAD && qid >= 0 && slice == 0) {
     float* od = cand_d + ((size_t)qid * chunks_max + it.chunk) * kKeep;
     int* oi = cand_i + ((size_t)qid * chunks_max + it.chunk) * kKeep;
     const float INF = __int_as_float(0x7f800000);
@@ -1836,6 +1961,8 @@ struct ItemPlan {
   std::vector<KnnItem> items;
   int chunks_max = 1;
   int tpc = 1;              // node tiles per chunk
+  int n_items = 0;          // work items; after them `items` holds one item of each query tile
+  int n_qtiles = 0;         // query tiles
 };
 
 // the index field of the candidate keys: the low bits of a key hold a node's
@@ -1875,6 +2002,7 @@ static void plan_items(const KnnStore* s, const int* h_q_mode, long long Q, int 
   pl->chunks_max = chunks_max;
   pl->tpc = tpc;
   pl->items.clear();
+  pl->n_qtiles = 0;
   pl->mode_chunks.assign(n_modes, 0);
   for (int m = 0; m < n_modes; m++) {
     if (pl->qcount[m] == 0 || s->mode_tiles[m] == 0) continue;
@@ -1889,8 +2017,9 @@ static void plan_items(const KnnStore* s, const int* h_q_mode, long long Q, int 
         it.tile0 = c * tpc;
         it.tile1 = std::min(s->mode_tiles[m], (c + 1) * tpc);
         it.chunk = c;
-        it.pad = 0;
+        it.qtile = pl->n_qtiles;
         pl->items.push_back(it);
+        if (c == nch - 1) pl->n_qtiles++;
       }
   }
   // longest items first (CTAs start in index order: the short ones fill the
@@ -1898,6 +2027,10 @@ static void plan_items(const KnnStore* s, const int* h_q_mode, long long Q, int 
   std::stable_sort(pl->items.begin(), pl->items.end(), [](const KnnItem& a, const KnnItem& b) {
     return (long long)(a.tile1 - a.tile0) * a.qn > (long long)(b.tile1 - b.tile0) * b.qn;
   });
+  pl->n_items = (int)pl->items.size();
+  pl->items.reserve(pl->n_items + pl->n_qtiles);
+  for (int i = 0; i < pl->n_items; i++)
+    if (pl->items[i].chunk == 0) pl->items.push_back(pl->items[i]);
 }
 
 // Shared memory of a candidate CTA.  The euclidean kernel takes 256 tensor-
@@ -1905,7 +2038,7 @@ static void plan_items(const KnnStore* s, const int* h_q_mode, long long Q, int 
 // fit in shared memory, so no CTA waits for columns); the per-agent kernel
 // takes all 512 columns and is held to one CTA per SM by asking for at least
 // 120 KB, so two CTAs never wait on each other for the columns.
-static size_t tc_smem_bytes(const KnnStore* s) {
+static size_t tc_smem_bytes(const KnnStore* s) {   // (candidate columns: scanning threads only)
   const int NT = s->dev.NT;
   const bool eucl = s->dev.fmt == KNN_FMT_EUCL;
   const int nthreads = 128 * (eucl ? TcSplit<KNN_FMT_EUCL>::S : TcSplit<KNN_FMT_AGENT>::S);
@@ -1963,7 +2096,8 @@ cudaError_t knn_query(KnnStore* s, const double* d_qs, long long Q, const int* h
   const size_t b_eps = al(sizeof(float) * std::max<long long>(Q, 1));
   const size_t b_fb = al(sizeof(long long) * std::max<long long>(Q, 1));
   const size_t b_ctr = 256;
-  const size_t need = b_order + b_qmode + b_items + b_mch + b_g + b_cd + b_ci + b_cb + b_eps + b_fb + b_ctr;
+  const size_t b_qt = al((size_t)std::max(pl.n_qtiles, 1) * kQTileBlock);
+  const size_t need = b_order + b_qmode + b_items + b_mch + b_g + b_cd + b_ci + b_cb + b_eps + b_fb + b_qt + b_ctr;
   if (scr->bytes < need) {
     if (scr->block) cudaFree(scr->block);
     scr->block = nullptr;
@@ -1982,6 +2116,7 @@ cudaError_t knn_query(KnnStore* s, const double* d_qs, long long Q, const int* h
   float* d_cb = (float*)p; p += b_cb;
   float* d_eps = (float*)p; p += b_eps;
   long long* d_fb = (long long*)p; p += b_fb;
+  unsigned char* d_qt = p; p += b_qt;   // packed query tiles
   int* d_ctr = (int*)p;   // [0] fallback count, [1] error bits
   // order, query modes, items, chunk counts and the shared thresholds' start
   // values sit back to back in the device block: stage them in pinned memory
@@ -2009,13 +2144,14 @@ cudaError_t knn_query(KnnStore* s, const double* d_qs, long long Q, const int* h
   raise_smem_limit<KNN_FMT_EUCL, false>();
   raise_smem_limit<KNN_FMT_AGENT, false>();
   if (!items.empty()) {
-    if (s->dev.fmt == KNN_FMT_EUCL) {
-      knn_tc_kernel<KNN_FMT_EUCL, false><<<(int)items.size(), 128 * TcSplit<KNN_FMT_EUCL>::S, smem, st>>>(s->dev, d_qs, d_order, d_items, chunks_max,
-                                                                         d_cd, d_ci, d_cb, d_g, d_eps, d_ctr + 1, RadOut{}, imask);
-    } else {
-      knn_tc_kernel<KNN_FMT_AGENT, false><<<(int)items.size(), 128 * TcSplit<KNN_FMT_AGENT>::S, smem, st>>>(s->dev, d_qs, d_order, d_items, chunks_max,
-                                                                          d_cd, d_ci, d_cb, d_g, d_eps, d_ctr + 1, RadOut{}, imask);
-    }
+    knn_pack_queries_kernel<<<dim3((unsigned)pl.n_qtiles, kTileM / kPackRows), 32 * kPackRows, 0, st>>>(
+        s->dev, d_qs, d_order, d_items + pl.n_items, d_qt, d_eps, nullptr);
+    if (s->dev.fmt == KNN_FMT_EUCL)
+      knn_tc_kernel<KNN_FMT_EUCL, false><<<pl.n_items, 128 * TcSplit<KNN_FMT_EUCL>::S + 32, smem, st>>>(
+          s->dev, d_qt, d_order, d_items, chunks_max, d_cd, d_ci, d_cb, d_g, d_ctr + 1, RadOut{}, imask);
+    else
+      knn_tc_kernel<KNN_FMT_AGENT, false><<<pl.n_items, 128 * TcSplit<KNN_FMT_AGENT>::S + 32, smem, st>>>(
+          s->dev, d_qt, d_order, d_items, chunks_max, d_cd, d_ci, d_cb, d_g, d_ctr + 1, RadOut{}, imask);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -2328,7 +2464,8 @@ cudaError_t near_query(NearState* ns, KnnStore* s, const double* d_qs, long long
   const size_t b_offs = al(sizeof(long long) * (Q + 1));
   const size_t b_q32 = al(sizeof(float) * std::max<long long>(Q, 1) * std::max(s->D, 1));
   const size_t b_stage = al(sizeof(int) * std::max<long long>(Q, 1) * kNearStage);
-  const size_t need = b_up + b_bits + b_cnt + b_offs + 256 + b_q32 + b_stage;
+  const size_t b_qt = al((size_t)pl.n_qtiles * kQTileBlock);
+  const size_t need = b_up + b_bits + b_cnt + b_offs + 256 + b_q32 + b_stage + b_qt;
   if (ns->scr.bytes < need) {
     if (ns->scr.block) cudaFree(ns->scr.block);
     ns->scr.block = nullptr;
@@ -2350,6 +2487,7 @@ cudaError_t near_query(NearState* ns, KnnStore* s, const double* d_qs, long long
   long long* d_ctr = (long long*)(p + b_up + b_bits + b_cnt + b_offs);   // [0] total, [1] error bits
   float* d_q32 = (float*)(p + b_up + b_bits + b_cnt + b_offs + 256);
   int* d_stage = (int*)(p + b_up + b_bits + b_cnt + b_offs + 256 + b_q32);
+  unsigned char* d_qt = (unsigned char*)d_stage + b_stage;   // packed query tiles
   cudaError_t e = cudaMemcpyAsync(p, hp, b_up, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_cnt, 0, b_cnt + 256, st);   // the counts, then the counters
   if (e == cudaSuccess) e = to_f32(d_qs, d_q32, Q * s->D, st);
@@ -2357,16 +2495,16 @@ cudaError_t near_query(NearState* ns, KnnStore* s, const double* d_qs, long long
   if (tc && !pl.items.empty()) {
     const size_t smem = tc_smem_bytes(tc);
     const RadOut ro{d_bits, d_woff, d_rad2};
+    knn_pack_queries_kernel<<<dim3((unsigned)pl.n_qtiles, kTileM / kPackRows), 32 * kPackRows, 0, st>>>(
+        tc->dev, d_qs, d_order, d_items + pl.n_items, d_qt, nullptr, d_rad2);
     if (s->dev.fmt == KNN_FMT_EUCL) {
       raise_smem_limit<KNN_FMT_EUCL, true>();
-      knn_tc_kernel<KNN_FMT_EUCL, true><<<(int)pl.items.size(), 128 * TcSplit<KNN_FMT_EUCL>::S, smem, st>>>(
-          tc->dev, d_qs, d_order, d_items, pl.chunks_max, nullptr, nullptr, nullptr, nullptr, nullptr,
-          (int*)(d_ctr + 1), ro, 0u);
+      knn_tc_kernel<KNN_FMT_EUCL, true><<<pl.n_items, 128 * TcSplit<KNN_FMT_EUCL>::S + 32, smem, st>>>(
+          tc->dev, d_qt, d_order, d_items, pl.chunks_max, nullptr, nullptr, nullptr, nullptr, (int*)(d_ctr + 1), ro, 0u);
     } else {
       raise_smem_limit<KNN_FMT_AGENT, true>();
-      knn_tc_kernel<KNN_FMT_AGENT, true><<<(int)pl.items.size(), 128 * TcSplit<KNN_FMT_AGENT>::S, smem, st>>>(
-          tc->dev, d_qs, d_order, d_items, pl.chunks_max, nullptr, nullptr, nullptr, nullptr, nullptr,
-          (int*)(d_ctr + 1), ro, 0u);
+      knn_tc_kernel<KNN_FMT_AGENT, true><<<pl.n_items, 128 * TcSplit<KNN_FMT_AGENT>::S + 32, smem, st>>>(
+          tc->dev, d_qt, d_order, d_items, pl.chunks_max, nullptr, nullptr, nullptr, nullptr, (int*)(d_ctr + 1), ro, 0u);
     }
   }
   if (e == cudaSuccess) e = cudaGetLastError();
