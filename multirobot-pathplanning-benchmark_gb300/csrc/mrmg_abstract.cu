@@ -552,7 +552,7 @@ __global__ void edges_kernel(AbstractDev s, const void* q1, const void* q2, int 
 // ---------------------------------------------------------------------------
 template <int DIM>
 __global__ void __launch_bounds__(256) configs_fused_kernel(AbstractDev s, const void* q, int dtype, long long n,
-                                                            uint8_t* out, int* ctr) {
+                                                            uint8_t* out, int* ctr, CallDone done) {
   extern __shared__ __align__(16) double sm_cfg[];
   const AbstractDev cs = staged_view(s, (unsigned char*)sm_cfg);
   __syncthreads();
@@ -587,6 +587,10 @@ __global__ void __launch_bounds__(256) configs_fused_kernel(AbstractDev s, const
     if (i < n) out[i] = v;
   }
   if (ctr && lane == 0 && npend) atomicAdd(&ctr[kCtrPending], npend);
+  if (done.cta) {
+    __syncthreads();
+    if (threadIdx.x == 0) signal_done(done);
+  }
 }
 
 // Edges, flat: each CTA takes `epc` edges at a time; its warps compute the
@@ -600,7 +604,7 @@ template <int DIM>
 __global__ void __launch_bounds__(256) edges_flat_kernel(AbstractDev s, const void* q1, const void* q2, int dtype,
                                                          long long n, double res, int incl, const long long* Np,
                                                          long long N_start, long long N_max, uint8_t* out, int* ctr,
-                                                         int epc, uint8_t* cta_err) {
+                                                         int epc, uint8_t* cta_err, CallDone done) {
   extern __shared__ __align__(16) double sm_ab[];
   const AbstractDev cs = staged_view(s, (unsigned char*)sm_ab);
   __shared__ int s_err;   // error bits of this CTA when reported per CTA (cta_err)
@@ -761,34 +765,36 @@ __global__ void __launch_bounds__(256) edges_flat_kernel(AbstractDev s, const vo
   }
   if (ctr && lane == 0 && npend) atomicAdd(&ctr[kCtrPending], npend);
   if (cta_err && threadIdx.x == 0) cta_err[blockIdx.x] = (uint8_t)s_err;   // after the loop's last barrier
+  if (done.cta && threadIdx.x == 0) signal_done(done);
 }
 
 }  // namespace
 
 // the fused kernels, compiled for agent dimensions 2 and 3 and for any
 static void launch_configs_fused(const AbstractDev& s, int grid, int threads, cudaStream_t st, const void* q,
-                                 int dtype, long long n, uint8_t* out, int* ctr) {
+                                 int dtype, long long n, uint8_t* out, int* ctr, const CallDone& done) {
   const size_t sm = tab_bytes(s) + (size_t)(threads / 32) * s.D * sizeof(double);   // tables, per-warp coordinates
-  if (s.dim == 2) configs_fused_kernel<2><<<grid, threads, sm, st>>>(s, q, dtype, n, out, ctr);
-  else if (s.dim == 3) configs_fused_kernel<3><<<grid, threads, sm, st>>>(s, q, dtype, n, out, ctr);
-  else configs_fused_kernel<0><<<grid, threads, sm, st>>>(s, q, dtype, n, out, ctr);
+  if (s.dim == 2) configs_fused_kernel<2><<<grid, threads, sm, st>>>(s, q, dtype, n, out, ctr, done);
+  else if (s.dim == 3) configs_fused_kernel<3><<<grid, threads, sm, st>>>(s, q, dtype, n, out, ctr, done);
+  else configs_fused_kernel<0><<<grid, threads, sm, st>>>(s, q, dtype, n, out, ctr, done);
 }
 
 static size_t flat_smem(const AbstractDev& s) { return tab_bytes(s) + (size_t)kFlatMaxEpc * s.D * 32; }
 
 static void launch_edges_flat(const AbstractDev& s, int grid, cudaStream_t st, const void* q1, const void* q2,
                               int dtype, long long n, double res, int incl, const long long* Np, long long N_start,
-                              long long N_max, uint8_t* out, int* ctr, int epc, uint8_t* cta_err) {
+                              long long N_max, uint8_t* out, int* ctr, int epc, uint8_t* cta_err,
+                              const CallDone& done) {
   const size_t sm = flat_smem(s);
   if (s.dim == 2)
     edges_flat_kernel<2><<<grid, 256, sm, st>>>(s, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, ctr, epc,
-                                                cta_err);
+                                                cta_err, done);
   else if (s.dim == 3)
     edges_flat_kernel<3><<<grid, 256, sm, st>>>(s, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, ctr, epc,
-                                                cta_err);
+                                                cta_err, done);
   else
     edges_flat_kernel<0><<<grid, 256, sm, st>>>(s, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, ctr, epc,
-                                                cta_err);
+                                                cta_err, done);
 }
 
 cudaError_t abstract_configs(const AbstractDev& s, const void* q, int dtype, long long n,
@@ -799,7 +805,7 @@ cudaError_t abstract_configs(const AbstractDev& s, const void* q, int dtype, lon
   const int threads = 128;
   const long long want = (n + threads - 1) / threads;
   const int grid = (int)std::max(1ll, std::min(want, (long long)ls.num_sms * 16));
-  launch_configs_fused(s, grid, threads, st, q, dtype, n, out, sc.ctr);
+  launch_configs_fused(s, grid, threads, st, q, dtype, n, out, sc.ctr, CallDone{});
   return cudaGetLastError();
 }
 
@@ -811,22 +817,24 @@ static int flat_epc(long long n, int num_sms) {
 
 
 cudaError_t abstract_configs_mapped(const AbstractDev& s, const void* q, int dtype, long long n, uint8_t* out,
-                                    int num_sms, cudaStream_t st) {
+                                    const CallDone& done, int num_sms, cudaStream_t st, int* grid_out) {
   const int threads = 128;
   const long long want = (n + threads - 1) / threads;
   const int grid = (int)std::max(1ll, std::min(want, (long long)num_sms * 16));
-  launch_configs_fused(s, grid, threads, st, q, dtype, n, out, nullptr);
+  *grid_out = grid;
+  launch_configs_fused(s, grid, threads, st, q, dtype, n, out, nullptr, done);
   return cudaGetLastError();
 }
 
 cudaError_t abstract_edges_mapped(const AbstractDev& s, const void* q1, const void* q2, int dtype, long long n,
                                   double res, int incl, const long long* Np, long long N_start, long long N_max,
-                                  uint8_t* out, uint8_t* cta_err, int num_sms, cudaStream_t st, int* grid_out) {
+                                  uint8_t* out, uint8_t* cta_err, const CallDone& done, int num_sms, cudaStream_t st,
+                                  int* grid_out) {
   const int epc = flat_epc(n, num_sms);
   const long long want = (n + epc - 1) / epc;
   const int grid = (int)std::max(1ll, std::min(want, (long long)num_sms * 8));
   *grid_out = grid;
-  launch_edges_flat(s, grid, st, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, nullptr, epc, cta_err);
+  launch_edges_flat(s, grid, st, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, nullptr, epc, cta_err, done);
   return cudaGetLastError();
 }
 
@@ -850,7 +858,8 @@ cudaError_t abstract_edges(const AbstractDev& s, const void* q1, const void* q2,
     const int epc = flat_epc(n, ls.num_sms);
     const long long want = (n + epc - 1) / epc;
     const int grid = (int)std::min(want, (long long)ls.num_sms * 8);
-    launch_edges_flat(s, grid, st, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, sc.ctr, epc, nullptr);
+    launch_edges_flat(s, grid, st, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, sc.ctr, epc, nullptr,
+                      CallDone{});
     return cudaGetLastError();
   }
   const int warps = 8;

@@ -1,5 +1,6 @@
 // mrmg_api.cu -- the C ABI: scene handles, per-handle scratch, status codes.
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -203,7 +204,8 @@ LaunchShape shape(mrmg_scene* sc) {
 
 // the scene's stream and mapped staging buffer (host-pointer calls, below)
 int ensure_stage(mrmg_scene* sc, size_t bytes);
-constexpr size_t kStageHead = 16 * 1024;   // per-CTA statistics / error bytes at the head of the mapped buffer
+constexpr size_t kStageDone = 16 * 1024;   // a byte per CTA (CallDone), after the per-CTA statistics / error bytes
+constexpr size_t kStageHead = kStageDone + 4096;   // head of the mapped buffer
 
 int finish_call(mrmg_scene* sc, cudaStream_t st, int flags) {
   cudaError_t e = cudaMemcpyAsync(sc->h_ctr, sc->d_ctr, sizeof(int) * kNumCtr, cudaMemcpyDeviceToHost, st);
@@ -978,7 +980,8 @@ int mrmg_is_collision_free_batch(mrmg_scene* sc, const void* d_q, int32_t dtype,
   if (sc->kind == 0 && !(flags & MRMG_FLAG_ASYNC)) {
     // synchronous abstract call: the fused kernel alone (pending
     // configurations are decided inline), no counter round trip
-    cudaError_t e = abstract_configs_mapped(ab, d_q, dtype, n, d_out, sc->num_sms, st);
+    int grid = 0;
+    cudaError_t e = abstract_configs_mapped(ab, d_q, dtype, n, d_out, CallDone{}, sc->num_sms, st, &grid);
     if (e != cudaSuccess) return cuda_fail(e, "launch configs");
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "kernel execution");
@@ -1038,8 +1041,8 @@ int mrmg_is_edge_collision_free_batch(mrmg_scene* sc, const void* d_q1, const vo
     if (rc) return rc;
     int grid = 0;
     cudaError_t e = abstract_edges_mapped(sc->ab, d_q1, d_q2, dtype, n, resolution, include_endpoints,
-                                          (const long long*)d_N, N_start, N_max, d_out, sc->m_stage, sc->num_sms, st,
-                                          &grid);
+                                          (const long long*)d_N, N_start, N_max, d_out, sc->m_stage, CallDone{}, sc->num_sms,
+                                          st, &grid);
     if (e != cudaSuccess) return cuda_fail(e, "launch edges");
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "kernel execution");
@@ -1173,13 +1176,39 @@ bool host_edge_N(const void* q1, const void* q2, int dtype, long long e, int D, 
   return true;
 }
 
+// the CTAs' end bytes, cleared for the next call (its grid is at most 16 CTAs per SM)
+CallDone next_done(mrmg_scene* sc) {
+  if ((size_t)sc->num_sms * 16 > kStageHead - kStageDone) return CallDone{nullptr};
+  std::memset(sc->h_stage + kStageDone, 0, kStageHead - kStageDone);
+  __atomic_thread_fence(__ATOMIC_RELEASE);
+  return CallDone{sc->m_stage + kStageDone};
+}
+
+// Wait for the end bytes of a call's `grid` CTAs; after a while (a long call, a busy
+// device, a failed kernel, which never sets them) for the stream.  The stream is
+// still behind the kernel's retirement: later work on it is ordered as ever.
+cudaError_t wait_done(mrmg_scene* sc, int grid) {
+  const uint8_t* end = sc->h_stage + kStageDone;
+  const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(200);
+  int c = (size_t)sc->num_sms * 16 > kStageHead - kStageDone ? -1 : 0;   // CTAs seen to be through
+  while (c >= 0) {
+    for (int i = 0; i < 32; i++) {
+      while (c < grid && __atomic_load_n(end + c, __ATOMIC_ACQUIRE)) c++;
+      if (c == grid) return cudaSuccess;
+    }
+    if (std::chrono::steady_clock::now() > until) break;
+  }
+  return cudaStreamSynchronize(sc->own_stream);
+}
+
 // launch the single-launch kernel on the mapped buffer, wait, and fill the
 // scene's statistics from the per-CTA slots
 int run_small(mrmg_scene* sc, const ArmDev& a, SmallBatch& b) {
   int grid = 0;
+  b.done = next_done(sc);
   cudaError_t e = arm_small(a, b, sc->num_sms, sc->own_stream, &grid);
   if (e != cudaSuccess) return cuda_fail(e, "launch small batch");
-  e = cudaStreamSynchronize(sc->own_stream);
+  e = wait_done(sc, grid);
   if (e != cudaSuccess) return cuda_fail(e, "kernel execution");
   const int* st = (const int*)sc->h_stage;
   long long cfg = 0, pend = 0;
@@ -1229,10 +1258,11 @@ int mrmg_is_collision_free_host(mrmg_scene* sc, const void* h_q, int32_t dtype, 
     // one launch, verdicts written straight into the mapped buffer
     AbstractDev ab = sc->ab;
     ab.sph_batch_form = (flags & MRMG_FLAG_BATCH_FORM) ? 1 : 0;
-    cudaError_t e = abstract_configs_mapped(ab, in_q, dtype, n, sc->m_stage + o_hit, sc->num_sms,
-                                            sc->own_stream);
+    int grid = 0;
+    cudaError_t e = abstract_configs_mapped(ab, in_q, dtype, n, sc->m_stage + o_hit, next_done(sc),
+                                            sc->num_sms, sc->own_stream, &grid);
     if (e != cudaSuccess) return cuda_fail(e, "launch configs");
-    e = cudaStreamSynchronize(sc->own_stream);
+    e = wait_done(sc, grid);
     if (e != cudaSuccess) return cuda_fail(e, "kernel execution");
     std::memcpy(h_out, H + o_hit, (size_t)n);
     return MRMG_OK;
@@ -1342,10 +1372,10 @@ int mrmg_is_edge_collision_free_host(mrmg_scene* sc, const void* h_q1, const voi
     // bits come back per CTA in the head of the buffer
     int grid = 0;
     cudaError_t e = abstract_edges_mapped(sc->ab, in_q1, in_q2, dtype, n, resolution, include_endpoints, in_N,
-                                          N_start, N_max, sc->m_stage + o_hit, sc->m_stage, sc->num_sms,
-                                          sc->own_stream, &grid);
+                                          N_start, N_max, sc->m_stage + o_hit, sc->m_stage, next_done(sc),
+                                          sc->num_sms, sc->own_stream, &grid);
     if (e != cudaSuccess) return cuda_fail(e, "launch edges");
-    e = cudaStreamSynchronize(sc->own_stream);
+    e = wait_done(sc, grid);
     if (e != cudaSuccess) return cuda_fail(e, "kernel execution");
     int bits = 0;
     for (int c = 0; c < grid; c++) bits |= H[c];

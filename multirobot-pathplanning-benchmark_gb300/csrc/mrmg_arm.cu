@@ -1590,7 +1590,10 @@ __global__ void __launch_bounds__(128, 1) arm_small_kernel(ArmDev s, SmallBatch 
     if (stat_pend) atomicAdd(&s_stat[1], stat_pend);
   }
   __syncthreads();
-  if (threadIdx.x < 2) b.stats[2 * blockIdx.x + threadIdx.x] = s_stat[threadIdx.x];
+  if (threadIdx.x == 0) {
+    ((int2*)b.stats)[blockIdx.x] = make_int2(s_stat[0], s_stat[1]);
+    if (b.done.cta) signal_done(b.done);
+  }
 }
 
 // sphere centres for the error-bound check: warp per configuration

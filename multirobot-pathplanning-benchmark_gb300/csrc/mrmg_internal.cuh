@@ -160,6 +160,21 @@ struct LaunchShape {
   int num_sms;
 };
 
+// A synchronous host call's end, told by the kernel itself: each CTA sets its byte
+// of the mapped buffer once its results are there, and the host polls the bytes
+// instead of waiting for the grid to retire and the stream to report it.  Four
+// 7-DoF arms, 5 boxes, one configuration 18.1 -> 15.8 us a call, one edge 22.7 ->
+// 20.2 us; two discs, 1,000 configurations and 1,000 edges 49 -> 45 us for both.
+// (One word, stored by the last CTA to count itself in: 16.4 and 21.2 us.)
+struct CallDone {
+  uint8_t* cta;          // mapped [grid], or null: the host waits for the stream
+};
+// by one thread of the CTA, after a barrier behind which no thread writes results
+__device__ __forceinline__ void signal_done(const CallDone& d) {
+  __threadfence_system();
+  *(volatile uint8_t*)(d.cta + blockIdx.x) = 1;
+}
+
 // one small synchronous batch (arm_small): inputs, hits and statistics in
 // mapped pinned host memory, per-edge flags in device memory
 constexpr int kSmallWarps = 4;   // warps per CTA of the small-batch kernel
@@ -178,6 +193,7 @@ struct SmallBatch {
   int* stats;            // [2 * CTAs] per CTA: configurations evaluated, FP64 decisions
   unsigned* flags;       // [n]     device: edge e collides in this call iff flags[e] == epoch
   unsigned epoch;
+  CallDone done;
 };
 
 // Raises a kernel's dynamic shared-memory limit to the device's opt-in
@@ -261,10 +277,11 @@ int abstract_prepare(const AbstractDev& s);   // kernel attributes, once per sce
 // single launches on caller-visible (e.g. mapped host) buffers, no counters;
 // the edge kernel reports its error bits per CTA in cta_err[grid] (plain stores)
 cudaError_t abstract_configs_mapped(const AbstractDev& s, const void* q, int dtype, long long n, uint8_t* out,
-                                    int num_sms, cudaStream_t st);
+                                    const CallDone& done, int num_sms, cudaStream_t st, int* grid_out);
 cudaError_t abstract_edges_mapped(const AbstractDev& s, const void* q1, const void* q2, int dtype, long long n,
                                   double res, int incl, const long long* Np, long long N_start, long long N_max,
-                                  uint8_t* out, uint8_t* cta_err, int num_sms, cudaStream_t st, int* grid_out);
+                                  uint8_t* out, uint8_t* cta_err, const CallDone& done, int num_sms, cudaStream_t st,
+                                  int* grid_out);
 
 cudaError_t arm_configs(const ArmDev& s, const void* q, int dtype, long long n, uint8_t* out,
                         const CallScratch& sc, const LaunchShape& ls, int full, cudaStream_t st);
