@@ -1203,10 +1203,10 @@ cudaError_t wait_done(mrmg_scene* sc, int grid) {
 
 // launch the single-launch kernel on the mapped buffer, wait, and fill the
 // scene's statistics from the per-CTA slots
-int run_small(mrmg_scene* sc, const ArmDev& a, SmallBatch& b) {
+int run_small(mrmg_scene* sc, const ArmDev& a, SmallBatch& b, const SmallRows& rows) {
   int grid = 0;
   b.done = next_done(sc);
-  cudaError_t e = arm_small(a, b, sc->num_sms, sc->own_stream, &grid);
+  cudaError_t e = arm_small(a, b, rows, sc->num_sms, sc->own_stream, &grid);
   if (e != cudaSuccess) return cuda_fail(e, "launch small batch");
   e = wait_done(sc, grid);
   if (e != cudaSuccess) return cuda_fail(e, "kernel execution");
@@ -1271,10 +1271,16 @@ int mrmg_is_collision_free_host(mrmg_scene* sc, const void* h_q, int32_t dtype, 
     SmallBatch b{};
     b.n = (int)n; b.items = (int)n; b.edges = 0; b.dtype = dtype; b.incl = 0; b.N_start = 0;
     b.q1 = in_q; b.hit = sc->m_stage + o_hit; b.stats = (int*)sc->m_stage;
+    SmallRows rows;
+    if (qbytes <= sizeof(rows)) {
+      std::memcpy(rows.b, h_q, qbytes);
+      b.inl = 1;
+      b.q1 = nullptr;
+    }
     b.flags = sc->d_small_flags;
     rc = next_epoch(sc, &b.epoch);
     if (rc) return rc;
-    rc = run_small(sc, a, b);
+    rc = run_small(sc, a, b, rows);
     if (rc) return rc;
     for (long long i = 0; i < n; i++) h_out[i] = H[o_hit + i] ? 0 : 1;
     return MRMG_OK;
@@ -1391,10 +1397,20 @@ int mrmg_is_edge_collision_free_host(mrmg_scene* sc, const void* h_q1, const voi
     b.off = (const int*)(sc->m_stage + o_off); b.N = (const int*)(sc->m_stage + o_N32);
     b.q1 = in_q1; b.q2 = in_q2; b.hit = sc->m_stage + o_hit;
     b.stats = (int*)sc->m_stage;
+    SmallRows rows;
+    const size_t r_N = 4 * ((size_t)n + 1), r_q1 = pad16(r_N + 4 * (size_t)n), r_q2 = pad16(r_q1 + qbytes);
+    if (r_q2 + qbytes <= sizeof(rows)) {
+      std::memcpy(rows.b, H + o_off, r_N);
+      std::memcpy(rows.b + r_N, H + o_N32, 4 * (size_t)n);
+      std::memcpy(rows.b + r_q1, h_q1, qbytes);
+      std::memcpy(rows.b + r_q2, h_q2, qbytes);
+      b.inl = 1;
+      b.off = nullptr; b.N = (const int*)r_N; b.q1 = (const void*)r_q1; b.q2 = (const void*)r_q2;
+    }
     b.flags = sc->d_small_flags;
     rc = next_epoch(sc, &b.epoch);
     if (rc) return rc;
-    rc = run_small(sc, sc->arm, b);
+    rc = run_small(sc, sc->arm, b, rows);
     if (rc) return rc;
     for (long long i = 0; i < n; i++) h_out[i] = H[o_hit + i] ? 0 : 1;
     return MRMG_OK;

@@ -1514,7 +1514,14 @@ __global__ void __launch_bounds__(kScanThreads, 5) arm_scan_kernel(ArmDev s, con
 // byte; positions of an edge already seen to collide are skipped.
 // ---------------------------------------------------------------------------
 template <int GPL, int SPG>
-__global__ void __launch_bounds__(128, 1) arm_small_kernel(ArmDev s, SmallBatch b) {
+__global__ void __launch_bounds__(128, 1) arm_small_kernel(const __grid_constant__ ArmDev s, SmallBatch b,
+                                                       const __grid_constant__ SmallRows rows) {
+  if (b.inl) {
+    b.off = (const int*)(rows.b + (size_t)b.off);
+    b.N = (const int*)(rows.b + (size_t)b.N);
+    b.q1 = rows.b + (size_t)b.q1;
+    b.q2 = rows.b + (size_t)b.q2;
+  }
   extern __shared__ __align__(16) unsigned char smem_arm[];
   __shared__ int s_stat[2];
   ArmSmem t;
@@ -1552,11 +1559,12 @@ __global__ void __launch_bounds__(128, 1) arm_small_kernel(ArmDev s, SmallBatch 
     const long long N = b.N[e];
     const long long iv = bfs_at(N, b.N_start + (it - b.off[e]));
     if (!b.incl && (iv == 0 || iv == N - 1)) continue;
-    if (flags[e] == b.epoch) continue;                      // another position already collides
+    const unsigned seen = flags[e];
     EdgeSourceDF sdf;
     float mloc;
     bool nanf;
     load_edge(b.q1, b.q2, b.dtype, e, D, lane, &sdf, &mloc, &nanf);
+    if (seen == b.epoch) continue;                          // another position already collides
     sdf.nm1 = (float)(int)(N - 1);                          // N <= 2^24 on this path
     sdf.rn = __frcp_rn(sdf.nm1);
     sdf.fi = (float)(int)iv;
@@ -2018,7 +2026,8 @@ bool arm_small_ok(const ArmDev& s) {
   return arm_gpl_for_spg(s.SPG) > 0 && smem_pass(s, kSmallWarps, true) + 64 <= (size_t)227 * 1024;   // + static shared memory
 }
 
-cudaError_t arm_small(const ArmDev& s, const SmallBatch& b, int num_sms, cudaStream_t st, int* grid_out) {
+cudaError_t arm_small(const ArmDev& s, const SmallBatch& b, const SmallRows& rows, int num_sms, cudaStream_t st,
+                      int* grid_out) {
   *grid_out = 0;
   if (b.items <= 0) return cudaSuccess;
   const int gpl = arm_gpl_for_spg(s.SPG);
@@ -2029,7 +2038,7 @@ cudaError_t arm_small(const ArmDev& s, const SmallBatch& b, int num_sms, cudaStr
   *grid_out = grid;
 #define MRMG_ARM_SMALL(G_, S_)                                                                     \
   if (gpl == G_ && s.SPG == S_) {                                                                  \
-    arm_small_kernel<G_, S_><<<grid, warps * 32, smem, st>>>(s, b);                                \
+    arm_small_kernel<G_, S_><<<grid, warps * 32, smem, st>>>(s, b, rows);                          \
     return cudaGetLastError();                                                                     \
   }
   MRMG_ARM_SMALL(1, 6)
