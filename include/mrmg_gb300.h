@@ -177,7 +177,7 @@ int mrmg_scene_info(const mrmg_scene *scene, int64_t *out7, double *out_band);
  * variable MRMG_STAGE_HOST_INPUTS=1 asks for staged copies. */
 int mrmg_host_access(int32_t *out);
 
-/* The serving batcher's input gather (serving.py): one launch copies every
+/* The input gather of a serving step: one launch copies every
  * planner instance's request arrays from host memory into a step's device
  * buffers -- configurations into rows [0, ccap) of both d_q1 and d_q2 (the
  * edge q -> q), edge starts and ends into rows [ccap, ccap + ecap), edge step
@@ -194,6 +194,18 @@ int mrmg_host_access(int32_t *out);
  * copying.  Asynchronous.  No reference counterpart. */
 int mrmg_serving_gather(const void *h_table, int32_t max_src, int32_t q_dim, int64_t ccap, int64_t ecap,
                         float *d_q1, float *d_q2, int64_t *d_N, int32_t *d_err, void *stream);
+
+/* A serving step's gather and edge checks (arm scenes): mrmg_serving_gather
+ * into d_q1 / d_q2 / d_N, then the checks of every row as
+ * mrmg_is_edge_collision_free_batch with MRMG_FLAG_ASYNC, FP32 endpoints,
+ * step counts d_N and d_out.  Large steps are gathered in parts on
+ * gather_stream while `stream` scans the parts before; both are joined on
+ * `stream` (also under capture).  *d_gather_err is zeroed first.  Call it once
+ * outside a capture before capturing it (events, scratch).  No reference
+ * counterpart. */
+int mrmg_serving_check(mrmg_scene *scene, const void *h_table, int32_t max_src, int64_t ccap, int64_t ecap,
+                       float *d_q1, float *d_q2, int64_t *d_N, int32_t *d_gather_err, int32_t include_endpoints,
+                       uint8_t *d_out, void *stream, void *gather_stream);
 
 /* The collision kernels stage a scene's FP32 tables (boxes, spheres, frames,
  * group pairs) into shared memory with one bulk asynchronous copy (the TMA

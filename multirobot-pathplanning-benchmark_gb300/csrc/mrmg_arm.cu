@@ -1191,7 +1191,7 @@ __global__ void __launch_bounds__(256, GPL == 1 ? 3 : (GPL == 2 ? 2 : 1)) arm_ed
 // warp); a warp takes new ones from the queue when half of its places are free,
 // which keeps the set-up (an edge's step count, base frames) to dense rounds.
 // ---------------------------------------------------------------------------
-constexpr int kScanThreads = 128;
+constexpr int kScanThreads = 128, kScanCtas = 5;
 constexpr int kMaxScanMask = 16384;   // (group, box) reach tests per CTA, at most; beyond: every box is tested
 
 __host__ __device__ inline size_t scan_smem(const ArmDev& s) {
@@ -1229,10 +1229,10 @@ __device__ __forceinline__ void scan_joint(const void* q1, const void* q2, int d
 }
 
 template <int SPG, bool EDGES>
-__global__ void __launch_bounds__(kScanThreads, 5) arm_scan_kernel(ArmDev s, const void* q1, const void* q2, int dtype,
-                                                                   long long n, float res32, int incl,
+__global__ void __launch_bounds__(kScanThreads, kScanCtas) arm_scan_kernel(ArmDev s, const void* q1, const void* q2, int dtype,
+                                                                   long long lo, long long hi, float res32, int incl,
                                                                    const long long* Np, long long N_start,
-                                                                   long long N_max, uint8_t* out, int* ctr,
+                                                                   long long N_max, uint8_t* out, int* ctr, int queue,
                                                                    SurvivorEdge* surv) {
   extern __shared__ __align__(16) unsigned char smem_arm[];
   __shared__ int s_gbeg[kMaxRobots + 1], s_joint[kMaxRobots];
@@ -1298,14 +1298,14 @@ __global__ void __launch_bounds__(kScanThreads, 5) arm_scan_kernel(ArmDev s, con
     const int free_places = __popc(idle) / R;
     if (!exhausted && 2 * free_places >= places) {
       long long base = 0;
-      if (lane == 0) base = atomicAdd(&ctr[kCtrScan], free_places);
+      if (lane == 0) base = lo + atomicAdd(&ctr[queue], free_places);
       base = __shfl_sync(MRMG_FULL, base, 0);
-      exhausted = base + free_places >= n;
+      exhausted = base + free_places >= hi;
       const bool fresh = used && idx < 0;
       bool none = false;      // an edge with no checked position: free
       if (fresh) {
         const long long c = base + __popc(idle & ((1u << (place * R)) - 1u)) / R;
-        if (c < n) {
+        if (c < hi) {
           idx = c;
           bad = false;
           kc = 0;
@@ -1958,17 +1958,19 @@ static bool use_scan(const ArmDev& s, long long n, int full) {
          scan_smem(s) <= (size_t)100 * 1024;
 }
 
+bool arm_edges_scan(const ArmDev& s, long long n, int full) { return use_scan(s, n, full); }
+
 template <bool EDGES>
-static cudaError_t launch_scan(const ArmDev& s, const void* q1, const void* q2, int dtype, long long n, double res,
-                               int incl, const long long* Np, long long N_start, long long N_max, uint8_t* out,
-                               const CallScratch& sc, int num_sms, cudaStream_t st) {
+static cudaError_t launch_scan(const ArmDev& s, const void* q1, const void* q2, int dtype, long long lo, long long hi,
+                               double res, int incl, const long long* Np, long long N_start, long long N_max,
+                               uint8_t* out, const CallScratch& sc, int queue, int ctas, cudaStream_t st) {
   const size_t smem = scan_smem(s);
   const int per_cta = kScanThreads / 32 * (32 / s.R);
-  const int grid = (int)std::max(1ll, std::min((n + per_cta - 1) / per_cta, (long long)num_sms * 5));
+  const int grid = (int)std::max(1ll, std::min((hi - lo + per_cta - 1) / per_cta, (long long)ctas));
 #define MRMG_ARM_SCAN(S_)                                                                          \
   if (s.SPG == S_) {                                                                               \
-    arm_scan_kernel<S_, EDGES><<<grid, kScanThreads, smem, st>>>(s, q1, q2, dtype, n, (float)res, incl, Np, N_start, \
-                                                                 N_max, out, sc.ctr, sc.surv);     \
+    arm_scan_kernel<S_, EDGES><<<grid, kScanThreads, smem, st>>>(s, q1, q2, dtype, lo, hi, (float)res, incl, Np,    \
+                                                                 N_start, N_max, out, sc.ctr, queue, sc.surv); \
     return cudaGetLastError();                                                                     \
   }
   MRMG_ARM_SCAN(6)
@@ -1986,7 +1988,7 @@ cudaError_t arm_configs(const ArmDev& s, const void* q, int dtype, long long n, 
   int grid = (int)std::max(1ll, std::min(want, (long long)ls.ctas));
   const bool scan = use_scan(s, n, full);
   cudaError_t e = cudaSuccess;
-  if (scan) e = launch_scan<false>(s, q, nullptr, dtype, n, 0.0, 0, nullptr, 0, -1, out, sc, ls.num_sms, st);
+  if (scan) e = launch_scan<false>(s, q, nullptr, dtype, 0, n, 0.0, 0, nullptr, 0, -1, out, sc, kCtrScan, ls.num_sms * kScanCtas, st);
   if (e == cudaSuccess) e = launch_configs<false>(s, gpl, q, dtype, n, out, sc, grid, ls.warps, smem1, full, scan, st);
   if (e != cudaSuccess) return e;
   return launch_configs<true>(s, gpl, q, dtype, n, out, sc, ls.num_sms * kResolveCtas, kResolveWarps,
@@ -1996,14 +1998,25 @@ cudaError_t arm_configs(const ArmDev& s, const void* q, int dtype, long long n, 
 cudaError_t arm_edges(const ArmDev& s, const void* q1, const void* q2, int dtype, long long n,
                       double res, int incl, const long long* Np, long long N_start,
                       long long N_max, uint8_t* out, const CallScratch& sc,
-                      const LaunchShape& ls, int full, cudaStream_t st) {
+                      const LaunchShape& ls, int full, cudaStream_t st, const PartFeed* feed) {
   const int gpl = arm_gpl_for_spg(s.SPG);
   const size_t smem1 = smem_pass(s, ls.warps, false);
   long long want = (n + ls.warps - 1) / ls.warps;
   int grid = (int)std::max(1ll, std::min(want, (long long)ls.ctas));
   const bool scan = use_scan(s, n, full);
   cudaError_t e = cudaSuccess;
-  if (scan) e = launch_scan<true>(s, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, sc, ls.num_sms, st);
+  const int parts = feed ? feed->parts : 1;
+  long long lo = 0;
+  for (int j = 0; j < parts && e == cudaSuccess; j++) {
+    if (feed) e = cudaStreamWaitEvent(st, feed->ready[j], 0);
+    const long long hi = feed ? feed->end[j] : n;
+    // beside the copy of the next part, the scan leaves it a CTA's registers
+    if (scan && e == cudaSuccess && hi > lo)
+      e = launch_scan<true>(s, q1, q2, dtype, lo, hi, res, incl, Np, N_start, N_max, out, sc,
+                            j ? kCtrScanParts + j : kCtrScan, ls.num_sms * (j + 1 < parts ? kScanCtas - 1 : kScanCtas),
+                            st);
+    lo = hi;
+  }
   if (e == cudaSuccess)
     e = launch_edges<false>(s, gpl, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, sc, grid, ls.warps, smem1,
                             full, scan, st);

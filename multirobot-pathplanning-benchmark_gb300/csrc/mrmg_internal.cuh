@@ -136,7 +136,9 @@ constexpr int kCtrL1 = 6, kCtrMaxJ = 7, kCtrQueueB = 8;
 constexpr int kCtrScan = 12, kCtrListed = 13;   // scan: its queue, and the items listed for the warp kernels
 constexpr int kCtrPendLost = 11;   // pending positions did not fit the list
 constexpr int kCtrDoneB = 10;   // CTAs of the last phase-B launch that have finished
-constexpr int kNumCtr = 16;
+constexpr int kCtrScanParts = 16;   // the queues of the scans of a batch's further parts (PartFeed)
+constexpr int kMaxParts = 4;
+constexpr int kNumCtr = kCtrScanParts + kMaxParts;
 
 // an edge that survived its first checked configuration: its remaining
 // BFS positions [p_next, nmax) are dealt to all warps
@@ -153,6 +155,14 @@ struct CallScratch {
   long long* pend;      // pending item list
   SurvivorEdge* surv;   // surviving edges (arm edge checks)
   long long pend_cap;
+};
+
+// A batch whose rows arrive in parts, copied on another stream: the scan of a part
+// waits for that part only, so it runs while the next one is copied.
+struct PartFeed {
+  int parts;
+  long long end[kMaxParts];       // the parts' last rows, exclusive
+  cudaEvent_t ready[kMaxParts];
 };
 
 struct LaunchShape {
@@ -228,8 +238,8 @@ cudaError_t arm_penetration(const ArmDev& s, const void* q, int dtype, long long
                             cudaStream_t st);
 
 // the serving batcher's gather of host request arrays (mrmg_serving_gather)
-cudaError_t serving_gather(const void* table, int max_src, int D, long long ccap, long long ecap, float* q1,
-                           float* q2, long long* N, int* err, cudaStream_t st);
+cudaError_t serving_gather(const void* table, int max_src, int D, long long ccap, long long ecap, long long lo,
+                           long long hi, float* q1, float* q2, long long* N, int* err, int num_sms, cudaStream_t st);
 
 // whether every arm kernel's shared memory fits a CTA with this tuning
 bool arm_tuning_fits(const ArmDev& s);
@@ -299,7 +309,8 @@ cudaError_t arm_configs(const ArmDev& s, const void* q, int dtype, long long n, 
 cudaError_t arm_edges(const ArmDev& s, const void* q1, const void* q2, int dtype, long long n,
                       double res, int incl, const long long* Np, long long N_start,
                       long long N_max, uint8_t* out, const CallScratch& sc,
-                      const LaunchShape& ls, int full, cudaStream_t st);
+                      const LaunchShape& ls, int full, cudaStream_t st, const PartFeed* feed = nullptr);
+bool arm_edges_scan(const ArmDev& s, long long n, int full);   // the batch takes the scan: its rows may come in parts
 bool arm_small_ok(const ArmDev& s);   // the single-launch kernel fits the scene's shared memory
 cudaError_t arm_small(const ArmDev& s, const SmallBatch& b, const SmallRows& rows, int num_sms, cudaStream_t st,
                       int* grid_out);

@@ -18,9 +18,10 @@ one CUDA graph launch:
 The graph brings the step's endpoints and counts to the device, runs the
 persistent edge pipeline once over the whole step, and copies the verdicts
 back.  Where the device reads pageable host memory (GB300 over its coherent
-host link; ``mrmg_host_access``), the graph's first launch gathers the
-requests' own arrays from host memory through a table of their addresses
-(``mrmg_serving_gather``): no host packing pass and no staging copy.
+host link; ``mrmg_host_access``), the graph gathers the requests' own arrays
+from host memory through a table of their addresses, large steps in parts on a
+second stream beside the scan of the parts before (``mrmg_serving_check``): no
+host packing pass and no staging copy.
 Elsewhere the requests are packed into pinned staging buffers on a thread
 pool and copied.  The staging buffers hold FP32 endpoints (half the copy of FP64): the
 verdicts (and step counts N) are the reference's for the FP32 values, so
@@ -56,8 +57,8 @@ def edge_steps(q1: np.ndarray, q2: np.ndarray, resolution: float) -> np.ndarray:
 
 class _StepGraph:
     """One capacity bucket: device buffers, one graph, and either pinned
-    host staging (packed) or a gather table (direct: the graph's first launch
-    reads the requests' own host arrays, mrmg_serving_gather)."""
+    host staging (packed) or a gather table (direct: the graph reads the
+    requests' own host arrays, mrmg_serving_check)."""
 
     def __init__(self, scene: Gb300Scene, ccap: int, ecap: int, include_endpoints: bool, direct: bool = False,
                  max_src: int = 1024):
@@ -93,6 +94,9 @@ class _StepGraph:
         ew = C.c_void_p()
         _lib.check(lib.mrmg_scene_error_word(scene.h, C.byref(ew)))
         self._err_view = torch.as_tensor(_DeviceWord(ew.value), device="cuda")
+        if self.direct:   # modules load and events are made outside the capture (the table is empty: no row is checked)
+            self.gstream = torch.cuda.Stream()
+            self._check()
         with torch.cuda.stream(self.stream):   # modules load outside the capture
             scene.is_edge_collision_free_batch(self.q1[:1], self.q2[:1], 0.0, self.incl, N=self.N[:1],
                                                out=self.out[:1], stream=self.stream)
@@ -101,15 +105,18 @@ class _StepGraph:
         with torch.cuda.graph(self.graph, stream=self.stream):
             self._enqueue()
 
+    def _check(self):
+        """The direct step's gather (in parts, on a second stream) and checks."""
+        _lib.check(self.scene.lib.mrmg_serving_check(self.scene.h, self.table.data_ptr(), self.max_src, self.ccap,
+                                                     self.ecap, self.q1.data_ptr(), self.q2.data_ptr(),
+                                                     self.N.data_ptr(), self.gerr.data_ptr(), int(self.incl),
+                                                     self.out.data_ptr(), self.stream.cuda_stream,
+                                                     self.gstream.cuda_stream), "serving step")
+
     def _enqueue(self):
         s, c = self.stream, self.ccap
         if self.direct:
-            with torch.cuda.stream(s):
-                self.gerr.zero_()
-            _lib.check(self.scene.lib.mrmg_serving_gather(self.table.data_ptr(), self.max_src, self.scene.q_dim,
-                                                          self.ccap, self.ecap, self.q1.data_ptr(), self.q2.data_ptr(),
-                                                          self.N.data_ptr(), self.gerr.data_ptr(), s.cuda_stream),
-                       "serving gather")
+            self._check()
         else:
             with torch.cuda.stream(s):
                 self.q1[:c].copy_(self.cfg_pin, non_blocking=True)
@@ -117,8 +124,8 @@ class _StepGraph:
                 self.q1[c:].copy_(self.e1_pin, non_blocking=True)
                 self.q2[c:].copy_(self.e2_pin, non_blocking=True)
                 self.N.copy_(self.N_pin, non_blocking=True)
-        self.scene.is_edge_collision_free_batch(self.q1, self.q2, 0.0, self.incl, N=self.N, out=self.out, stream=s,
-                                                flags=_lib.MRMG_FLAG_ASYNC)
+            self.scene.is_edge_collision_free_batch(self.q1, self.q2, 0.0, self.incl, N=self.N, out=self.out, stream=s,
+                                                    flags=_lib.MRMG_FLAG_ASYNC)
         with torch.cuda.stream(s):
             self.err.copy_(self._err_view)
             self.out_pin.copy_(self.out, non_blocking=True)
@@ -177,7 +184,7 @@ class ServingBatcher:
                  config_quantum: int = 1 << 16, edge_quantum: int = 1 << 14, direct=None, max_sources: int = 1024):
         """``direct`` (default: where the device reads pageable host memory,
         mrmg_host_access): ``step`` hands the graph a table of the requests'
-        own arrays, which its first launch reads from host memory, instead of
+        own arrays, which it reads from host memory, instead of
         packing them into pinned staging on the host first."""
         if scene.kind != 1:
             raise TypeError("the serving batcher drives arm scenes")
@@ -321,7 +328,7 @@ class ServingBatcher:
 
     def _step_direct(self, t0, cs, e1, e2, Ns, nc, ne) -> StepResult:
         """The step through the gather table: no host copy of the requests;
-        the graph's first launch reads them where they are."""
+        the graph reads them where they are."""
         g = self._graph(nc, ne, direct=True)
         tab = g.table.numpy()
         k = 4
