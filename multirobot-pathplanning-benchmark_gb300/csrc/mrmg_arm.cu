@@ -69,10 +69,19 @@ __host__ __device__ inline size_t warp32_bytes(const ArmDev& s) {
          align16(sizeof(float4) * s.G) + align16(sizeof(uint32_t) * list_cap(s));
 }
 
-// per-warp FP64 work area for pass 2: joint values, cos/sin, sphere centres
+// frames per robot: its base and every link
+__host__ __device__ inline int frame_links(const ArmDev& s) {
+  int m = 0;
+  for (int r = 0; r < s.R; r++) m = s.nl[r] > m ? s.nl[r] : m;
+  return m + 1;
+}
+
+// per-warp FP64 work area for pass 2: joint values, cos/sin, and the links' frames
+// or the sphere centres
 __host__ __device__ inline size_t warp64_bytes(const ArmDev& s) {
+  const size_t frames = (size_t)12 * s.R * frame_links(s), centres = (size_t)3 * s.G * s.SPG;
   return align16(sizeof(double) * s.D) + align16(sizeof(double) * 2 * s.D) +
-         align16(sizeof(double) * 3 * s.G * s.SPG);
+         align16(sizeof(double) * (frames > centres ? frames : centres));
 }
 
 // The FP32 tables into shared memory at `base` (arm_table_layout): one bulk
@@ -213,6 +222,64 @@ __device__ void chain64(const ArmDev& s, const double* wth, const double* wcs, i
       p[i] = __dadd_rn(p[i], __dadd_rn(__dadd_rn(__dmul_rn(r0, ac), __dmul_rn(r1, as)), __dmul_rn(r2, dd)));
     }
   }
+}
+
+// One row (of rotation and position) of the frames of every link of robot r, by
+// chain64's operations in chain64's order: a row needs no other row of its chain.
+// A lane per (robot, row) issues 26 FP64 instructions per joint where a lane per
+// sphere group, which repeats its robot's chain up to its link, issues 63, and
+// the FP64 pipe takes 19 cycles for each, however many lanes are active.  Sphere
+// centres are formed where a test needs one.  The pass over the 4 undecided of
+// 200,000 configurations: 22 -> 15 us, the 14 of 100,000 edges 38 -> 24 us (cold
+// instructions and table reads are what is left).
+// f: [link][row][4] (R row, p).
+__device__ void chain64_row(const ArmDev& s, const double* wth, const double* wcs, int r, int i, double* f) {
+  const double* bp = s.base64 + r * 12;
+  const double* hp = s.dh64 + r * kMaxLinks * 4;
+  double h0 = hp[0], h1 = hp[1], h2 = hp[2], h3 = hp[3];
+  double a[3] = {bp[3 * i], bp[3 * i + 1], bp[3 * i + 2]}, p = bp[9 + i];
+  int jo = s.q_off[r];
+  const int nl = s.nl[r];
+  if (s.base_kind[r] == 1) {
+    if (i < 2) {
+      const double x = wth[jo + i], cs = wcs[2 * (jo + 2)], sn = wcs[2 * (jo + 2) + 1];
+#pragma unroll
+      for (int j = 0; j < 3; j++)
+        a[j] = i == 0 ? __dsub_rn(__dmul_rn(cs, bp[j]), __dmul_rn(sn, bp[3 + j]))
+                      : __dadd_rn(__dmul_rn(sn, bp[j]), __dmul_rn(cs, bp[3 + j]));
+      p = __dadd_rn(x, i == 0 ? __dsub_rn(__dmul_rn(cs, bp[9]), __dmul_rn(sn, bp[10]))
+                              : __dadd_rn(__dmul_rn(sn, bp[9]), __dmul_rn(cs, bp[10])));
+    }
+    jo += 3;
+  }
+  f += 4 * i;
+  for (int j = 0;; j++, f += 12) {
+    f[0] = a[0]; f[1] = a[1]; f[2] = a[2]; f[3] = p;
+    if (j >= nl) break;
+    const double ad = h0, dd = h1, ca = h2, sa = h3;
+    if (j + 1 < nl) {   // the next link's parameters are on their way meanwhile
+      hp += 4;
+      h0 = hp[0]; h1 = hp[1]; h2 = hp[2]; h3 = hp[3];
+    }
+    const double cs = wcs[2 * (jo + j)], sn = wcs[2 * (jo + j) + 1];
+    const double sca = __dmul_rn(sn, ca), cca = __dmul_rn(cs, ca);
+    const double ssa = __dmul_rn(sn, sa), csa = __dmul_rn(cs, sa);
+    const double ac = __dmul_rn(ad, cs), as = __dmul_rn(ad, sn);
+    const double r0 = a[0], r1 = a[1], r2 = a[2];
+    a[0] = __dadd_rn(__dmul_rn(r0, cs), __dmul_rn(r1, sn));
+    a[1] = __dadd_rn(__dsub_rn(__dmul_rn(r1, cca), __dmul_rn(r0, sca)), __dmul_rn(r2, sa));
+    a[2] = __dadd_rn(__dsub_rn(__dmul_rn(r0, ssa), __dmul_rn(r1, csa)), __dmul_rn(r2, ca));
+    p = __dadd_rn(p, __dadd_rn(__dadd_rn(__dmul_rn(r0, ac), __dmul_rn(r1, as)), __dmul_rn(r2, dd)));
+  }
+}
+// centre of sphere slot `slot` of group `gi` (robot | link << 8)
+__device__ __forceinline__ void centre64(const ArmDev& s, const double* frames, int nf, int gi, int slot, double* c) {
+  const double* f = frames + ((gi & 0xff) * nf + (gi >> 8)) * 12;
+  const double* l = s.sph64 + (size_t)slot * 5;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+    c[i] = __dadd_rn(f[4 * i + 3], __dadd_rn(__dadd_rn(__dmul_rn(f[4 * i], l[0]), __dmul_rn(f[4 * i + 1], l[1])),
+                                             __dmul_rn(f[4 * i + 2], l[2])));
 }
 
 // exact sphere-box test (numpy order for 3 coordinates)
@@ -396,8 +463,18 @@ __device__ uint8_t eval_config(const ArmDev& s, const ArmSmem& t, float2* wcs, f
   const bool all_ok = __all_sync(MRMG_FULL, ok);
   if (!RESOLVE && !all_ok) return V_PENDING;
   __syncwarp();
+  // the frames of every link, where the centres of all spheres (tested only if
+  // the FP32 path cannot place them) would go
+  const int nf = RESOLVE ? frame_links(s) : 0;
   if constexpr (RESOLVE) {
-#pragma unroll
+    if (all_ok) {
+      for (int x = lane; x < 3 * s.R; x += 32)
+        chain64_row(s, wth64, wcs64, x / 3, x % 3, wc64 + (size_t)(x / 3) * nf * 12);
+      __syncwarp();
+    }
+  }
+  if (RESOLVE && !all_ok) {
+#pragma unroll 1
     for (int u = 0; u < GPL; u++) {
       const int g = lane + 32 * u;
       if (g < s.G) {
@@ -415,7 +492,7 @@ __device__ uint8_t eval_config(const ArmDev& s, const ArmSmem& t, float2* wcs, f
       }
     }
     __syncwarp();
-    if (!all_ok) return exact_all_collide(s, wc64, lane) ? V_COLLIDE : V_FREE;
+    return exact_all_collide(s, wc64, lane) ? V_COLLIDE : V_FREE;
   }
 
   // --- FP32 chain + sphere centres (and group bound centres) of the owned groups
@@ -498,7 +575,9 @@ __device__ uint8_t eval_config(const ArmDev& s, const ArmSmem& t, float2* wcs, f
                 if (ss < bd.x) coll = true;
                 else if (RESOLVE) {
                   const int slot = g * SPG + v;
-                  coll |= exact_box_hit(wc64 + (size_t)slot * 3, s.box64 + (size_t)b * 6, s.sph64[(size_t)slot * 5 + 4]);
+                  double c64[3];
+                  centre64(s, wc64, nf, t.grp[g], slot, c64);
+                  coll |= exact_box_hit(c64, s.box64 + (size_t)b * 6, s.sph64[(size_t)slot * 5 + 4]);
                 } else {
                   unc = true;
                 }
@@ -628,7 +707,9 @@ __device__ uint8_t eval_config(const ArmDev& s, const ArmSmem& t, float2* wcs, f
               if (ss < bd.x) coll = true;
               else if (RESOLVE) {
                 const int slot = g * SPG + v;
-                coll |= exact_box_hit(wc64 + (size_t)slot * 3, s.box64 + (size_t)b * 6, s.sph64[(size_t)slot * 5 + 4]);
+                double c64[3];
+                centre64(s, wc64, nf, t.grp[g], slot, c64);
+                coll |= exact_box_hit(c64, s.box64 + (size_t)b * 6, s.sph64[(size_t)slot * 5 + 4]);
               } else {
                 unc = true;
               }
@@ -750,8 +831,10 @@ __device__ uint8_t eval_config(const ArmDev& s, const ArmSmem& t, float2* wcs, f
               if (Wl > 0.f && ss < Wl * Wl) coll = true;
               else if (RESOLVE) {
                 const int sa = ga * SPG + v, sb = gb * SPG + w;
-                coll |= exact_pair_hit(wc64 + (size_t)sa * 3, wc64 + (size_t)sb * 3,
-                                       s.sph64[(size_t)sa * 5 + 3], s.sph64[(size_t)sb * 5 + 3]);
+                double ca64[3], cb64[3];
+                centre64(s, wc64, nf, t.grp[ga], sa, ca64);
+                centre64(s, wc64, nf, t.grp[gb], sb, cb64);
+                coll |= exact_pair_hit(ca64, cb64, s.sph64[(size_t)sa * 5 + 3], s.sph64[(size_t)sb * 5 + 3]);
               } else {
                 unc = true;
               }
