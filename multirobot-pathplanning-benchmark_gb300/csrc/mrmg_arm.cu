@@ -877,11 +877,14 @@ template <int GPL, int SPG, bool RESOLVE>
 __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ? 2 : 1))) arm_configs_kernel(ArmDev s, const void* q, int dtype, long long n,
                                                           uint8_t* out, int* ctr, long long* pend, const SurvivorEdge* list,
                                                           int full) {
+  if (RESOLVE) after_previous();
+  else next_may_start();
   // pass 2: as many CTAs stay as there are undecided items for their warps
-  if (RESOLVE && (long long)blockIdx.x * (blockDim.x >> 5) >= ctr[kCtrPending]) return;
+  if (RESOLVE && (long long)blockIdx.x * (blockDim.x >> 5) >= *(volatile int*)&ctr[kCtrPending]) return;
   extern __shared__ __align__(16) unsigned char smem_arm[];
   ArmSmem t;
   stage_tables(s, smem_arm, &t);
+  if (!RESOLVE) after_previous();
   __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   float2* wcs; float* wqv; float4* wsph; double* w64;
@@ -1006,11 +1009,14 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
                                                         long long N_max, uint8_t* out, int* ctr,
                                                         long long* pend, long long pend_cap, SurvivorEdge* surv, int listed,
                                                         int full) {
+  if (RESOLVE) after_previous();
+  else next_may_start();
   // pass 2: as many CTAs stay as there are undecided items for their warps
-  if (RESOLVE && (long long)blockIdx.x * (blockDim.x >> 5) >= ctr[kCtrPending]) return;
+  if (RESOLVE && (long long)blockIdx.x * (blockDim.x >> 5) >= *(volatile int*)&ctr[kCtrPending]) return;
   extern __shared__ __align__(16) unsigned char smem_arm[];
   ArmSmem t;
   stage_tables(s, smem_arm, &t);
+  if (!RESOLVE) after_previous();
   __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   float2* wcs; float* wqv; float4* wsph; double* w64;
@@ -1173,6 +1179,12 @@ __global__ void __launch_bounds__(256, GPL == 1 ? 3 : (GPL == 2 ? 2 : 1)) arm_ed
   // the last launch (j_hi < 0) also finalizes: its last CTA to finish sets the
   // survivors' verdicts (or CTA 0, when the launch has no positions left)
   const bool fin = j_hi < 0;
+  next_may_start();
+  extern __shared__ __align__(16) unsigned char smem_arm[];
+  ArmSmem t;
+  stage_tables(s, smem_arm, &t);
+  after_previous();
+  __syncthreads();
   const int nsv = ctr[kCtrL1];
   const long long maxj = j_hi < 0 ? (long long)ctr[kCtrMaxJ] : min((long long)j_hi, (long long)ctr[kCtrMaxJ]);
   const long long first = (long long)nsv * j_lo;
@@ -1181,10 +1193,6 @@ __global__ void __launch_bounds__(256, GPL == 1 ? 3 : (GPL == 2 ? 2 : 1)) arm_ed
     if (fin && blockIdx.x == 0) finalize_survivors(ctr, surv, out);
     return;
   }
-  extern __shared__ __align__(16) unsigned char smem_arm[];
-  ArmSmem t;
-  stage_tables(s, smem_arm, &t);
-  __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   float2* wcs; float* wqv; float4* wsph; double* w64;
   warp_areas(s, smem_arm, table_bytes(s), wib, false, &wcs, &wqv, &wsph, &w64);
@@ -1204,9 +1212,9 @@ __global__ void __launch_bounds__(256, GPL == 1 ? 3 : (GPL == 2 ? 2 : 1)) arm_ed
     if (id < total) {
       l = (int)(id % nsv);
       const long long j = id / nsv;
-      const long long p = __ldg(&surv[l].p_next) + j;
-      if (p < __ldg(&surv[l].nmax) && (full || !vsurv[l].dead)) {
-        const long long N = __ldg(&surv[l].N);
+      const long long p = surv[l].p_next + j;
+      if (p < surv[l].nmax && (full || !vsurv[l].dead)) {
+        const long long N = surv[l].N;
         const long long c = bfs_at(N, p);
         if (incl || (c != 0 && c != N - 1)) iv = c;
       }
@@ -1219,8 +1227,8 @@ __global__ void __launch_bounds__(256, GPL == 1 ? 3 : (GPL == 2 ? 2 : 1)) arm_ed
       const long long is = __shfl_sync(MRMG_FULL, iv, srcl);
       int dead = (lane == 0 && !full) ? vsurv[ls].dead : 0;   // read once, decide warp-uniformly
       if (__shfl_sync(MRMG_FULL, dead, 0)) continue;          // another warp found its collision
-      const long long e = __ldg(&surv[ls].e);
-      const int N = __ldg(&surv[ls].N);
+      const long long e = surv[ls].e;
+      const int N = surv[ls].N;
       EdgeSourceDF sdf;
       float mloc;
       bool nanf;
@@ -1319,6 +1327,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanCtas) arm_scan_kernel(ArmDe
                                                                    SurvivorEdge* surv) {
   extern __shared__ __align__(16) unsigned char smem_arm[];
   __shared__ int s_gbeg[kMaxRobots + 1], s_joint[kMaxRobots];
+  next_may_start();
   ArmSmem t;
   stage_tables(s, smem_arm, &t);
   float4* bp = (float4*)(smem_arm + table_bytes(s));   // boxes in pairs: centre x x y y, z z / half x x, y y z z
@@ -1904,8 +1913,10 @@ cudaError_t launch_configs(const ArmDev& s, int gpl, const void* q, int dtype, l
 #define MRMG_ARM_CFG(G_, S_)                                                                       \
   if (gpl == G_ && s.SPG == S_) {                                                                  \
     auto k = arm_configs_kernel<G_, S_, RESOLVE>;                                                  \
-    k<<<grid, warps * 32, smem, st>>>(s, q, dtype, n, out, sc.ctr, sc.pend,                         \
-                                      listed ? sc.surv : nullptr, full);                            \
+    const SurvivorEdge* list = listed ? sc.surv : nullptr;                                         \
+    if (RESOLVE || listed)                                                                         \
+      return launch_after(k, grid, warps * 32, smem, st, s, q, dtype, n, out, sc.ctr, sc.pend, list, full); \
+    k<<<grid, warps * 32, smem, st>>>(s, q, dtype, n, out, sc.ctr, sc.pend, list, full);           \
     return cudaGetLastError();                                                                     \
   }
   MRMG_ARM_CFG(1, 6)
@@ -1923,6 +1934,9 @@ cudaError_t launch_edges(const ArmDev& s, int gpl, const void* q1, const void* q
 #define MRMG_ARM_EDGE(G_, S_)                                                                      \
   if (gpl == G_ && s.SPG == S_) {                                                                  \
     auto k = arm_edges_kernel<G_, S_, RESOLVE>;                                                    \
+    if (RESOLVE || listed)                                                                         \
+      return launch_after(k, grid, warps * 32, smem, st, s, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out, \
+                          sc.ctr, sc.pend, sc.pend_cap, sc.surv, listed, full);                    \
     k<<<grid, warps * 32, smem, st>>>(s, q1, q2, dtype, n, res, incl, Np, N_start, N_max, out,     \
                                       sc.ctr, sc.pend, sc.pend_cap, sc.surv, listed, full);                             \
     return cudaGetLastError();                                                                     \
@@ -1959,9 +1973,8 @@ cudaError_t launch_phase_b(const ArmDev& s, int gpl, const void* q1, const void*
 #define MRMG_ARM_PB(G_, S_)                                                                        \
   if (gpl == G_ && s.SPG == S_) {                                                                  \
     grid = std::min(grid, num_sms * phase_b_occupancy<G_, S_>(warps, smem));                       \
-    arm_edges_phase_b<G_, S_><<<grid, warps * 32, smem, st>>>(s, q1, q2, dtype, incl, sc.ctr, sc.surv, full, \
-                                                              j_lo, j_hi, out, sc.pend, sc.pend_cap); \
-    return cudaGetLastError();                                                                     \
+    return launch_after(arm_edges_phase_b<G_, S_>, grid, warps * 32, smem, st, s, q1, q2, dtype, incl, sc.ctr, \
+                        sc.surv, full, j_lo, j_hi, out, sc.pend, sc.pend_cap);                                                                     \
   }
   MRMG_ARM_PB(1, 6)
   MRMG_ARM_PB(2, 5)

@@ -170,6 +170,30 @@ struct LaunchShape {
   int num_sms;
 };
 
+// Chains of kernels on one stream.  launch_after starts a kernel as soon as every
+// CTA of the kernel before it has said next_may_start (or left), so its launch and
+// what it does before after_previous() overlap that kernel's last wave.  Each CTA of
+// such a kernel calls after_previous before it reads or writes what earlier kernels
+// do (and reads that with plain loads, not the non-coherent path).
+// 100,000 cluttered edges (five kernels): 236 -> 227 us; 60,000 mostly free ones
+// 1,666 -> 1,655 us; 200,000 configurations 166 -> 165 us.
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // A synchronous host call's end, told by the kernel itself: each CTA sets its byte
 // of the mapped buffer once its results are there, and the host polls the bytes
 // instead of waiting for the grid to retire and the stream to report it.  Four
