@@ -282,17 +282,21 @@ struct SliceTab {
 // sequential unfused sums of d*d, IEEE sqrt, strict '>' maxima).  The squares,
 // the root and the maxima run on the integer pipes with the same bits
 // (mrmg_exact.cuh), a sum starts with its first square (0 + x = x): per
-// coordinate two FP64 operations are left, a subtraction and an addition.
-template <class Diff>
+// coordinate two FP64 operations are left, a subtraction and an addition.  FAST1:
+// the FP64 instructions instead, whose latency is the shorter where a warp or two
+// per SM compute a handful of distances.
+template <bool FAST1 = false, class Diff>
 __device__ __forceinline__ double square_sum(int s, int e, Diff d) {
   if (s >= e) return 0.0;
-  double acc = square_rn(d(s));
-  for (int k = s + 1; k < e; k++) acc = __dadd_rn(acc, square_rn(d(k)));
+  auto sq = [](double x) { return FAST1 ? __dmul_rn(x, x) : square_rn(x); };
+  double acc = sq(d(s));
+  for (int k = s + 1; k < e; k++) acc = __dadd_rn(acc, sq(d(k)));
   return acc;
 }
-template <class Diff>
+template <bool FAST1 = false, class Diff>
 __device__ __forceinline__ double dist_of(const SliceTab& t, int metric, Diff d) {
-  if (metric == MRMG_METRIC_EUCLIDEAN) return sqrt_rn(square_sum(0, t.end_all, d));
+  auto root = [](double x) { return FAST1 ? __dsqrt_rn(x) : sqrt_rn(x); };
+  if (metric == MRMG_METRIC_EUCLIDEAN) return root(square_sum<FAST1>(0, t.end_all, d));
   if (metric == MRMG_METRIC_MAX) {
     double m = abs64(d(0));
     for (int k = 1; k < t.D; k++) { const double v = abs64(d(k)); if (above(v, m)) m = v; }
@@ -300,7 +304,7 @@ __device__ __forceinline__ double dist_of(const SliceTab& t, int metric, Diff d)
   }
   double red = 0.0;
   for (int i = 0; i < t.A; i++) {
-    const double r = sqrt_rn(square_sum(t.s[i], t.e[i], d));
+    const double r = root(square_sum<FAST1>(t.s[i], t.e[i], d));
     if (i == 0) red = r;
     else if (metric == MRMG_METRIC_SUM_EUCLIDEAN) red = __dadd_rn(red, r);
     else if (above(r, red)) red = r;

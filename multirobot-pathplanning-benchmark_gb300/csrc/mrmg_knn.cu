@@ -187,9 +187,10 @@ inline RowPlan row_plan64(const SliceTab& t, int metric, const void* qs, const v
 // operations in the same order.  One nearest and one radius query on 200,000 nodes
 // (28-D), both calls: 190 us before, 176-185 us with the staging of the results.
 static __device__ __noinline__ double sqrt_call(double s) { return sqrt_rn(s); }
+template <bool FAST1 = false>
 __device__ __forceinline__ double dist_rows(const double* __restrict__ qq, const double* __restrict__ xx,
                                             const SliceTab& t, int metric, RowPlan rows) {
-  if (!rows.n4) return dist_of(t, metric, [&](int j) { return __dsub_rn(qq[j], xx[j]); });
+  if (!rows.n4) return dist_of<FAST1>(t, metric, [&](int j) { return __dsub_rn(qq[j], xx[j]); });
   const double2* q2 = (const double2*)qq;
   const double2* x2 = (const double2*)xx;
   double acc = 0.0, red = 0.0;   // (0 + x = x: a sum may start from 0)
@@ -206,9 +207,10 @@ __device__ __forceinline__ double dist_rows(const double* __restrict__ qq, const
         const double2 qv = __ldg(q2 + b + i);
 #pragma unroll
         for (int c = 0; c < 2; c++) {
-          acc = __dadd_rn(acc, square_rn(__dsub_rn(c ? qv.y : qv.x, c ? xv[i].y : xv[i].x)));
+          const double d = __dsub_rn(c ? qv.y : qv.x, c ? xv[i].y : xv[i].x);
+          acc = __dadd_rn(acc, FAST1 ? __dmul_rn(d, d) : square_rn(d));
           if ((rows.ends >> (2 * (b + i) + c)) & 1u) {   // an agent's last coordinate (euclidean: the last)
-            const double r = sqrt_call(acc);
+            const double r = FAST1 ? __dsqrt_rn(acc) : sqrt_call(acc);
             if (first || above(r, red)) red = r;
             first = false;
             acc = 0.0;
@@ -217,6 +219,26 @@ __device__ __forceinline__ double dist_rows(const double* __restrict__ qq, const
       }
   }
   return red;
+}
+
+// The warp's (distance key, index) pairs, a lane each (none: infinity, 0x7fffffff),
+// sorted; the first k are written.
+__device__ __forceinline__ void write_sorted(long long d, int id, int lane, int k, long long* out_idx, double* out_dist) {
+#pragma unroll
+  for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+    for (int o = size >> 1; o; o >>= 1) {
+      const long long od = __shfl_xor_sync(MRMG_FULL, d, o);
+      const int oi = __shfl_xor_sync(MRMG_FULL, id, o);
+      const bool less = od < d || (od == d && oi < id);             // the other lane's comes first
+      const bool low = ((lane & o) == 0) == ((lane & size) == 0);   // this lane takes the first of the two
+      if (less == low && (od != d || oi != id)) { d = od; id = oi; }
+    }
+  if (lane < k) {
+    const bool none = id == 0x7fffffff;
+    out_idx[lane] = none ? -1 : id;
+    out_dist[lane] = none ? __longlong_as_double(0x7ff0000000000000ll) : __longlong_as_double(d);
+  }
 }
 
 // q32 / x32: FP32 copies (rounded to nearest) of the FP64 rows qq / xx
@@ -606,16 +628,30 @@ __global__ void knn_split32_merge_kernel(const double* __restrict__ qs, const lo
         sid[w++] = cand_idx[it * k + r];
     __syncwarp();
     // FP64 re-rank, one candidate per lane; (distance, index) order
+    const double* qq = qs + q * t.D;
+    const double* xb = nodes + mode_beg[m] * t.D;
+    if (ncand <= 32 && k <= 32) {
+      // sorted across the lanes, in FP64 instructions (one warp waits for their
+      // latency here): k = 16 of one query on 12,500 nodes 104 -> 94 us a call
+      long long d = 0x7ff0000000000000ll;
+      int id = 0x7fffffff;
+      if (lane < ncand) {
+        id = sid[lane];
+        d = dkey(dist_rows<true>(qq, xb + (long long)id * t.D, t, metric, rows));
+        if (d > 0x7ff0000000000000ll) { d = 0x7ff0000000000000ll; id = 0x7fffffff; }   // (NaN)
+      }
+      write_sorted(d, id, lane, k, out_idx + q * k, out_dist + q * k);
+      __syncwarp();
+      continue;
+    }
     long long td[KM];
     long long ti[KM];
 #pragma unroll
     for (int i = 0; i < KM; i++) { td[i] = 0x7ff0000000000000ll; ti[i] = 0x7fffffffffffffffll; }
-    const double* qq = qs + q * t.D;
-    const double* xb = nodes + mode_beg[m] * t.D;
     for (int x = lane; x < ncand; x += 32) {
       const long long id = sid[x];
       const double* xx = xb + id * t.D;
-      const long long d = dkey(dist_rows(qq, xx, t, metric, rows));
+      const long long d = dkey(dist_rows<true>(qq, xx, t, metric, rows));
       if (d < td[k - 1] || (d == td[k - 1] && id < ti[k - 1])) {
 #pragma unroll
         for (int i = KM - 1; i > 0; i--) {
@@ -1512,21 +1548,7 @@ __global__ void __launch_bounds__(32 * kMergeWarps, 4) knn_merge_kernel(const do
         d = dkey(dist_rows(qq, nodes + (mode_beg[m] + id) * t.D, t, metric, rows));
         if (!(d < 0x7ff0000000000000ll)) { d = 0x7ff0000000000000ll; id = 0x7fffffff; }   // (an infinite distance is no neighbour)
       }
-#pragma unroll
-      for (int size = 2; size <= 32; size <<= 1)
-#pragma unroll
-        for (int o = size >> 1; o; o >>= 1) {
-          const long long od = __shfl_xor_sync(MRMG_FULL, d, o);
-          const int oi = __shfl_xor_sync(MRMG_FULL, id, o);
-          const bool less = od < d || (od == d && oi < id);          // the other lane's comes first
-          const bool low = ((lane & o) == 0) == ((lane & size) == 0);   // this lane takes the first of the two
-          if (less == low && (od != d || oi != id)) { d = od; id = oi; }
-        }
-      if (lane < k) {
-        const bool none = id == 0x7fffffff;
-        out_idx[q * k + lane] = none ? -1 : id;
-        out_dist[q * k + lane] = none ? DINF : __longlong_as_double(d);
-      }
+      write_sorted(d, id, lane, k, out_idx + q * k, out_dist + q * k);
       continue;
     }
     long long td[16];
@@ -1738,7 +1760,9 @@ __global__ void near_dist_kernel(const double* __restrict__ qs, long long Q, con
     const long long q = owner_of(offs, Q, p);
     const double* qq = qs + q * t.D;
     const double* xx = nodes + (mode_beg[q_mode[q]] + out_idx[p]) * t.D;
-    out_dist[p] = dist_rows(qq, xx, t, metric, rows);
+    // a warp or two: the FP64 instructions' latency is shorter (10.1 -> 9.4 us); more:
+    // their pipe is what is scarce
+    out_dist[p] = total <= 64 ? dist_rows<true>(qq, xx, t, metric, rows) : dist_rows(qq, xx, t, metric, rows);
   }
 }
 
