@@ -474,7 +474,7 @@ def run_gb300(args):
             "warmup": args.warmup, "ms_per_step": total_ms / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32+f64", "data": "synthetic",
             "config": bench_config(world, n),
-            "form": "batched, CUDA-graph captured (counter reset, phase A, phase B1, phase B2 + finalize, FP64 "
+            "form": "batched, CUDA-graph captured (counter reset, scan, phase A, phase B1, phase B2 + finalize, FP64 "
                     "re-check pass, status copy)",
             "verdict_mismatches": mism,
             "clocks": clk,
@@ -492,7 +492,7 @@ def run_gb300(args):
                                        "copied back"},
             "e2e_batch_call": {"value": call_e2e, "unit": UNIT,
                                "api": "Gb300ArmEnvironment.batch_is_edge_collision_free(pinned tensors)"},
-            "gpu_launches": 4 * args.steps,
+            "gpu_launches": 5 * args.steps,   # scan, phase A, B1, B2, FP64 pass
             "wall_s_timed": t_wall,
             "autotune": tune,
         }

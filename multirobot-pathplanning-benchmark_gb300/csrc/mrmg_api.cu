@@ -1363,6 +1363,7 @@ int mrmg_is_collision_free_host(mrmg_scene* sc, const void* h_q, int32_t dtype, 
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
   CallScratch cs{sc->d_ctr, sc->d_pend, sc->d_surv, sc->pend_cap};
   LaunchShape ls = shape(sc);
+  ls.host_rows = sc->pageable;
   if (sc->kind == 0) {
     AbstractDev ab = sc->ab;
     ab.sph_batch_form = (flags & MRMG_FLAG_BATCH_FORM) ? 1 : 0;
@@ -1498,6 +1499,7 @@ int mrmg_is_edge_collision_free_host(mrmg_scene* sc, const void* h_q1, const voi
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
   CallScratch cs{sc->d_ctr, sc->d_pend, sc->d_surv, sc->pend_cap};
   LaunchShape ls = shape(sc);
+  ls.host_rows = sc->pageable;
   e = sc->kind == 0
           ? abstract_edges(sc->ab, k_q1, k_q2, dtype, n, resolution, include_endpoints, dN, N_start, N_max,
                            Dv + o_hit, cs, ls, st)

@@ -2048,7 +2048,10 @@ int arm_prepare(const ArmDev& s, int warps) {
 // them for its lanes.  Measured, four arms, uniform configurations (before -> with
 // the scan): 200,000 among 50, 36, 22, 20 boxes 309 -> 197, 334 -> 230, 344 ->
 // 249, 378 -> 351 us, among 5 boxes 417 -> 499 us; 40,000 among 50, 36, 22 146 ->
-// 141, 146 -> 149, 157 -> 146 us; 10,000 among 50 89 -> 105 us.
+// 141, 146 -> 149, 157 -> 146 us; 10,000 among 50 89 -> 105 us.  Rows that are read
+// in place from host memory go without it (LaunchShape::host_rows): its lanes read
+// joint by joint, and what it lists is read again over the link; 100,000 edges from
+// numpy arrays 242 us without, 285 us with it.
 constexpr long long kScanMinLanes = 1ll << 18;
 constexpr int kScanMinBoxes = 16;
 static bool use_scan(const ArmDev& s, long long n, int full) {
@@ -2084,7 +2087,7 @@ cudaError_t arm_configs(const ArmDev& s, const void* q, int dtype, long long n, 
   const size_t smem1 = smem_pass(s, ls.warps, false);
   long long want = (n + (long long)ls.warps * s.cfg_chunk - 1) / ((long long)ls.warps * s.cfg_chunk);
   int grid = (int)std::max(1ll, std::min(want, (long long)ls.ctas));
-  const bool scan = use_scan(s, n, full);
+  const bool scan = use_scan(s, n, full) && !ls.host_rows;
   cudaError_t e = cudaSuccess;
   if (scan) e = launch_scan<false>(s, q, nullptr, dtype, 0, n, 0.0, 0, nullptr, 0, -1, out, sc, kCtrScan, ls.num_sms * kScanCtas, st);
   if (e == cudaSuccess) e = launch_configs<false>(s, gpl, q, dtype, n, out, sc, grid, ls.warps, smem1, full, scan, st);
@@ -2101,7 +2104,7 @@ cudaError_t arm_edges(const ArmDev& s, const void* q1, const void* q2, int dtype
   const size_t smem1 = smem_pass(s, ls.warps, false);
   long long want = (n + ls.warps - 1) / ls.warps;
   int grid = (int)std::max(1ll, std::min(want, (long long)ls.ctas));
-  const bool scan = use_scan(s, n, full);
+  const bool scan = use_scan(s, n, full) && !ls.host_rows;
   cudaError_t e = cudaSuccess;
   const int parts = feed ? feed->parts : 1;
   long long lo = 0;

@@ -168,6 +168,7 @@ struct PartFeed {
 struct LaunchShape {
   int ctas, warps;   // persistent grid
   int num_sms;
+  bool host_rows = false;   // the rows are read in place from host memory: once, by whole warps (no scan)
 };
 
 // Chains of kernels on one stream.  launch_after starts a kernel as soon as every
