@@ -1097,25 +1097,41 @@ __global__ void __launch_bounds__(32 * kPackRows) knn_pack_queries_kernel(
   float* rows = (float*)(tile + kQTileBytes);
   const int D = st.D;
   const long long qid = r < it.qn ? qorder[it.q0 + r] : -1;
+  // a lane per coordinate: the row's, or the agents' one agent after another (at
+  // most 28; their slices may lie anywhere in a longer row)
+  int coord = lane < D ? lane : -1, first[4] = {0, 0, 0, 0};
+  if (st.fmt != KNN_FMT_EUCL) {
+    coord = -1;
+    int at = 0;
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+      if (a < st.A) {
+        first[a] = at;
+        const int j = lane - at, d = st.agent_e[a] - st.agent_s[a];
+        if (j >= 0 && j < d) coord = st.agent_s[a] + j;
+        at += d;
+      }
+  }
   double x = 0.0;
-  if (qid >= 0 && lane < D) x = qs[qid * D + lane];
+  if (qid >= 0 && coord >= 0) x = qs[qid * D + coord];
   float hi, lo;
   split2(x, &hi, &lo);
   float a1[2], a2[2];
 #pragma unroll
   for (int i = 0; i < 2; i++) {
     const int c = 2 * lane + i;
-    int src = -1;              // the coordinate whose hi part column c holds
+    int src = -1;              // the lane whose coordinate's hi part column c holds
     bool low = false, half = false;
     if (st.fmt == KNN_FMT_EUCL) {
       low = c < D;
       half = c >= D && c < D + 3;
       src = c < D ? c : (c >= D + 3 && c < 2 * D + 3 ? c - D - 3 : -1);
     } else if ((c >> 4) < st.A) {
-      const int s = st.agent_s[c >> 4], d = st.agent_e[c >> 4] - s, j = c & 15;
+      const int a = c >> 4, f = a == 0 ? first[0] : a == 1 ? first[1] : a == 2 ? first[2] : first[3];
+      const int d = st.agent_e[a] - st.agent_s[a], j = c & 15;
       low = j < d;
       half = j == 2 * d || j == 2 * d + 1;
-      src = j < d ? s + j : (j < 2 * d ? s + j - d : -1);
+      src = j < d ? f + j : (j < 2 * d ? f + j - d : -1);
     }
     const float vh = __shfl_sync(MRMG_FULL, hi, src & 31), vl = __shfl_sync(MRMG_FULL, lo, src & 31);
     a1[i] = qid < 0 ? 0.f : (half ? -0.5f : (src >= 0 ? vh : 0.f));
@@ -1132,12 +1148,13 @@ __global__ void __launch_bounds__(32 * kPackRows) knn_pack_queries_kernel(
     qn = (float)n2;
   } else {
     // lane a sums agent a's coordinates
-    const int s = lane < st.A ? st.agent_s[lane] : 0, d = lane < st.A ? st.agent_e[lane] - s : 0;
+    const int d = lane < st.A ? st.agent_e[lane] - st.agent_s[lane] : 0;
+    const int f0 = lane == 0 ? first[0] : lane == 1 ? first[1] : lane == 2 ? first[2] : first[3];
     int dmax = 0;
     for (int a = 0; a < st.A; a++) dmax = max(dmax, st.agent_e[a] - st.agent_s[a]);
     double na = 0.0;
     for (int j = 0; j < dmax; j++) {
-      const double v = __shfl_sync(MRMG_FULL, x2, (s + j) & 31);
+      const double v = __shfl_sync(MRMG_FULL, x2, (f0 + j) & 31);
       if (j < d) na += v;
     }
     const float f = (float)na;
