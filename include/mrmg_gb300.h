@@ -414,7 +414,9 @@ int mrmg_scene_reserve(mrmg_scene *scene, int64_t n, void *stream);
 int mrmg_status_from_error_bits(int32_t bits);
 
 /* Statistics of the scene's last completed call: [0] items re-checked in
- * FP64 (pass two), [1] device error bits, [2] configurations evaluated by the
+ * FP64 (pass two; undecided edge positions are counted one by one until the
+ * scratch for them is full, their edges are then walked whole), [1] device
+ * error bits, [2] configurations evaluated by the
  * edge kernel's first pass, [3] reserved. */
 int mrmg_last_call_stats(const mrmg_scene *scene, int64_t *out4);
 

@@ -22,6 +22,7 @@
 
 #include "mrmg_bulk.cuh"
 #include "mrmg_internal.cuh"
+#include "mrmg_pending.cuh"
 
 namespace mrmg {
 namespace {
@@ -938,6 +939,12 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
 // An entry of the pending list: the edge, and an undecided position + 1 (with
 // kPendBfs: its place in the BFS order; 0: the whole edge)
 constexpr int kPendBfs = 1 << 30;
+struct PendCount {
+  int* ctr;
+  __device__ bool lost() const { return *(volatile int*)&ctr[kCtrPendLost] != 0; }
+  __device__ int add() { return atomicAdd(&ctr[kCtrPending], 1); }
+  __device__ void lose() { *(volatile int*)&ctr[kCtrPendLost] = 1; }
+};
 __device__ __forceinline__ long long pend_entry(long long e, int code) { return e | ((long long)code << 32); }
 
 // this lane's joints of edge e as double-floats: a = q1, d = q2 - q1
@@ -1035,7 +1042,7 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
     long long e;
     int code = 0;
     if (RESOLVE) {
-      const int listed = min(ctr[kCtrPending], (int)min(pend_cap, 0x7fffffffll));
+      const int listed = pend_listed(ctr[kCtrPending], pend_cap);
       if (k >= (long long)listed + (ctr[kCtrPendLost] ? ctr[kCtrL1] : 0)) break;
       if (k < listed) {
         e = pend[k] & 0xffffffffll;
@@ -1244,9 +1251,10 @@ __global__ void __launch_bounds__(256, GPL == 1 ? 3 : (GPL == 2 ? 2 : 1)) arm_ed
         if (code == V_COLLIDE) {
           vsurv[sv].dead = 1;
         } else {
-          const int slot = atomicAdd(&ctr[kCtrPending], 1);
-          if (slot < pend_cap) pend[slot] = pend_entry(surv[sv].e, at + 1);
-          else vsurv[sv].pend = ctr[kCtrPendLost] = 1;
+          PendCount count{ctr};
+          const int slot = pend_claim(count, pend_cap);
+          if (slot >= 0) pend[slot] = pend_entry(surv[sv].e, at + 1);
+          else vsurv[sv].pend = 1;
         }
       }
     }
