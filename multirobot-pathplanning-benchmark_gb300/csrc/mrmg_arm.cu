@@ -1047,7 +1047,12 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
       if (k < listed) {
         e = pend[k] & 0xffffffffll;
         code = (int)(pend[k] >> 32);
-        if (code && out[e] == V_COLLIDE) continue;      // another position of the edge collides
+        if (code) {
+          // another position of the edge collides (its warp may be storing that now:
+          // read once, decide warp-uniformly)
+          const int dead = lane == 0 && *(volatile const uint8_t*)(out + e) == V_COLLIDE;
+          if (__shfl_sync(MRMG_FULL, dead, 0)) continue;
+        }
       } else {                                          // the list overflowed: survivors with a lost entry
         const SurvivorEdge& sv = surv[k - listed];
         if (!sv.pend || sv.dead) continue;
