@@ -1037,7 +1037,11 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
   // per edge is uneven (a free first configuration is a full evaluation)
   while (true) {
     long long k = 0;
-    if (lane == 0) k = atomicAdd(&ctr[RESOLVE ? kCtrQueue2 : kCtrQueue], 1);
+    if (lane == 0) {
+      // (pass 2: listed positions, then survivors, up to 2^31 of each)
+      if (RESOLVE) k = (long long)atomicAdd((unsigned long long*)&ctr[kCtrQueueP], 1ull);
+      else k = atomicAdd(&ctr[kCtrQueue], 1);
+    }
     k = __shfl_sync(MRMG_FULL, k, 0);
     long long e;
     int code = 0;

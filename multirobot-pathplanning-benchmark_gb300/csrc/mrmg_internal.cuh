@@ -129,10 +129,10 @@ struct PenParams {
 
 // per-call scratch counters (device): [0] work queue, [1] pending count,
 // [2] error bits, [3] pass-two queue, [4..5] configurations evaluated (64-bit),
-// [6] surviving edges, [7] longest remaining position range, [8..9] phase-B
-// queue (64-bit), [10] finished CTAs of the last phase-B launch
+// [6] surviving edges, [7] longest remaining position range, [8..9] pass-two
+// queue of arm edges (64-bit), [10] finished CTAs of the last phase-B launch
 constexpr int kCtrQueue = 0, kCtrPending = 1, kCtrErr = 2, kCtrQueue2 = 3, kCtrStat0 = 4;
-constexpr int kCtrL1 = 6, kCtrMaxJ = 7, kCtrQueueB = 8;
+constexpr int kCtrL1 = 6, kCtrMaxJ = 7, kCtrQueueP = 8;
 constexpr int kCtrScan = 12, kCtrListed = 13;   // scan: its queue, and the items listed for the warp kernels
 constexpr int kCtrPendLost = 11;   // pending positions did not fit the list
 constexpr int kCtrDoneB = 10;   // CTAs of the last phase-B launch that have finished
