@@ -770,35 +770,52 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                : "memory");
 }
 
-// 32 lanes x 32 consecutive FP32 columns of TMEM (warp-wide): the load, and the
-// wait for every load issued before (the registers hold nothing until then)
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&r)[32]) {
+// 32 lanes x 32 consecutive FP32 columns of TMEM (warp-wide), or twice that from
+// two places.  Load and wait are one statement: the registers of a load hold
+// nothing before its wait, and the compiler may move or copy what it takes for
+// values, so none is named in between.  The barrier first: the lanes come here
+// from branches of their own, and the load is the whole warp's.
+#define MRMG_R32(r_)                                                                                                \
+  "=r"(r_[0]), "=r"(r_[1]), "=r"(r_[2]), "=r"(r_[3]), "=r"(r_[4]), "=r"(r_[5]), "=r"(r_[6]), "=r"(r_[7]),            \
+      "=r"(r_[8]), "=r"(r_[9]), "=r"(r_[10]), "=r"(r_[11]), "=r"(r_[12]), "=r"(r_[13]), "=r"(r_[14]), "=r"(r_[15]), \
+      "=r"(r_[16]), "=r"(r_[17]), "=r"(r_[18]), "=r"(r_[19]), "=r"(r_[20]), "=r"(r_[21]), "=r"(r_[22]),             \
+      "=r"(r_[23]), "=r"(r_[24]), "=r"(r_[25]), "=r"(r_[26]), "=r"(r_[27]), "=r"(r_[28]), "=r"(r_[29]),             \
+      "=r"(r_[30]), "=r"(r_[31])
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
+  uint32_t r[32];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%"
-      "28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
+      "28,%29,%30,%31}, [%32];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : MRMG_R32(r)
+      : "r"(taddr)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
 }
-// The registers of a load whose wait has passed, as values: the empty asm keeps
-// every use below the wait.
-__device__ __forceinline__ void tmem_take(uint32_t (&r)[32], float (&v)[32]) {
+__device__ __forceinline__ void tmem_ld32x2(uint32_t ta, uint32_t tb, float (&va)[32], float (&vb)[32]) {
+  uint32_t ra[32], rb[32];
+  __syncwarp();
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%"
+      "28,%29,%30,%31}, [%64];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%"
+      "58,%59,%60,%61,%62,%63}, [%65];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : MRMG_R32(ra), MRMG_R32(rb)
+      : "r"(ta), "r"(tb)
+      : "memory");
 #pragma unroll
   for (int i = 0; i < 32; i++) {
-    asm volatile("" : "+r"(r[i]));
-    v[i] = __uint_as_float(r[i]);
+    va[i] = __uint_as_float(ra[i]);
+    vb[i] = __uint_as_float(rb[i]);
   }
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  tmem_ld32_issue(taddr, r);
-  tmem_ld_wait();
-  tmem_take(r, v);
-}
+#undef MRMG_R32
 
 // shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups
 // 1024 bytes apart; `addr` may carry a K offset inside the 128-byte row
@@ -1359,53 +1376,32 @@ __global__ void __launch_bounds__(128 * TcSplit<FMT>::S + 32, 1) knn_tc_kernel(K
           scan(v, t, c0);
         }
       } else if (FMT == KNN_FMT_EUCL) {
-        // the next 32 columns are on their way while these are scanned
-        // (straight-line code: a load's registers must not pass a branch, where
-        // the compiler could copy them before the wait)
-        static_assert(NCOL == 128 || FMT != KNN_FMT_EUCL, "four loads per tile");
-        uint32_t r0[32], r1[32], r2[32], r3[32];
-        float v[32];
-        tmem_ld32_issue(lane_base, r0);
-        tmem_ld_wait();
-        tmem_ld32_issue(lane_base + 32, r1);
-        tmem_take(r0, v);
+        static_assert(NCOL == 128 || FMT != KNN_FMT_EUCL, "two double loads per tile");
+        float v[32], w[32];
+        tmem_ld32x2(lane_base, lane_base + 32, v, w);
         scan(v, t, 0);
-        tmem_ld_wait();
-        tmem_ld32_issue(lane_base + 64, r2);
-        tmem_take(r1, v);
-        scan(v, t, 32);
-        tmem_ld_wait();
-        tmem_ld32_issue(lane_base + 96, r3);
-        tmem_take(r2, v);
-        scan(v, t, 64);
-        tmem_ld_wait();
+        scan(w, t, 32);
+        tmem_ld32x2(lane_base + 64, lane_base + 96, v, w);
         release();
-        tmem_take(r3, v);
-        scan(v, t, 96);
+        scan(v, t, 64);
+        scan(w, t, 96);
       } else {
         // all four agents' columns (those past the last agent hold nothing that is used)
         const int c0 = slice * NCOL;
-        float m[32];
-        uint32_t r0[32], r1[32], r2[32], r3[32];
-        tmem_ld32_issue(lane_base + c0, r0);
-        tmem_ld32_issue(lane_base + 64 + c0, r1);
-        tmem_ld_wait();
-        tmem_ld32_issue(lane_base + 128 + c0, r2);
-        tmem_ld32_issue(lane_base + 192 + c0, r3);
+        float m[32], v[32], w[32];
 #pragma unroll
         for (int i = 0; i < 32; i++) m[i] = -__int_as_float(0x7f800000);
-        auto fold = [&](uint32_t (&r)[32], float qa) {
-          float v[32];
-          tmem_take(r, v);
+        auto fold = [&](const float (&x)[32], float qa) {
 #pragma unroll
-          for (int i = 0; i < 32; i++) m[i] = fmaxf(m[i], fmaf(-2.f, v[i], qa));
+          for (int i = 0; i < 32; i++) m[i] = fmaxf(m[i], fmaf(-2.f, x[i], qa));
         };
-        fold(r0, qna[0]);
-        if (st.A > 1) fold(r1, qna[1]);
-        tmem_ld_wait();
+        tmem_ld32x2(lane_base + c0, lane_base + 64 + c0, v, w);
+        fold(v, qna[0]);
+        if (st.A > 1) fold(w, qna[1]);
+        tmem_ld32x2(lane_base + 128 + c0, lane_base + 192 + c0, v, w);
         release();
-        if (st.A > 2) fold(r2, qna[2]);
-        if (st.A > 3) fold(r3, qna[3]);
+        if (st.A > 2) fold(v, qna[2]);
+        if (st.A > 3) fold(w, qna[3]);
         scan(m, t, c0);
       }
       if (!RAD && qrow >= 0) {
