@@ -70,7 +70,8 @@ __host__ __device__ inline int pen_first_sphere(const PenDev& pd, int R, int r) 
 __device__ __forceinline__ int cluster_size() { int v; asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(v)); return v; }
 __device__ __forceinline__ int cluster_rank() { int v; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(v)); return v; }
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+  // (not the .aligned forms: half warps come from branches of their own)
+  asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
   uint32_t a;
