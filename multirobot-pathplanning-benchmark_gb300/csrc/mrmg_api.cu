@@ -7,6 +7,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <exception>
+#include <limits>
 #include <mutex>
 #include <new>
 #include <numeric>
@@ -319,8 +320,8 @@ void pen_tables(const ArmSrc& a, int R, const std::vector<char>& on, const std::
   t->pen_task.clear();
   int real = 0;
   for (int r = 0; r < kMaxRobots; r++) {
-    // this robot's spheres; an odd count is made even by a sphere of radius
-    // -1e30 at the last one's place, which adds nothing to any pair
+    // this robot's spheres; an odd count is made even by an empty sphere (radius
+    // -infinity) at the last one's place, which the kernel leaves out of every pair
     const int s0 = (int)t->pen_sph.size();
     int cnt[kMaxLinks + 1] = {}, last = -1;
     for (int sl = 0; r < R && sl < a.G * a.SPG; sl++) {
@@ -334,7 +335,7 @@ void pen_tables(const ArmSrc& a, int R, const std::vector<char>& on, const std::
     real += (int)t->pen_sph.size() - s0;
     if ((t->pen_sph.size() - s0) & 1) {
       float4 none = t->pen_sph.back();
-      none.w = -1e30f;
+      none.w = -std::numeric_limits<float>::infinity();
       t->pen_sph.push_back(none);
       cnt[last]++;
     }

@@ -123,8 +123,11 @@ struct Side {
 // Floor of the squared distances whose reciprocal root is taken: added to the
 // last product of the sum, it leaves every square above 1e-22 m^2 unchanged.
 constexpr float kTiny2 = 1e-30f;
-// x2 of a partner that is not there: e = 0
-constexpr float kNone = -1e30f;
+// x2 of a partner that is not there: -infinity, so e = 0 for any beta
+#define MRMG_PEN_NONE __int_as_float(0xff800000)
+// the sphere of radius -infinity that makes a robot's count even: its pairs get
+// MRMG_PEN_NONE for beta times the radius
+__device__ __forceinline__ bool empty_sphere(float radius) { return radius < -3.402823466e38f; }
 
 // Pairs whose 1 + e are multiplied before one log2 is taken of the product:
 // log2 is an eighth of an FMA on this part (measured 16 against 128 per clock
@@ -350,7 +353,7 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
   // ---- stage tables and the segment's waypoints (rows t0-1 .. t0+SEG)
   for (int i = tid; i < S; i += blockDim.x) {
     sph[i] = pd.sph[i];
-    br[i] = pp.beta * 1.4426950408889634f * pd.sph[i].w;
+    br[i] = empty_sphere(sph[i].w) ? MRMG_PEN_NONE : pp.beta * 1.4426950408889634f * sph[i].w;
   }
   for (int i = tid; i < 6 * ((B + 1) / 2); i += blockDim.x) {   // pair i / 6: centre x, y, z, half extent x, y, z
     const int b = 2 * (i / 6), k = i % 6, c = b + 1 < B ? b + 1 : b;
@@ -450,7 +453,7 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
       d.nx = bc2(-C[cen<SEG>(i, 0, wl)]);
       d.ny = bc2(-C[cen<SEG>(i, 1, wl)]);
       d.nz = bc2(-C[cen<SEG>(i, 2, wl)]);
-      d.K = bc2(fmaf(bl, sph[i].w, blm));
+      d.K = bc2(empty_sphere(sph[i].w) ? MRMG_PEN_NONE : fmaf(bl, sph[i].w, blm));
       d.ps = d.pr = d.gx = d.gy = d.gz = bc2(0.f);
       return d;
     };
@@ -473,7 +476,7 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
     }
     if (B > 2 * even) {   // the boxes left: a place without a box adds nothing
       const int k = even + half, left = B - 2 * k;   // of this half's pair: both there when 2 or more, the first when 1
-      const float kx = left > 0 ? 0.f : kNone, ky = left > 1 ? 0.f : kNone;
+      const float kx = left > 0 ? 0.f : MRMG_PEN_NONE, ky = left > 1 ? 0.f : MRMG_PEN_NONE;
       boxes(left > 0 ? k : even, add2(a.K, make_float2(kx, ky)), add2(b.K, make_float2(kx, ky)));
     }
     flush_product<COST>(a);
@@ -484,7 +487,7 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
       sphere_step<decltype(with_cost)::value, GRAD, DIRECT>(a, b, C2[(3 * j) * SEG], C2[(3 * j + 1) * SEG],
                                                             C2[(3 * j + 2) * SEG], r, nbl);
     };
-    const float2 none = bc2(kNone);
+    const float2 none = bc2(MRMG_PEN_NONE);
     {   // the later robots' spheres
       const int j0 = task.w / 2, j1 = S / 2, je = j0 + ((j1 - j0) & ~(HV - 1));
 #pragma unroll 4
