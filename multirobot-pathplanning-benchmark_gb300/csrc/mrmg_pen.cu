@@ -43,7 +43,8 @@ __host__ __device__ inline size_t al4(size_t n) { return (n + 3) & ~(size_t)3; }
 template <int SEG>
 struct PenLayout {
   size_t C, G, OZ, W, QG, sph, box, br, part, total;
-  __host__ __device__ PenLayout(int S, int B, int D, bool grad, int warps, int Sg, int Rg) {
+  // tasks: pair tasks where a cluster shares the segment (their costs are kept one by one), else 0
+  __host__ __device__ PenLayout(int S, int B, int D, bool grad, int warps, int tasks, int Sg, int Rg) {
     size_t o = 0;
     C = o;   o += (size_t)S * 3 * SEG;                          // sphere centres [S/2][3][SEG][2]
     G = o;   o += grad ? (size_t)Sg * 3 * SEG : 0;              // dcost/dcentre  [Sg*3][SEG]
@@ -53,7 +54,7 @@ struct PenLayout {
     sph = o; o += (size_t)S * 4;
     box = o; o += (size_t)((B + 1) / 2) * 12;                    // pairs of boxes [(B+1)/2][6][2]
     br = o;  o += al4((size_t)S);                               // beta log2(e) radius
-    part = o; o += (size_t)warps * 64;
+    part = o; o += (size_t)32 * (tasks > 2 * warps ? tasks : 2 * warps);
     total = o;
   }
 };
@@ -65,28 +66,20 @@ __device__ __forceinline__ int cen(int s, int i, int wl) { return (((s >> 1) * 3
 
 __host__ __device__ inline int pen_first_sphere(const PenDev& pd, int R, int r) { return r < R ? pd.lk[r][0] : pd.S; }
 
-// the CTAs of a cluster: size, this CTA's rank, barrier, and loads from the
-// same shared-memory place of CTA `rank`
+// the CTAs of a cluster: size, this CTA's rank, barrier, and stores to the same
+// shared-memory place of CTA `rank`
 __device__ __forceinline__ int cluster_size() { int v; asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(v)); return v; }
 __device__ __forceinline__ int cluster_rank() { int v; asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(v)); return v; }
-__device__ __forceinline__ void cluster_sync() {
-  // (not the .aligned forms: half warps come from branches of their own)
-  asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory");
-}
+// (not the .aligned forms: half warps come from branches of their own)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
 __device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
   uint32_t a;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
   return a;
 }
-__device__ __forceinline__ float cluster_ld(const float* p, int rank) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr(p, rank)) : "memory");
-  return v;
-}
-__device__ __forceinline__ double cluster_ld64(const double* p, int rank) {
-  double v;
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(cluster_addr(p, rank)) : "memory");
-  return v;
+__device__ __forceinline__ void cluster_st(float* p, int rank, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr(p, rank)), "f"(v) : "memory");
 }
 
 // MUFU approximations (PTX): 2^x, log2, sqrt, 1/sqrt, 1/x
@@ -309,13 +302,17 @@ __device__ __forceinline__ void acc2(float& h, float& l, float v) {
 // Bound: issue slots (cost: 15 warp instructions per 32 pairs, 83 % of them
 // used) and, with the gradient, the FMA and special-function pipes together
 // (18 instructions; 17 and 16 of 27 cycles per 32 pairs).  512 paths of 256
-// waypoints, four arms, 50 boxes: cost 1.55 -> 1.27 ms, gradient 3.63 -> 2.81
-// ms, both 4.03 -> 3.19 ms, against one log2 and one reciprocal per pair, two
+// waypoints, four arms, 50 boxes: cost 1.55 -> 1.24 ms, gradient 3.63 -> 2.76
+// ms, both 4.03 -> 3.06 ms, against one log2 and one reciprocal per pair, two
 // spheres per packed instruction and 32-waypoint gradient CTAs (one per SM).
-// Unrolling the sphere loop by 1, 2, 4 or 8: cost 1.31, 1.31, 1.24, 1.23 ms, the
-// gradient unchanged.  12 paths of 45 waypoints: cost 117 -> 80 us, gradient 185
-// -> 80 us, from the clusters.
-template <int SEG, bool COST, bool GRAD, bool DIRECT>
+// The sphere loop unrolled by 1, 2, 4 or 8: cost 1.31, 1.31, 1.24, 1.23 ms, the
+// gradient unchanged; the box loop by 1 or 2: gradient 2.80, 2.76 ms, both 3.09,
+// 3.06 ms.  SHARED (clusters): 12 paths of 45 waypoints, 20 boxes: cost 47 us,
+// gradient 46 us, both 56 us; with the joint gradients of each CTA's own spheres
+// added up over the CTAs (whose bits then depend on the split) 47, 46 and 56 us,
+// with sphere gradients fetched behind the barrier, not stored before it, 52, 49
+// and 60 us.
+template <int SEG, bool COST, bool GRAD, bool DIRECT, bool SHARED>
 __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 32 ? 1 : 2)
     pen_kernel(ArmDev a, PenDev pd, PenParams pp, const float* __restrict__ paths, int T, int nseg,
                const float* __restrict__ gout, double* __restrict__ seg_cost, float* __restrict__ wp_cost,
@@ -327,9 +324,10 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
   // waypoint, and its share of a warp's partners and robots
   constexpr int HV = 32 / SEG;
   const int wl = lane & (SEG - 1), half = HV > 1 ? lane / SEG : 0;
-  // the CTAs of a cluster share one segment: each runs its kinematics and a
-  // share of the pair tasks
-  const int split = cluster_size(), rank = cluster_rank();
+  // SHARED: the CTAs of a cluster share one segment: each runs its kinematics and
+  // a share of the pair tasks
+  const int split = SHARED ? cluster_size() : 1, rank = SHARED ? cluster_rank() : 0;
+  if (SHARED) cluster_arrive();   // (waited for before the first store to another CTA)
   const long long sidx = blockIdx.x / split;
   const long long p = sidx / nseg;
   const int seg = (int)(sidx - p * nseg);
@@ -338,7 +336,7 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
   // and joints [j_lo, j_hi) (robots' joints are contiguous in robot order)
   const int s_lo = pen_first_sphere(pd, R, gr0), s_hi = pen_first_sphere(pd, R, gr1);
   const int j_lo = a.q_off[gr0], j_hi = gr1 < R ? a.q_off[gr1] : D;
-  const PenLayout<SEG> L(S, B, D, GRAD, NW, s_hi - s_lo, gr1 - gr0);
+  const PenLayout<SEG> L(S, B, D, GRAD, NW, SHARED ? pd.NTK : 0, s_hi - s_lo, gr1 - gr0);
   float* C = smf + L.C;
   float* Gs = smf + L.G;
   float* OZ = smf + L.OZ;
@@ -368,11 +366,8 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
       W[i] = (t >= 0 && t < T) ? src[(long long)(t0 - 1) * D + i] : 0.f;
     }
   }
-  if (GRAD) {
+  if (GRAD)
     for (int i = tid; i < SEG * D; i += blockDim.x) QG[i] = 0.f;
-    if (split > 1)   // spheres of the other CTAs' tasks add nothing to this CTA's joint gradients
-      for (int i = tid; i < (s_hi - s_lo) * 3 * SEG; i += blockDim.x) Gs[i] = 0.f;
-  }
   __syncthreads();
 
   // ---- forward kinematics: (half) warp r walks robot r's chain, lane = waypoint
@@ -442,6 +437,17 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
   const float blm = bl * pp.margin;
   float acc_h = 0.f, acc_l = 0.f;
   const int VW = NW * split, vw = warp * split + rank;   // the cluster's warps, dealt over its CTAs
+  if (SHARED) cluster_wait();   // every CTA runs
+  // The sums of a segment do not depend on how many CTAs share it, so a path's
+  // cost and gradient have the same bits alone and in any batch: each CTA gets every
+  // sphere's gradient, the first one every task's cost, and adds them up as a CTA
+  // alone does.
+  auto put = [&](int s, int i, float v) {   // dcost/dcentre, coordinate i of sphere s
+    float* g = Gs + (3 * (s - s_lo) + i) * SEG + wl;
+    if (!SHARED) *g = v;
+    else
+      for (int r = 0; r < split; r++) cluster_st(g, r, v);
+  };
   for (int base = 0, turn = 0; base < NTK; base += VW, turn ^= 1) {
     const int tk = turn ? base + VW - 1 - vw : base + vw;
     if (tk >= NTK) continue;
@@ -467,6 +473,7 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
       box_step<COST, GRAD, DIRECT>(a, b, bx, nbl, Ka, Kb);
     };
     const int nb2 = B / 2, even = nb2 & ~(HV - 1);
+#pragma unroll 2
     for (int k = 0; k < even; k += HV) {
       boxes(k + half, a.K, b.K);
       if (COST && (k / HV) % kProd == kProd - 1) {
@@ -513,28 +520,39 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
 #pragma unroll
       for (int i = 0; i < 3; i++) {
         if (HV == 1) {
-          Gs[(3 * (i0 - s_lo) + i) * SEG + wl] = is * g[i];
-          Gs[(3 * (i1 - s_lo) + i) * SEG + wl] = is * h[i];
+          put(i0, i, is * g[i]);
+          put(i1, i, is * h[i]);
         } else {   // both halves' sums: half 0 stores the first sphere's, half 1 the second's
           const float mine = half ? h[i] : g[i], other = half ? g[i] : h[i];
-          Gs[(3 * (i0 + half - s_lo) + i) * SEG + wl] = is * (mine + __shfl_xor_sync(MRMG_FULL, other, SEG & 31));
+          put(i0 + half, i, is * (mine + __shfl_xor_sync(MRMG_FULL, other, SEG & 31)));
         }
       }
     }
-    if (COST) acc2(acc_h, acc_l, (a.ps.x + a.ps.y) + (b.ps.x + b.ps.y));
+    if (COST) {
+      const float v = (a.ps.x + a.ps.y) + (b.ps.x + b.ps.y);
+      if (SHARED) cluster_st(part + tk * 32 + lane, 0, v);
+      else acc2(acc_h, acc_l, v);
+    }
   }
-  if (COST) {
+  if (SHARED) {
+    cluster_arrive();   // every CTA's tasks are done
+    cluster_wait();
+    if (COST && rank == 0)
+      for (int base = 0, turn = 0; base < NTK; base += NW, turn ^= 1) {
+        const int tk = turn ? base + NW - 1 - warp : base + warp;
+        if (tk < NTK) acc2(acc_h, acc_l, part[tk * 32 + lane]);
+      }
+  }
+  if (COST && rank == 0) {   // (where tasks' costs lie in `part`, these are places of this warp's own tasks)
     part[warp * 32 + lane] = acc_h;
-    part[(NW + warp) * 32 + lane] = acc_l;
+    part[(2 * NW - 1 - warp) * 32 + lane] = acc_l;
   }
   __syncthreads();
 
-  double csum = 0.0;   // warp 0: this CTA's pair terms of waypoint t0 + wl
-  if (COST && warp == 0) {
-    for (int w = 0; w < NW; w++) csum += (double)part[w * 32 + lane] + (double)part[(NW + w) * 32 + lane];
+  double csum = 0.0;   // warp 0 of the first CTA: the pair terms of waypoint t0 + wl
+  if (COST && warp == 0 && rank == 0) {
+    for (int w = 0; w < NW; w++) csum += (double)part[w * 32 + lane] + (double)part[(2 * NW - 1 - w) * 32 + lane];
     if (HV > 1) csum += __shfl_xor_sync(MRMG_FULL, csum, SEG & 31);
-    __syncwarp();
-    ((double*)part)[lane] = csum;
   }
   if (GRAD) {
     // ---- joint gradients from the sphere gradients, tip to base
@@ -570,12 +588,9 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
       }
     }
   }
-  if (split > 1) cluster_sync();   // every CTA's sums are in place
-
   const int t = t0 + wl;
   if (COST && warp == 0 && rank == 0) {
     double c = csum;
-    for (int r = 1; r < split; r++) c += cluster_ld64((double*)part + lane, r);
     c *= 0.69314718055994531 * (double)pp.inv_beta * (double)pp.inv_scale;   // ln 2 / (beta scale)
     if (t + 1 < T) {
       const float* w0 = W + (wl + 1) * D;
@@ -610,15 +625,9 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
       float gsm = 0.f;
       if (tt > 0) gsm += sw2 * (wc - W[i]);
       if (tt + 1 < T) gsm -= sw2 * (W[i + 2 * D] - wc);
-      float qg = QG[i];
-      if (split > 1) {
-        qg = cluster_ld(QG + i, 0);
-        for (int r = 1; r < split; r++) qg += cluster_ld(QG + i, r);
-      }
-      dst[i] = go * (qg + gsm);
+      dst[i] = go * (QG[i] + gsm);
     }
   }
-  if (split > 1) cluster_sync();   // no CTA leaves while another reads its shared memory
 }
 
 __global__ void pen_sum_kernel(const double* __restrict__ seg, long long P, int nseg, double* __restrict__ cost) {
@@ -647,14 +656,19 @@ int pen_split(long long segs, int slots) {
   return best;
 }
 
-template <int SEG, bool COST, bool GRAD, bool DIRECT>
+template <int SEG>
+size_t smem_bytes(const ArmDev& a, const PenDev& pd, int grad, int warps, int tasks, int gr0, int gr1) {
+  return PenLayout<SEG>(pd.S, pd.B, a.D, grad != 0, warps, tasks,
+                        pen_first_sphere(pd, a.R, gr1) - pen_first_sphere(pd, a.R, gr0), gr1 - gr0)
+             .total * sizeof(float);
+}
+
+template <int SEG, bool COST, bool GRAD, bool DIRECT, bool SHARED>
 cudaError_t launch_one(const ArmDev& a, const PenDev& pd, const PenParams& pp, const float* paths, long long P, int T,
                        const float* gout, double* seg, float* wp, float* grad, int warps, int split, int gr0, int gr1,
                        cudaStream_t st) {
-  const PenLayout<SEG> L(pd.S, pd.B, a.D, GRAD, warps, pen_first_sphere(pd, a.R, gr1) - pen_first_sphere(pd, a.R, gr0),
-                         gr1 - gr0);
-  const size_t smem = L.total * sizeof(float);
-  auto kernel = pen_kernel<SEG, COST, GRAD, DIRECT>;
+  const size_t smem = smem_bytes<SEG>(a, pd, GRAD, warps, SHARED ? pd.NTK : 0, gr0, gr1);
+  auto kernel = pen_kernel<SEG, COST, GRAD, DIRECT, SHARED>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int nseg = pen_segments(T, SEG);
@@ -668,7 +682,7 @@ cudaError_t launch_one(const ArmDev& a, const PenDev& pd, const PenParams& pp, c
   at.val.clusterDim.x = split;
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = split > 1 ? 1 : 0;
+  cfg.numAttrs = SHARED ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, a, pd, pp, paths, T, nseg, gout, seg, wp, grad, gr0, gr1);
 }
 
@@ -677,11 +691,14 @@ cudaError_t launch_one(const ArmDev& a, const PenDev& pd, const PenParams& pp, c
 template <int SEG, bool COST, bool GRAD>
 cudaError_t launch_form(const ArmDev& a, const PenDev& pd, const PenParams& pp, const float* paths, long long P, int T,
                         const float* gout, double* seg, float* wp, float* grad, int warps, int gr0, int gr1,
-                        int num_sms, cudaStream_t st) {
+                        int num_sms, size_t smem_sm, cudaStream_t st) {
   // the largest x2 of any pair: centres coincide, or lie deepest in a box
   const bool direct = pp.beta * 1.4426951f * (pp.margin + pd.reach) <= kDirectMax;
   const int nseg = pen_segments(T, SEG);
-  const int split = pen_split(P * nseg, num_sms * (GRAD && SEG == 32 ? 1 : 2));
+  int split = pen_split(P * nseg, num_sms * (GRAD && SEG == 32 ? 1 : 2));
+  // (1 KB per CTA is the system's; a cluster keeps its tasks' costs in shared memory too)
+  while (split > 1 && smem_bytes<SEG>(a, pd, GRAD, warps, pd.NTK, gr0, gr1) + 1024 > smem_sm)
+    split /= 2;
   const long long step = std::max(1ll, 0x7fffffffll / ((long long)nseg * split));
   cudaError_t e = cudaSuccess;
   for (long long p0 = 0; p0 < P && e == cudaSuccess; p0 += step) {
@@ -692,23 +709,17 @@ cudaError_t launch_form(const ArmDev& a, const PenDev& pd, const PenParams& pp, 
     double* sg = seg ? seg + p0 * nseg : nullptr;
     float* wc = wp ? wp + wp0 : nullptr;
     float* g = grad ? grad + wp0 * a.D : nullptr;
-    if (direct) e = launch_one<SEG, COST, GRAD, true>(a, pd, pp, w, n, T, go, sg, wc, g, warps, split, gr0, gr1, st);
-    else e = launch_one<SEG, COST, GRAD, false>(a, pd, pp, w, n, T, go, sg, wc, g, warps, split, gr0, gr1, st);
+    auto launch = direct ? (split > 1 ? launch_one<SEG, COST, GRAD, true, true> : launch_one<SEG, COST, GRAD, true, false>)
+                         : (split > 1 ? launch_one<SEG, COST, GRAD, false, true> : launch_one<SEG, COST, GRAD, false, false>);
+    e = launch(a, pd, pp, w, n, T, go, sg, wc, g, warps, split, gr0, gr1, st);
   }
   return e;
-}
-
-template <int SEG>
-size_t smem_bytes(const ArmDev& a, const PenDev& pd, int grad, int warps, int gr0, int gr1) {
-  return PenLayout<SEG>(pd.S, pd.B, a.D, grad != 0, warps,
-                        pen_first_sphere(pd, a.R, gr1) - pen_first_sphere(pd, a.R, gr0), gr1 - gr0)
-             .total * sizeof(float);
 }
 
 }  // namespace
 
 size_t pen_smem_bytes(const ArmDev& a, const PenDev& pd, int grad, int warps, int gr0, int gr1) {
-  return smem_bytes<32>(a, pd, grad, warps, gr0, gr1);
+  return smem_bytes<32>(a, pd, grad, warps, 0, gr0, gr1);
 }
 
 int pen_grad_groups(const ArmDev& a, const PenDev& pd, int warps, size_t smem_max, int* bounds) {
@@ -736,26 +747,26 @@ cudaError_t pen_launch(const ArmDev& a, const PenDev& pd, const PenParams& pp, c
   const bool want_cost = cost || wp_cost;
   // gradient form: half-warp segments where two of their CTAs fit an SM
   const int gw = std::min(warps, kPenGradWarps);
-  const bool halves = grad && n_groups <= 1 && 2 * (smem_bytes<16>(a, pd, 1, gw, 0, a.R) + 1024) <= smem_sm;
+  const bool halves = grad && n_groups <= 1 && 2 * (smem_bytes<16>(a, pd, 1, gw, 0, 0, a.R) + 1024) <= smem_sm;
   cudaError_t e = cudaSuccess;
   int nseg = pen_segments(T, 32);   // segments whose costs are summed
   if (grad && n_groups <= 1 && halves) {
     nseg = pen_segments(T, 16);
     if (want_cost)
-      e = launch_form<16, true, true>(a, pd, pp, paths, P, T, gout, seg, wp_cost, grad, gw, 0, a.R, num_sms, st);
+      e = launch_form<16, true, true>(a, pd, pp, paths, P, T, gout, seg, wp_cost, grad, gw, 0, a.R, num_sms, smem_sm, st);
     else
-      e = launch_form<16, false, true>(a, pd, pp, paths, P, T, gout, nullptr, nullptr, grad, gw, 0, a.R, num_sms, st);
+      e = launch_form<16, false, true>(a, pd, pp, paths, P, T, gout, nullptr, nullptr, grad, gw, 0, a.R, num_sms, smem_sm, st);
   } else if (grad && n_groups <= 1) {
     if (want_cost)
-      e = launch_form<32, true, true>(a, pd, pp, paths, P, T, gout, seg, wp_cost, grad, warps, 0, a.R, num_sms, st);
+      e = launch_form<32, true, true>(a, pd, pp, paths, P, T, gout, seg, wp_cost, grad, warps, 0, a.R, num_sms, smem_sm, st);
     else
-      e = launch_form<32, false, true>(a, pd, pp, paths, P, T, gout, nullptr, nullptr, grad, warps, 0, a.R, num_sms, st);
+      e = launch_form<32, false, true>(a, pd, pp, paths, P, T, gout, nullptr, nullptr, grad, warps, 0, a.R, num_sms, smem_sm, st);
   } else {
     if (want_cost || !grad)
-      e = launch_form<32, true, false>(a, pd, pp, paths, P, T, gout, seg, wp_cost, nullptr, warps, 0, a.R, num_sms, st);
+      e = launch_form<32, true, false>(a, pd, pp, paths, P, T, gout, seg, wp_cost, nullptr, warps, 0, a.R, num_sms, smem_sm, st);
     for (int g = 0; grad && g < n_groups && e == cudaSuccess; g++)
       e = launch_form<32, false, true>(a, pd, pp, paths, P, T, gout, nullptr, nullptr, grad, warps, bounds[g],
-                                       bounds[g + 1], num_sms, st);
+                                       bounds[g + 1], num_sms, smem_sm, st);
   }
   if (e != cudaSuccess || !cost) return e;
   const int blocks = (int)std::min<long long>((P + 255) / 256, 4096);
