@@ -869,6 +869,36 @@ __device__ __forceinline__ void warp_areas(const ArmDev& s, unsigned char* smem_
   *w64 = (double*)p;
 }
 
+// The rows behind the scan: those it listed (entries' pad), then, where it found
+// that it does not pay, the rows it left, a range per part of the batch.  Copied
+// to shared memory once: every item's atomic on the queue takes the counters'
+// line out of the SM's L1 cache, and a load of it per item waits behind all SMs'
+// atomics (200,000 free edges, first positions: 582 us without the list, 798 us
+// with one such load per item, 981 us with three).
+struct ScanRows {
+  int listed, first[kMaxParts], count[kMaxParts];
+};
+__device__ __forceinline__ void load_scan_rows(const int* ctr, ScanRows* r) {   // a barrier must follow
+  if (threadIdx.x < kMaxParts) {
+    r->first[threadIdx.x] = ctr[kCtrScanTails + 2 * threadIdx.x];
+    r->count[threadIdx.x] = ctr[kCtrScanTails + 2 * threadIdx.x + 1];
+    if (threadIdx.x == 0) r->listed = ctr[kCtrListed];
+  }
+}
+__device__ __forceinline__ long long scan_total(const ScanRows& r) {
+  long long n = r.listed;
+#pragma unroll
+  for (int j = 0; j < kMaxParts; j++) n += r.count[j];
+  return n;
+}
+__device__ __forceinline__ long long scan_item(const ScanRows& r, const SurvivorEdge* list, long long k) {
+  if (k < r.listed) return list[k].pad;
+  k -= r.listed;
+  int j = 0;
+  while (j + 1 < kMaxParts && k >= r.count[j]) k -= r.count[j++];
+  return r.first[j] + k;
+}
+
 // ---------------------------------------------------------------------------
 // Configurations (warp per configuration, configurations taken from a work
 // queue in chunks of s.cfg_chunk).
@@ -883,9 +913,13 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
   // pass 2: as many CTAs stay as there are undecided items for their warps
   if (RESOLVE && (long long)blockIdx.x * (blockDim.x >> 5) >= *(volatile int*)&ctr[kCtrPending]) return;
   extern __shared__ __align__(16) unsigned char smem_arm[];
+  __shared__ ScanRows s_rows;
   ArmSmem t;
   stage_tables(s, smem_arm, &t);
-  if (!RESOLVE) after_previous();
+  if (!RESOLVE) {
+    after_previous();
+    load_scan_rows(ctr, &s_rows);
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   float2* wcs; float* wqv; float4* wsph; double* w64;
@@ -893,15 +927,16 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
   const int D = s.D;
   while (true) {
     long long k0 = 0;
-    // what the scan left is few and mostly free: one at a time
-    const int take = RESOLVE || list ? 1 : s.cfg_chunk;
+    // with a list: the rows the scan listed, then the rows it left.  What it listed
+    // is few and mostly free: one at a time.
+    const long long lim = RESOLVE ? (long long)ctr[kCtrPending] : (list ? scan_total(s_rows) : n);
+    const int take = RESOLVE || (list && s_rows.listed > lim / 2) ? 1 : s.cfg_chunk;
     if (lane == 0) k0 = atomicAdd(&ctr[RESOLVE ? kCtrQueue2 : kCtrQueue], take);
     k0 = __shfl_sync(MRMG_FULL, k0, 0);
-    const long long lim = RESOLVE ? (long long)ctr[kCtrPending] : (list ? (long long)ctr[kCtrListed] : n);
     if (k0 >= lim) break;
     const int cnt = (int)min((long long)take, lim - k0);
     for (int c = 0; c < cnt; c++) {
-      const long long i = RESOLVE ? pend[k0] : (list ? (long long)list[k0 + c].pad : k0 + c);
+      const long long i = RESOLVE ? pend[k0] : (list ? scan_item(s_rows, list, k0 + c) : k0 + c);
       const CfgSource src{q, dtype, i, D};
       uint8_t v = eval_config<GPL, SPG, RESOLVE>(s, t, wcs, wqv, wsph, w64, lane, src, full != 0);
       if (lane == 0) {
@@ -1021,9 +1056,13 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
   // pass 2: as many CTAs stay as there are undecided items for their warps
   if (RESOLVE && (long long)blockIdx.x * (blockDim.x >> 5) >= *(volatile int*)&ctr[kCtrPending]) return;
   extern __shared__ __align__(16) unsigned char smem_arm[];
+  __shared__ ScanRows s_rows;
   ArmSmem t;
   stage_tables(s, smem_arm, &t);
-  if (!RESOLVE) after_previous();
+  if (!RESOLVE) {
+    after_previous();
+    load_scan_rows(ctr, &s_rows);
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   float2* wcs; float* wqv; float4* wsph; double* w64;
@@ -1063,8 +1102,8 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
         e = sv.e;
       }
     } else {
-      if (k >= (listed ? (long long)ctr[kCtrListed] : n)) break;
-      e = listed ? (long long)surv[k].pad : k;
+      if (k >= (listed ? scan_total(s_rows) : n)) break;
+      e = listed ? scan_item(s_rows, surv, k) : k;
     }
     EdgeSourceDF sdf;
     float mloc;
@@ -1302,6 +1341,20 @@ __global__ void __launch_bounds__(256, GPL == 1 ? 3 : (GPL == 2 ? 2 : 1)) arm_ed
 // which keeps the set-up (an edge's step count, base frames) to dense rounds.
 // ---------------------------------------------------------------------------
 constexpr int kScanThreads = 128, kScanCtas = 5;
+// Whether that pays depends on the rows: what it ends is saved, what it lists is
+// walked twice.  So the warps add up what they see: a row that ends is worth
+// kScanWorth eighths of the longest chain's steps, a step of a row costs one, and
+// kScanSlack eighths per place are lent until the first rows can have ended.
+// Where the balance of all warps falls below that, rows under way are listed as
+// they are and the rows not begun are left to the warp kernels as one range, after
+// two or three steps in a batch of free rows.  Four arms, without the scan -> the
+// whole scan -> this, us: 200,000 free configurations among 50 boxes 713 -> 1,024
+// -> 714, of 16 boxes out of reach 452 -> 531 -> 465; 70,000 of them 305 -> 421 ->
+// 332 and 220 -> 238 -> 222 (10 to 25 us are what a batch of free configurations
+// pays); 200,000 edges of two steps from free configurations among 50 boxes 1,228
+// -> 1,452 -> 1,130; uniform configurations as with the whole scan.  Worth 6 or 8:
+// the same; slack 3 or 4: free batches 10 us more.
+constexpr int kScanWorth = 7, kScanSlack = 2;
 constexpr int kMaxScanMask = 16384;   // (group, box) reach tests per CTA, at most; beyond: every box is tested
 
 __host__ __device__ inline size_t scan_smem(const ArmDev& s) {
@@ -1342,10 +1395,11 @@ template <int SPG, bool EDGES>
 __global__ void __launch_bounds__(kScanThreads, kScanCtas) arm_scan_kernel(ArmDev s, const void* q1, const void* q2, int dtype,
                                                                    long long lo, long long hi, float res32, int incl,
                                                                    const long long* Np, long long N_start,
-                                                                   long long N_max, uint8_t* out, int* ctr, int queue,
+                                                                   long long N_max, uint8_t* out, int* ctr, int part,
                                                                    SurvivorEdge* surv) {
   extern __shared__ __align__(16) unsigned char smem_arm[];
   __shared__ int s_gbeg[kMaxRobots + 1], s_joint[kMaxRobots];
+  __shared__ int s_quit;   // the scan does not pay
   next_may_start();
   ArmSmem t;
   stage_tables(s, smem_arm, &t);
@@ -1353,6 +1407,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanCtas) arm_scan_kernel(ArmDe
   const int nw = (s.B + 31) / 32, np2 = (s.B + 1) / 2;
   uint32_t* reach = (uint32_t*)(bp + 3 * np2);         // [G][nw]: boxes within the group's reach
   __syncthreads();
+  if (threadIdx.x == 0) s_quit = 0;
   if (threadIdx.x <= s.R) {
     int c = 0;
     for (int g = 0; g < s.G; g++) c += (t.grp[g] & 0xff) < (int)threadIdx.x;
@@ -1394,6 +1449,18 @@ __global__ void __launch_bounds__(kScanThreads, kScanCtas) arm_scan_kernel(ArmDe
   __syncthreads();
 
   const int lane = threadIdx.x & 31, R = s.R, D = s.D;
+  int chain = 0;              // steps to the end of the longest chain
+  for (int i = 0; i < R; i++) chain = max(chain, s_gbeg[i + 1] - s_gbeg[i]);
+  int* queue = ctr + (part ? kCtrScanParts + part : kCtrScan);
+  unsigned long long* balance = (unsigned long long*)(ctr + kCtrScanBalance);
+  const int worth = max(1, chain * kScanWorth / 8);
+  const long long least = -(long long)max(1, chain * kScanSlack / 8) * (32 / R) * gridDim.x;
+  if (part) {   // what the parts before have shown
+    if (threadIdx.x == 0) s_quit = (long long)*(volatile unsigned long long*)balance < least;
+    __syncthreads();
+  }
+  long long seen = 0;
+  int gain = 0, turn = 0;
   const int places = 32 / R, place = lane / R, r = lane - place * R;   // configurations per warp; this lane's robot
   const bool used = place < places;
   const unsigned gmask = used ? ((1u << R) - 1u) << (place * R) : 0u;
@@ -1404,12 +1471,27 @@ __global__ void __launch_bounds__(kScanThreads, kScanCtas) arm_scan_kernel(ArmDe
   bool bad = false, exhausted = false;
   long long stat_cfg = 0;
   while (true) {
+    if (__any_sync(MRMG_FULL, *(volatile int*)&s_quit)) {   // list what is under way, leave the rest of the rows
+      const unsigned under = __ballot_sync(MRMG_FULL, idx >= 0 && lead);
+      int slot = 0;
+      if (lane == 0) {
+        if (under) slot = atomicAdd(&ctr[kCtrListed], __popc(under));
+        const int at = atomicMax(queue, (int)(hi - lo));
+        if (at < hi - lo) {
+          ctr[kCtrScanTails + 2 * part] = (int)(lo + at);
+          ctr[kCtrScanTails + 2 * part + 1] = (int)(hi - lo - at);
+        }
+      }
+      slot = __shfl_sync(MRMG_FULL, slot, 0);
+      if (idx >= 0 && lead) surv[slot + __popc(under & ((1u << lane) - 1u))].pad = (int)idx;
+      break;
+    }
     // ---- new configurations for the free places
     const unsigned idle = __ballot_sync(MRMG_FULL, used && idx < 0);
     const int free_places = __popc(idle) / R;
     if (!exhausted && 2 * free_places >= places) {
       long long base = 0;
-      if (lane == 0) base = lo + atomicAdd(&ctr[queue], free_places);
+      if (lane == 0) base = lo + atomicAdd(queue, free_places);
       base = __shfl_sync(MRMG_FULL, base, 0);
       exhausted = base + free_places >= hi;
       const bool fresh = used && idx < 0;
@@ -1600,6 +1682,17 @@ __global__ void __launch_bounds__(kScanThreads, kScanCtas) arm_scan_kernel(ArmDe
     if (dead && lead) {
       out[idx] = V_COLLIDE;
       stat_cfg++;
+    }
+    if (threadIdx.x < 32) {   // a warp per CTA keeps the balance (and looks at it when it is back, a post later)
+      gain += worth * __popc(__ballot_sync(MRMG_FULL, dead && lead)) - __popc(__ballot_sync(MRMG_FULL, idx >= 0 && lead));
+      if (turn < 4 || (turn & 7) == 0) {
+        if (lane == 0) {
+          if (seen < least) *(volatile int*)&s_quit = 1;
+          seen = (long long)atomicAdd(balance, (unsigned long long)(long long)gain) + gain;
+        }
+        gain = 0;
+      }
+      turn++;
     }
     if (lists) {
       int slot = 0;
@@ -2061,11 +2154,13 @@ int arm_prepare(const ArmDev& s, int warps) {
 }
 
 // The scan adds a pass of some 40 us of latency (seven links, one after another)
-// and pays where most configurations collide with a box and there are enough of
-// them for its lanes.  Measured, four arms, uniform configurations (before -> with
-// the scan): 200,000 among 50, 36, 22, 20 boxes 309 -> 197, 334 -> 230, 344 ->
-// 249, 378 -> 351 us, among 5 boxes 417 -> 499 us; 40,000 among 50, 36, 22 146 ->
-// 141, 146 -> 149, 157 -> 146 us; 10,000 among 50 89 -> 105 us.  Rows that are read
+// and pays where most configurations collide with a box (it stops where they do
+// not, see kScanWorth) and there are enough of them for its lanes.  Measured, four
+// arms, uniform configurations (without -> with the scan): 200,000 among 50, 22,
+// 20, 17 boxes 317 -> 161, 345 -> 219, 365 -> 321, 317 -> 160 us; 70,000 among 50,
+// 22 168 -> 121, 173 -> 133 us; when it was new, 40,000 among 50, 36, 22 146 ->
+// 141, 146 -> 149, 157 -> 146 us; 10,000 among 50 89 -> 105 us; 200,000 among 5
+// boxes, to the end, 417 -> 499 us.  Rows that are read
 // in place from host memory go without it (LaunchShape::host_rows): its lanes read
 // joint by joint, and what it lists is read again over the link; 100,000 edges from
 // numpy arrays 242 us without, 285 us with it.
@@ -2081,14 +2176,14 @@ bool arm_edges_scan(const ArmDev& s, long long n, int full) { return use_scan(s,
 template <bool EDGES>
 static cudaError_t launch_scan(const ArmDev& s, const void* q1, const void* q2, int dtype, long long lo, long long hi,
                                double res, int incl, const long long* Np, long long N_start, long long N_max,
-                               uint8_t* out, const CallScratch& sc, int queue, int ctas, cudaStream_t st) {
+                               uint8_t* out, const CallScratch& sc, int part, int ctas, cudaStream_t st) {
   const size_t smem = scan_smem(s);
   const int per_cta = kScanThreads / 32 * (32 / s.R);
   const int grid = (int)std::max(1ll, std::min((hi - lo + per_cta - 1) / per_cta, (long long)ctas));
 #define MRMG_ARM_SCAN(S_)                                                                          \
   if (s.SPG == S_) {                                                                               \
     arm_scan_kernel<S_, EDGES><<<grid, kScanThreads, smem, st>>>(s, q1, q2, dtype, lo, hi, (float)res, incl, Np,    \
-                                                                 N_start, N_max, out, sc.ctr, queue, sc.surv); \
+                                                                 N_start, N_max, out, sc.ctr, part, sc.surv); \
     return cudaGetLastError();                                                                     \
   }
   MRMG_ARM_SCAN(6)
@@ -2106,7 +2201,7 @@ cudaError_t arm_configs(const ArmDev& s, const void* q, int dtype, long long n, 
   int grid = (int)std::max(1ll, std::min(want, (long long)ls.ctas));
   const bool scan = use_scan(s, n, full) && !ls.host_rows;
   cudaError_t e = cudaSuccess;
-  if (scan) e = launch_scan<false>(s, q, nullptr, dtype, 0, n, 0.0, 0, nullptr, 0, -1, out, sc, kCtrScan, ls.num_sms * kScanCtas, st);
+  if (scan) e = launch_scan<false>(s, q, nullptr, dtype, 0, n, 0.0, 0, nullptr, 0, -1, out, sc, 0, ls.num_sms * kScanCtas, st);
   if (e == cudaSuccess) e = launch_configs<false>(s, gpl, q, dtype, n, out, sc, grid, ls.warps, smem1, full, scan, st);
   if (e != cudaSuccess) return e;
   return launch_configs<true>(s, gpl, q, dtype, n, out, sc, ls.num_sms * kResolveCtas, kResolveWarps,
@@ -2131,7 +2226,7 @@ cudaError_t arm_edges(const ArmDev& s, const void* q1, const void* q2, int dtype
     // beside the copy of the next part, the scan leaves it a CTA's registers
     if (scan && e == cudaSuccess && hi > lo)
       e = launch_scan<true>(s, q1, q2, dtype, lo, hi, res, incl, Np, N_start, N_max, out, sc,
-                            j ? kCtrScanParts + j : kCtrScan, ls.num_sms * (j + 1 < parts ? kScanCtas - 1 : kScanCtas),
+                            j, ls.num_sms * (j + 1 < parts ? kScanCtas - 1 : kScanCtas),
                             st);
     lo = hi;
   }

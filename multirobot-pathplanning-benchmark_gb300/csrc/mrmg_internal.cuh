@@ -138,7 +138,9 @@ constexpr int kCtrPendLost = 11;   // pending positions did not fit the list
 constexpr int kCtrDoneB = 10;   // CTAs of the last phase-B launch that have finished
 constexpr int kCtrScanParts = 16;   // the queues of the scans of a batch's further parts (PartFeed)
 constexpr int kMaxParts = 4;
-constexpr int kNumCtr = kCtrScanParts + kMaxParts;
+constexpr int kCtrScanTails = kCtrScanParts + kMaxParts;        // per part: first row and number of rows left unscanned
+constexpr int kCtrScanBalance = kCtrScanTails + 2 * kMaxParts;   // what the scan has saved so far, in its steps (64-bit)
+constexpr int kNumCtr = kCtrScanBalance + 2;
 
 // an edge that survived its first checked configuration: its remaining
 // BFS positions [p_next, nmax) are dealt to all warps
