@@ -22,6 +22,11 @@ constexpr int kMaxTileD = 128;    // coordinates staged per query
 constexpr int kNodesPerCta = 128;
 constexpr int kMinStaged = 4;     // queries from which staging a CTA's nodes pays (one query, 12,000 nodes, 28 coordinates:
                                   // 37 us in place, 42 us staged)
+// Distances of nodes read in place, too few to keep the FP64 pipe busy: the FP64
+// instructions, whose loads and chains overlap across coordinates (97 coordinates, 17
+// queries: 3,000 nodes 213 us, integer squares 498 us; 15,000 nodes 222 and 499 us);
+// 60 queries on 15,000 nodes 727 us in FP64 instructions, 552 us.
+constexpr long long kFewDists = 1ll << 18;
 constexpr size_t kMaxNodeTile = 96 * 1024;   // bytes of staged nodes: two CTAs per SM at least
 
 // out[q, m] = dist(queries[q] - nodes[m]).  A node per thread, the tile's
@@ -29,7 +34,7 @@ constexpr size_t kMaxNodeTile = 96 * 1024;   // bytes of staged nodes: two CTAs 
 // node's held in registers.  Else the CTA's nodes are staged in shared memory by
 // coordinate (XS; read from global memory, a row per lane, the L1 cache bound 28
 // coordinates at 0.94 ms per 1,000 x 10,000), or read in place where they do not fit.
-template <int DM, bool XS>
+template <int DM, bool XS, bool FAST1 = false>
 __global__ void __launch_bounds__(kNodesPerCta) dist_matrix_kernel(const double* __restrict__ qs, long long Q,
                                                                    const double* __restrict__ nodes, long long M,
                                                                    SliceTab t, int metric, double* __restrict__ out) {
@@ -66,7 +71,7 @@ __global__ void __launch_bounds__(kNodesPerCta) dist_matrix_kernel(const double*
             if (k < t.end_all) v = __dadd_rn(v, square_rn(__dsub_rn(qq[k], xr[k])));
           v = sqrt_rn(v);
         } else {
-          v = dist_of(t, metric, [&](int k) { return __dsub_rn(qq[k], XS ? xs[k * kNodesPerCta + threadIdx.x] : x[k]); });
+          v = dist_of<FAST1>(t, metric, [&](int k) { return __dsub_rn(qq[k], XS ? xs[k * kNodesPerCta + threadIdx.x] : x[k]); });
         }
         out[(q0 + j) * M + m] = v;
       }
@@ -132,6 +137,8 @@ cudaError_t dist_matrix(const double* qs, long long Q, const double* nodes, long
     e = allow_max_smem(dist_matrix_kernel<0, true>);
     if (e == cudaSuccess)
       dist_matrix_kernel<0, true><<<grid, kNodesPerCta, qt + tile, st>>>(qs, Q, nodes, M, t, metric, out);
+  } else if (Q * M < kFewDists) {
+    dist_matrix_kernel<0, false, true><<<grid, kNodesPerCta, qt, st>>>(qs, Q, nodes, M, t, metric, out);
   } else {
     dist_matrix_kernel<0, false><<<grid, kNodesPerCta, qt, st>>>(qs, Q, nodes, M, t, metric, out);
   }

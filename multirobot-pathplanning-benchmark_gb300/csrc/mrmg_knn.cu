@@ -73,7 +73,7 @@ __device__ __forceinline__ int warp_argmin(long long d, long long id) {
   return bl;
 }
 
-template <int KM>
+template <int KM, bool FAST1>
 __global__ void knn_exact_kernel(const double* __restrict__ qs, long long Q, const int* __restrict__ q_mode,
                                  const long long* __restrict__ q_list, long long n_list,
                                  const double* __restrict__ nodes, const long long* __restrict__ mode_beg,
@@ -96,7 +96,7 @@ __global__ void knn_exact_kernel(const double* __restrict__ qs, long long Q, con
     for (long long x = s + lane; x < e; x += 32) {
       const double* xx = nodes + x * D;
       auto dfun = [&](int j) { return __dsub_rn(qq[j], xx[j]); };
-      topk_insert<KM>(td, ti, k, dkey(dist_of(t, metric, dfun)), x - s);
+      topk_insert<KM>(td, ti, k, dkey(dist_of<FAST1>(t, metric, dfun)), x - s);
     }
     // merge the 32 sorted lane lists
     int head = 0;
@@ -241,14 +241,16 @@ __device__ __forceinline__ void write_sorted(long long d, int id, int lane, int 
   }
 }
 
-// q32 / x32: FP32 copies (rounded to nearest) of the FP64 rows qq / xx
+// q32 / x32: FP32 copies (rounded to nearest) of the FP64 rows qq / xx.  ROWS: the
+// plan has whole rows (whose registers would halve the warps of the other form).
+template <bool FAST1, bool ROWS>
 __device__ __forceinline__ bool within_radius(const float* __restrict__ q32, const float* __restrict__ x32,
                                               const double* __restrict__ qq, const double* __restrict__ xx,
                                               const SliceTab& t, int metric, const RadiusTest& r, RowPlan rows) {
   if (!(r.rp >= 0.0)) return false;   // distances are >= 0; NaN selects nothing
   if (metric == MRMG_METRIC_EUCLIDEAN || metric == MRMG_METRIC_MAX_EUCLIDEAN) {
     float qn = 0.f, xn = 0.f, m = 0.f;
-    if (rows.n4) {
+    if constexpr (ROWS) {
       float4 x4[8];
 #pragma unroll
       for (int i = 0; i < 8; i++)
@@ -296,7 +298,7 @@ __device__ __forceinline__ bool within_radius(const float* __restrict__ q32, con
     if (m > r.hi + bnd) return false;
   }
   auto dfun = [&](int j) { return __dsub_rn(qq[j], xx[j]); };
-  return dist_of(t, metric, dfun) <= r.rp;
+  return dist_of<FAST1>(t, metric, dfun) <= r.rp;
 }
 
 __global__ void f64_to_f32_kernel(const double* __restrict__ src, float* __restrict__ dst, long long n) {
@@ -324,7 +326,7 @@ __device__ __forceinline__ long long owner_of(const long long* __restrict__ off,
 // warp per item: the chunk's k best (distance key, mode-local index), ascending
 // (queries are listed entries: query qmap[l] for list entry l, or l itself
 // when qmap is NULL; q_mode is per list entry)
-template <int KM>
+template <int KM, bool FAST1>
 __global__ void knn_split_kernel(const double* __restrict__ qs, const long long* __restrict__ qmap, long long Q,
                                  const int* __restrict__ q_mode, const long long* __restrict__ ioff,
                                  const double* __restrict__ nodes,
@@ -349,7 +351,7 @@ __global__ void knn_split_kernel(const double* __restrict__ qs, const long long*
     for (long long x = s + lane; x < e; x += 32) {
       const double* xx = nodes + x * t.D;
       auto dfun = [&](int j) { return __dsub_rn(qq[j], xx[j]); };
-      topk_insert<KM>(td, ti, k, dkey(dist_of(t, metric, dfun)), x - b);
+      topk_insert<KM>(td, ti, k, dkey(dist_of<FAST1>(t, metric, dfun)), x - b);
     }
     int head = 0;
     for (int r = 0; r < k; r++) {
@@ -687,8 +689,10 @@ __global__ void knn_split32_merge_kernel(const double* __restrict__ qs, const lo
 }
 
 constexpr int kNearStage = 48;   // results staged per query, for the emit pass
+constexpr long long kFewResults = 8192;   // distances of results taken in FP64 instructions, at most
 
 // radius, exact: warp per (query, bitmap word), lane = node of the word
+template <bool FAST1, bool ROWS>
 __global__ void near_split_kernel(const double* __restrict__ qs, const float* __restrict__ qs32, long long Q,
                                   const int* __restrict__ q_mode, const double* __restrict__ nodes,
                                   const float* __restrict__ nodes32, const long long* __restrict__ mode_beg,
@@ -707,7 +711,7 @@ __global__ void near_split_kernel(const double* __restrict__ qs, const float* __
     bool in = false;
     if (id < mode_end[m] - mode_beg[m]) {
       const long long x = mode_beg[m] + id;
-      in = within_radius(qs32 + q * t.D, nodes32 + x * t.D, qs + q * t.D, nodes + x * t.D, t, metric,
+      in = within_radius<FAST1, ROWS>(qs32 + q * t.D, nodes32 + x * t.D, qs + q * t.D, nodes + x * t.D, t, metric,
                          radius_test(rp[q]), rows);
     }
     const unsigned mk = __ballot_sync(MRMG_FULL, in);
@@ -724,6 +728,17 @@ __global__ void near_split_kernel(const double* __restrict__ qs, const float* __
 
 }  // namespace
 
+// Warps of distances (a warp per query, or per query and chunk of nodes) too few
+// to keep the FP64 pipe busy, two per scheduler: they wait for the longer chains of
+// the integer squares and roots (mrmg_exact.cuh), so they take the FP64
+// instructions.  Whole calls with FP64 / integer arithmetic, sum over agents, 28-D:
+// one query on 150,000 nodes 101 / 127 us (293 warps), 700 queries on 700 nodes 126
+// / 130 us (1,050 warps), eight queries on 150,000 262 / 212 us (2,340 warps).
+// Lists longer than 16 leave the registers, and their insertion hides the FP64
+// pipe: FP64 instructions always (k = 40, 60 queries on 150,000 nodes 2,243 / 2,531
+// us).
+static bool few_warps(long long warps, int num_sms) { return warps <= 8ll * num_sms; }
+
 cudaError_t knn_exact(const double* qs, long long Q, const int* q_mode, const long long* q_list, long long n_list,
                       const double* nodes, const long long* mode_beg, const long long* mode_end, const SliceTab& t,
                       int metric, int k, long long* out_idx, double* out_dist, int num_sms, cudaStream_t st) {
@@ -731,12 +746,11 @@ cudaError_t knn_exact(const double* qs, long long Q, const int* q_mode, const lo
   if (total <= 0) return cudaSuccess;
   const int warps = 4;
   const int grid = (int)std::min<long long>((total + warps - 1) / warps, (long long)num_sms * 16);
-  if (k <= 16)
-    knn_exact_kernel<16><<<grid, warps * 32, 0, st>>>(qs, Q, q_mode, q_list, n_list, nodes, mode_beg, mode_end, t,
-                                                      metric, k, out_idx, out_dist);
-  else
-    knn_exact_kernel<kKnnMaxK><<<grid, warps * 32, 0, st>>>(qs, Q, q_mode, q_list, n_list, nodes, mode_beg, mode_end,
-                                                            t, metric, k, out_idx, out_dist);
+  auto kernel = k > 16                         ? knn_exact_kernel<kKnnMaxK, true>
+                : few_warps(total, num_sms) ? knn_exact_kernel<16, true>
+                                            : knn_exact_kernel<16, false>;
+  kernel<<<grid, warps * 32, 0, st>>>(qs, Q, q_mode, q_list, n_list, nodes, mode_beg, mode_end, t, metric, k, out_idx,
+                                      out_dist);
   return cudaGetLastError();
 }
 
@@ -1611,6 +1625,7 @@ constexpr int kNearWarps = 4;
 // bitmap, 56 us; 300 queries, whole call: 296 -> 228 us, with 11,600 results
 // each 4,910 -> 950 us.
 
+template <bool ROWS>
 __global__ void __launch_bounds__(32 * kNearWarps, 8) near_exact_kernel(const double* __restrict__ qs, const float* __restrict__ qs32, long long Q,
                                   const int* __restrict__ q_mode, const double* __restrict__ nodes,
                                   const float* __restrict__ nodes32, const long long* __restrict__ mode_beg,
@@ -1656,7 +1671,7 @@ __global__ void __launch_bounds__(32 * kNearWarps, 8) near_exact_kernel(const do
       const long long id = s_w[wib][w] * 32 + (loc & 31);
       if (id >= mode_end[m] - mode_beg[m]) continue;
       const long long xr = (mode_beg[m] + id) * t.D;
-      if (within_radius(qs32 + qx * t.D, nodes32 + xr, qs + qx * t.D, nodes + xr, t, metric, radius_test(rp[qx]),
+      if (within_radius<true, ROWS>(qs32 + qx * t.D, nodes32 + xr, qs + qx * t.D, nodes + xr, t, metric, radius_test(rp[qx]),
                         rows))
         atomicOr(&s_res[wib][w], 1u << (loc & 31));
     }
@@ -1773,9 +1788,9 @@ __global__ void near_dist_kernel(const double* __restrict__ qs, long long Q, con
     const long long q = owner_of(offs, Q, p);
     const double* qq = qs + q * t.D;
     const double* xx = nodes + (mode_beg[q_mode[q]] + out_idx[p]) * t.D;
-    // a warp or two: the FP64 instructions' latency is shorter (10.1 -> 9.4 us); more:
-    // their pipe is what is scarce
-    out_dist[p] = total <= 64 ? dist_rows<true>(qq, xx, t, metric, rows) : dist_rows(qq, xx, t, metric, rows);
+    // few warps: the FP64 instructions' latency is shorter (8 to 4,000 results 3 to 6 us
+    // less); more: their pipe is what is scarce (350,000 results 392 us a call, 364 us)
+    out_dist[p] = total <= kFewResults ? dist_rows<true>(qq, xx, t, metric, rows) : dist_rows(qq, xx, t, metric, rows);
   }
 }
 
@@ -2358,12 +2373,11 @@ static cudaError_t knn_split_query(KnnStore* s, KnnScratch* scr, const double* d
   if (e != cudaSuccess) return e;
   if (n_items > 0) {
     const int grid = (int)std::min<long long>((n_items + 3) / 4, (long long)num_sms * 16);
-    if (k <= 16)
-      knn_split_kernel<16><<<grid, 128, 0, st>>>(d_qs, d_map, L, d_qm, d_ioff, s->nodes, s->d_beg, s->d_end,
-                                                 s->slices, s->metric, k, d_ck, d_ci);
-    else
-      knn_split_kernel<kKnnMaxK><<<grid, 128, 0, st>>>(d_qs, d_map, L, d_qm, d_ioff, s->nodes, s->d_beg, s->d_end,
-                                                       s->slices, s->metric, k, d_ck, d_ci);
+    auto kernel = k > 16                           ? knn_split_kernel<kKnnMaxK, true>
+                  : few_warps(n_items, num_sms) ? knn_split_kernel<16, true>
+                                                : knn_split_kernel<16, false>;
+    kernel<<<grid, 128, 0, st>>>(d_qs, d_map, L, d_qm, d_ioff, s->nodes, s->d_beg, s->d_end, s->slices, s->metric, k,
+                                 d_ck, d_ci);
   }
   const int mgrid = (int)std::max<long long>(1, std::min<long long>((L + 3) / 4, (long long)num_sms * 16));
   if (k <= 16)
@@ -2630,13 +2644,19 @@ cudaError_t near_query(NearState* ns, KnnStore* s, const double* d_qs, long long
   if (tc) {
     const long long blocks = (Wtot + 32 * kNearWarps - 1) / (32 * kNearWarps);
     if (blocks > 0)
-      near_exact_kernel<<<(int)std::min<long long>(blocks, (long long)num_sms * 12), 32 * kNearWarps, 0, st>>>(
+      (rows.n4 ? near_exact_kernel<true> : near_exact_kernel<false>)<<<(int)std::min<long long>(blocks, (long long)num_sms * 12),
+                                                                        32 * kNearWarps, 0, st>>>(
           d_qs, d_q32, Q, d_qmode, nodes, s->nodes32, s->d_beg, s->d_end, t, metric, d_rp, d_woff, d_bits,
           (unsigned long long*)d_cnt, d_stage, rows);
   } else {
     if (Wtot > 0) {
       const int g2 = (int)std::min<long long>((Wtot + 3) / 4, (long long)num_sms * 16);
-      near_split_kernel<<<g2, 128, 0, st>>>(d_qs, d_q32, Q, d_qmode, nodes, s->nodes32, s->d_beg, s->d_end, t, metric,
+      // (the FP32 pre-test leaves few distances of two of the metrics)
+      const bool fp64 = metric == MRMG_METRIC_EUCLIDEAN || metric == MRMG_METRIC_MAX_EUCLIDEAN || few_warps(Wtot, num_sms);
+      auto kernel = rows.n4 ? near_split_kernel<true, true>
+                    : fp64 ? near_split_kernel<true, false>
+                           : near_split_kernel<false, false>;
+      kernel<<<g2, 128, 0, st>>>(d_qs, d_q32, Q, d_qmode, nodes, s->nodes32, s->d_beg, s->d_end, t, metric,
                                             d_rp, d_woff, d_bits, (unsigned long long*)d_cnt, d_stage, rows);
     }
   }
