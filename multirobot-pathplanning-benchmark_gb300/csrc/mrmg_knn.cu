@@ -1613,77 +1613,108 @@ __global__ void __launch_bounds__(32 * kMergeWarps, 4) knn_merge_kernel(const do
 // ---------------------------------------------------------------------------
 constexpr int kNearWarps = 4;
 
-// Exact check of the candidate bitmap.  A warp takes 32 consecutive words of all
-// queries' bitmaps (a lane each; most hold no bit), lists their set bits in
-// shared memory and spreads them over the lanes for the radius test, so neither a
-// long bitmap nor a dense word serialises one lane.  Bits that fail (or lie past
+// Exact check of the candidate bitmap.  A warp takes chunks of consecutive words of
+// all queries' bitmaps, 32 at a time (a lane each; most hold no bit), lists their
+// set bits in shared memory and spreads them over the lanes for the radius test, so
+// neither a long bitmap nor a dense word serialises one lane.  A word's query, first
+// node and radius are looked up once per word, not per candidate, the query by one
+// search per chunk; a query's count is one atomic per 32 words.  Bits that fail (or lie past
 // the mode's nodes) are cleared, the rest counted per query; a query's first
 // kNearStage results to arrive are staged, in any order, for the emit pass.
 // Bound: the candidates' rows from L2 (some 600 candidates per query lie within
 // the tile kernel's error bound of the radius).  2,001 queries on 150,000 nodes,
 // max over agents, 16 results each: 93 us with a warp per query walking its
 // bitmap, 56 us; 300 queries, whole call: 296 -> 228 us, with 11,600 results
-// each 4,910 -> 950 us.
-
+// each 4,910 -> 950 us.  4,000 queries on 40,000 nodes of one mode, 500 results
+// each: 147 us with a warp per query, 311 us with the look-ups per candidate and an
+// atomic per word, 190 us (the whole call 935, 962 and 827 us).  Six CTAs per SM: 8
+// spill 128 bytes a thread (879 us for that call), 7 851 us.
 template <bool ROWS>
-__global__ void __launch_bounds__(32 * kNearWarps, 8) near_exact_kernel(const double* __restrict__ qs, const float* __restrict__ qs32, long long Q,
+__global__ void __launch_bounds__(32 * kNearWarps, 6) near_exact_kernel(const double* __restrict__ qs, const float* __restrict__ qs32, long long Q,
                                   const int* __restrict__ q_mode, const double* __restrict__ nodes,
                                   const float* __restrict__ nodes32, const long long* __restrict__ mode_beg,
                                   const long long* __restrict__ mode_end, SliceTab t,
                                   int metric, const double* __restrict__ rp, const long long* __restrict__ woff,
                                   unsigned* __restrict__ bits, unsigned long long* __restrict__ counts,
-                                  int* __restrict__ stage, RowPlan rows) {
+                                  int* __restrict__ stage, RowPlan rows, int chunk) {
   __shared__ unsigned short s_list[kNearWarps][1024];   // word of the 32 and bit
   __shared__ unsigned s_res[kNearWarps][32];
+  // per word: its query, its first node, and the query's radius
   __shared__ int s_q[kNearWarps][32];
-  __shared__ long long s_w[kNearWarps][32];
+  __shared__ long long s_x[kNearWarps][32];
+  __shared__ double s_rp[kNearWarps][32];
+  __shared__ float2 s_r2[kNearWarps][32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const long long step = (long long)gridDim.x * kNearWarps * 32;
+  const long long step = (long long)gridDim.x * kNearWarps * chunk;
   const long long total = woff[Q];
   unsigned short* list = s_list[wib];
-  for (long long base = ((long long)blockIdx.x * kNearWarps + wib) * 32; base < total; base += step) {
-    const long long f = base + lane;
-    const unsigned mk = f < total ? bits[f] : 0u;
-    if (!__any_sync(MRMG_FULL, mk != 0u)) continue;
-    const int c = __popc(mk);
-    int incl = c;
+  for (long long c0 = ((long long)blockIdx.x * kNearWarps + wib) * chunk; c0 < total; c0 += step) {
+    long long q = owner_of(woff, Q, c0);   // of this lane's word, carried from word to word
+    for (long long base = c0; base < c0 + chunk && base < total; base += 32) {
+      const long long f = base + lane;
+      unsigned mk = f < total ? bits[f] : 0u;
+      if (!__any_sync(MRMG_FULL, mk != 0u)) continue;
+      if (f < total)
+        while (f >= woff[q + 1]) q++;
+      if (mk) {
+        const int m = q_mode[q];
+        const long long x0 = mode_beg[m] + (f - woff[q]) * 32, left = mode_end[m] - x0;
+        const RadiusTest rt = radius_test(rp[q]);
+        s_q[wib][lane] = (int)q;
+        s_x[wib][lane] = x0;
+        s_rp[wib][lane] = rt.rp;
+        s_r2[wib][lane] = make_float2(rt.lo, rt.hi);
+        const unsigned in = left >= 32 ? mk : (left > 0 ? mk & ((1u << left) - 1u) : 0u);
+        if (in != mk) bits[f] = in;   // (bits past the mode's nodes)
+        mk = in;
+      }
+      const int c = __popc(mk);
+      int incl = c;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(MRMG_FULL, incl, o);
-      if (lane >= o) incl += y;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(MRMG_FULL, incl, o);
+        if (lane >= o) incl += y;
+      }
+      const int n = __shfl_sync(MRMG_FULL, incl, 31);
+      int pos = incl - c;
+      for (unsigned mm = mk; mm; mm &= mm - 1) list[pos++] = (unsigned short)(lane * 32 + __ffs(mm) - 1);
+      s_res[wib][lane] = 0u;
+      __syncwarp();
+      for (int x = lane; x < n; x += 32) {
+        const int loc = list[x], w = loc >> 5;
+        const long long qr = (long long)s_q[wib][w] * t.D, xr = (s_x[wib][w] + (loc & 31)) * t.D;
+        const float2 r2 = s_r2[wib][w];
+        if (within_radius<true, ROWS>(qs32 + qr, nodes32 + xr, qs + qr, nodes + xr, t, metric,
+                                      RadiusTest{s_rp[wib][w], r2.x, r2.y}, rows))
+          atomicOr(&s_res[wib][w], 1u << (loc & 31));
+      }
+      __syncwarp();
+      unsigned res = s_res[wib][lane];
+      if (res != mk) bits[f] = res;
+      // the words' results counted: one atomic per query, by its first word's lane
+      const int rc = __popc(res);
+      int ri = rc;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(MRMG_FULL, ri, o);
+        if (lane >= o) ri += y;
+      }
+      if (__shfl_sync(MRMG_FULL, ri, 31)) {
+        const long long before = __shfl_up_sync(MRMG_FULL, q, 1);
+        const unsigned heads = __ballot_sync(MRMG_FULL, lane == 0 || q != before);
+        const int head = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+        const unsigned after = lane < 31 ? heads & (0xfffffffeu << lane) : 0u;
+        const int last = after ? __ffs(after) - 2 : 31;
+        const int first = __shfl_sync(MRMG_FULL, ri - rc, head);   // results of the words before the query's first
+        const int sum = __shfl_sync(MRMG_FULL, ri, last) - first;
+        unsigned long long at = 0;
+        if (lane == head && sum) at = atomicAdd(counts + q, (unsigned long long)sum);
+        at = __shfl_sync(MRMG_FULL, at, head) + (unsigned)(ri - rc - first);
+        for (; res && at < kNearStage; res &= res - 1)
+          stage[q * kNearStage + at++] = (int)((f - woff[q]) * 32 + __ffs(res) - 1);
+      }
+      __syncwarp();   // the next words reuse the lists
     }
-    const int n = __shfl_sync(MRMG_FULL, incl, 31);
-    int pos = incl - c;
-    // the words' queries: one search, then the next query while the word lies past this one
-    long long q = owner_of(woff, Q, base);
-    if (mk) {
-      while (f >= woff[q + 1]) q++;
-      s_q[wib][lane] = (int)q;
-      s_w[wib][lane] = f - woff[q];
-    }
-    for (unsigned mm = mk; mm; mm &= mm - 1) list[pos++] = (unsigned short)(lane * 32 + __ffs(mm) - 1);
-    s_res[wib][lane] = 0u;
-    __syncwarp();
-    for (int x = lane; x < n; x += 32) {
-      const int loc = list[x], w = loc >> 5;
-      const long long qx = s_q[wib][w];
-      const int m = q_mode[qx];
-      const long long id = s_w[wib][w] * 32 + (loc & 31);
-      if (id >= mode_end[m] - mode_beg[m]) continue;
-      const long long xr = (mode_beg[m] + id) * t.D;
-      if (within_radius<true, ROWS>(qs32 + qx * t.D, nodes32 + xr, qs + qx * t.D, nodes + xr, t, metric, radius_test(rp[qx]),
-                        rows))
-        atomicOr(&s_res[wib][w], 1u << (loc & 31));
-    }
-    __syncwarp();
-    unsigned res = s_res[wib][lane];
-    if (res != mk) bits[f] = res;
-    if (res) {
-      unsigned long long at = atomicAdd(counts + q, (unsigned long long)__popc(res));
-      for (; res && at < kNearStage; res &= res - 1)
-        stage[q * kNearStage + at++] = (int)((f - woff[q]) * 32 + __ffs(res) - 1);
-    }
-    __syncwarp();   // the next words reuse the lists
   }
 }
 
@@ -2642,12 +2673,16 @@ cudaError_t near_query(NearState* ns, KnnStore* s, const double* d_qs, long long
   const int grid = near_grid(Q, num_sms);
   const RowPlan rows = row_plan(t, metric);
   if (tc) {
-    const long long blocks = (Wtot + 32 * kNearWarps - 1) / (32 * kNearWarps);
-    if (blocks > 0)
+    if (Wtot > 0) {
+      // words per warp and turn: at least four turns of every warp
+      const long long turns = (Wtot + 31) / 32, warps = (long long)num_sms * 12 * kNearWarps;
+      const int chunk = 32 * (int)std::max(1ll, std::min(16ll, turns / (4 * warps)));
+      const long long blocks = (turns * 32 + (long long)kNearWarps * chunk - 1) / ((long long)kNearWarps * chunk);
       (rows.n4 ? near_exact_kernel<true> : near_exact_kernel<false>)<<<(int)std::min<long long>(blocks, (long long)num_sms * 12),
                                                                         32 * kNearWarps, 0, st>>>(
           d_qs, d_q32, Q, d_qmode, nodes, s->nodes32, s->d_beg, s->d_end, t, metric, d_rp, d_woff, d_bits,
-          (unsigned long long*)d_cnt, d_stage, rows);
+          (unsigned long long*)d_cnt, d_stage, rows, chunk);
+    }
   } else {
     if (Wtot > 0) {
       const int g2 = (int)std::min<long long>((Wtot + 3) / 4, (long long)num_sms * 16);
