@@ -18,9 +18,10 @@
 // walks one robot's chain for its waypoints) and is recomputed, not stored, when
 // the gradient is asked for.  Few segments: a cluster of CTAs shares each.  The gradient of a joint angle theta_k follows the geometric Jacobian:
 // with o, z the origin and z axis of frame k-1 and g_s = dcost/dc_s,
-//   dcost/dtheta_k = z . sum_{s beyond joint k} (c_s - o) x g_s
-//                  = z . (M - o x G),  M = sum c_s x g_s,  G = sum g_s,
-// accumulated from the tip back.  FP32 throughout; per-lane sums are
+//   dcost/dtheta_k = z . sum_{s beyond joint k} (c_s - o) x g_s = z . M,
+// accumulated from the tip back: M is moved from one joint's origin to the next,
+// M += (o' - o) x G with G = sum g_s, so its lever arms stay short (about the world's
+// origin, z . (M - o x G) loses digits to the difference).  FP32 throughout; per-lane sums are
 // compensated and segment totals are added in FP64 in a fixed order, so the
 // cost and gradient are deterministic (no atomics: with the gradient, each
 // inter-robot pair is evaluated from both sides).
@@ -560,34 +561,58 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
       const int r = gr0 + HV * warp + half;
       const int nl = a.nl[r];
       int jo = a.q_off[r] + (a.base_kind[r] == 1 ? 3 : 0);
-      float G0 = 0.f, G1 = 0.f, G2 = 0.f, M0 = 0.f, M1 = 0.f, M2 = 0.f;
+      // sums of g and of the moments, compensated: the rounding of the pair terms
+      // is then what is left of the error
+      float G[3] = {0.f, 0.f, 0.f}, M[3] = {0.f, 0.f, 0.f}, Gl[3] = {0.f, 0.f, 0.f}, Ml[3] = {0.f, 0.f, 0.f};
+      float o[3] = {0.f, 0.f, 0.f};   // the point M is about: the joint's frame origin
       float* qg = QG + wl * D;
-      for (int k = nl; k >= 0; k--) {
-        for (int s = pd.lk[r][k]; s < pd.lk[r][k + 1]; s++) {
-          const float c0 = C[cen<SEG>(s, 0, wl)], c1 = C[cen<SEG>(s, 1, wl)], c2 = C[cen<SEG>(s, 2, wl)];
-          const int sg = s - s_lo;
-          const float g0 = Gs[(3 * sg) * SEG + wl], g1 = Gs[(3 * sg + 1) * SEG + wl], g2 = Gs[(3 * sg + 2) * SEG + wl];
-          G0 += g0; G1 += g1; G2 += g2;
-          M0 += c1 * g2 - c2 * g1;
-          M1 += c2 * g0 - c0 * g2;
-          M2 += c0 * g1 - c1 * g0;
-        }
-        if (k == 0) break;
+      const bool planar = a.base_kind[r] == 1;
+      const int b0 = a.q_off[r];
+      for (int k = nl; k >= (planar ? 0 : 1); k--) {
         const float* oz = OZ + (size_t)(((r - gr0) * kMaxLinks + (k - 1)) * 6) * SEG + wl;
-        const float o0 = oz[0], o1 = oz[SEG], o2 = oz[2 * SEG];
-        const float z0 = oz[3 * SEG], z1 = oz[4 * SEG], z2 = oz[5 * SEG];
-        const float v0 = M0 - (o1 * G2 - o2 * G1), v1 = M1 - (o2 * G0 - o0 * G2), v2 = M2 - (o0 * G1 - o1 * G0);
-        qg[jo + k - 1] = z0 * v0 + z1 * v1 + z2 * v2;
+        float d[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          const float n = k > 0 ? oz[i * SEG] : (i < 2 ? W[(wl + 1) * D + b0 + i] : 0.f);
+          d[i] = o[i] - n;
+          o[i] = n;
+        }
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          const int j = (i + 1) % 3, l = (i + 2) % 3;
+          acc2(M[i], Ml[i], d[j] * (G[l] + Gl[l]) - d[l] * (G[j] + Gl[j]));
+        }
+        float gs[3] = {0.f, 0.f, 0.f}, ms[3] = {0.f, 0.f, 0.f};   // this link's spheres
+        for (int s = pd.lk[r][k]; s < pd.lk[r][k + 1]; s++) {
+          float c[3], g[3];
+#pragma unroll
+          for (int i = 0; i < 3; i++) {
+            c[i] = C[cen<SEG>(s, i, wl)] - o[i];
+            g[i] = Gs[(3 * (s - s_lo) + i) * SEG + wl];
+          }
+#pragma unroll
+          for (int i = 0; i < 3; i++) {
+            const int j = (i + 1) % 3, l = (i + 2) % 3;
+            gs[i] += g[i];
+            ms[i] += c[j] * g[l] - c[l] * g[j];
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          acc2(G[i], Gl[i], gs[i]);
+          acc2(M[i], Ml[i], ms[i]);
+        }
+        if (k > 0)
+          qg[jo + k - 1] = oz[3 * SEG] * (M[0] + Ml[0]) + oz[4 * SEG] * (M[1] + Ml[1]) + oz[5 * SEG] * (M[2] + Ml[2]);
       }
-      if (a.base_kind[r] == 1) {
-        const int b0 = a.q_off[r];
-        const float x = W[(wl + 1) * D + b0], y = W[(wl + 1) * D + b0 + 1];
-        qg[b0] = G0;
-        qg[b0 + 1] = G1;
-        qg[b0 + 2] = M2 - (x * G1 - y * G0);
+      if (planar) {
+        qg[b0] = G[0] + Gl[0];
+        qg[b0 + 1] = G[1] + Gl[1];
+        qg[b0 + 2] = M[2] + Ml[2];
       }
     }
   }
+
   const int t = t0 + wl;
   if (COST && warp == 0 && rank == 0) {
     double c = csum;
