@@ -33,7 +33,9 @@ namespace mrmg {
 namespace {
 
 constexpr int kMaxSplit = 8;              // CTAs that share a segment, at most (a portable cluster)
-constexpr double kFixedShare = 0.1;       // a CTA's fixed work over a whole segment's pair work
+// a CTA's fixed work over a whole segment's pair work: a part that does not depend
+// on the scene, and what is worth this many pairs per waypoint
+constexpr double kFixedShare = 0.05, kFixedPairs = 3000.0;
 
 __host__ __device__ inline size_t al4(size_t n) { return (n + 3) & ~(size_t)3; }
 
@@ -664,15 +666,20 @@ __global__ void pen_sum_kernel(const double* __restrict__ seg, long long P, int 
 }
 
 // CTAs per segment: a segment's pair tasks go to a cluster of `s` CTAs where the
-// segments alone leave SMs idle.  Modelled time: waves of CTAs, each paying the
-// fixed part (tables, kinematics, joint gradients: about a tenth of a segment's
-// time by clock stamps) and its share of the pairs.  24 segments on 152 SMs: one
-// CTA each 117 us, clusters of 8 80 us (cost kernel).
-int pen_split(long long segs, int slots) {
+// segments alone leave SMs idle.  Modelled time: rounds of a CTA per SM (two on one
+// SM take as long as one after the other), each paying the fixed part (tables,
+// kinematics, joint gradients) and its share of the pairs per waypoint.  24
+// segments on 152 SMs, four arms, 50 boxes: one CTA each 81 us, clusters of 8 50 us
+// (cost kernel).  Against the best of 1, 2, 4 and 8 on 189 calls (seven scenes of 56
+// to 304 spheres, 1 to 200 paths) the choice loses 0.5 %; rounds of all resident
+// CTAs and a fixed part of a tenth lost 5.4 % (200 segments of two mobile robots 55
+// us, a CTA each 52).
+int pen_split(long long segs, int num_sms, double pairs) {
+  const double fixed = kFixedShare + kFixedPairs / std::max(pairs, 1.0);
   int best = 1;
   double best_t = 0.0;
   for (int s = 1; s <= kMaxSplit; s *= 2) {
-    const double t = (double)((segs * s + slots - 1) / slots) * (kFixedShare + 1.0 / s);
+    const double t = (double)((segs * s + num_sms - 1) / num_sms) * (fixed + 1.0 / s);
     if (s == 1 || t < best_t) {
       best = s;
       best_t = t;
@@ -720,7 +727,9 @@ cudaError_t launch_form(const ArmDev& a, const PenDev& pd, const PenParams& pp, 
   // the largest x2 of any pair: centres coincide, or lie deepest in a box
   const bool direct = pp.beta * 1.4426951f * (pp.margin + pd.reach) <= kDirectMax;
   const int nseg = pen_segments(T, SEG);
-  int split = pen_split(P * nseg, num_sms * (GRAD && SEG == 32 ? 1 : 2));
+  // (with the gradient each pair of spheres is evaluated from both sides)
+  const double pairs = (double)pd.S * (pd.B + (double)pd.S * (a.R - 1) / a.R * (GRAD ? 1.0 : 0.5));
+  int split = pen_split(P * nseg, num_sms, pairs);
   // (1 KB per CTA is the system's; a cluster keeps its tasks' costs in shared memory too)
   while (split > 1 && smem_bytes<SEG>(a, pd, GRAD, warps, pd.NTK, gr0, gr1) + 1024 > smem_sm)
     split /= 2;
