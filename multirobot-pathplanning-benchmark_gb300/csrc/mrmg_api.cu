@@ -1083,11 +1083,16 @@ int mrmg_serving_check(mrmg_scene* sc, const void* h_table, int32_t max_src, int
     return fail(MRMG_ERR_ARG, "mrmg_serving_check: max_src 0..65534, capacities >= 0");
   const long long n = ccap + ecap;
   if (n > kMaxBatch) return fail(MRMG_ERR_ARG, "batch of %lld exceeds %lld items; split it", n, kMaxBatch);
-  if (n == 0) return MRMG_OK;
   cudaStream_t st = (cudaStream_t)stream, gs = (cudaStream_t)gather_stream;
+  cudaError_t e = cudaSuccess;
+  if (n == 0) {   // no rows to check; a table that names some is reported
+    e = cudaMemsetAsync(d_gather_err, 0, sizeof(int32_t), st);
+    if (e == cudaSuccess)
+      e = serving_gather(h_table, max_src, sc->q_dim, 0, 0, 0, 0, d_q1, d_q2, (long long*)d_N, d_gather_err, sc->num_sms, st);
+    return e == cudaSuccess ? MRMG_OK : cuda_fail(e, "launch serving gather");
+  }
   int rc = ensure_pending(sc, n, st);
   if (rc) return rc;
-  cudaError_t e = cudaSuccess;
   for (cudaEvent_t& ev : sc->part_ev)
     if (!ev && e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
   if (e != cudaSuccess) return cuda_fail(e, "cudaEventCreate");
