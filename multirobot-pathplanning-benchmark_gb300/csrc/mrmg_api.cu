@@ -98,7 +98,7 @@ struct ArmTables {
   // host data kept until the upload
   std::vector<float4> sph32, band32, gbs, pen_sph, pen_box;
   std::vector<double> sph64;
-  std::vector<int4> pen_task;
+  std::vector<int2> pen_task;
 };
 
 // work-queue counters are 32-bit: keep every batch well below 2^31
@@ -343,7 +343,7 @@ void pen_tables(const ArmSrc& a, int R, const std::vector<char>& on, const std::
     int acc = s0;
     for (int k = 0; k <= kMaxLinks; k++) { pd.lk[r][k] = acc; acc += cnt[k]; }
     pd.lk[r][kMaxLinks + 1] = acc;
-    for (int i = s0; i < s1; i += 2) t->pen_task.push_back(make_int4(i, i + 1, s0, s1));
+    for (int i = s0; i < s1; i += 2) t->pen_task.push_back(make_int2(s0, s1));
   }
   t->pen_box.assign(2 * boxes.size(), make_float4(0.f, 0.f, 0.f, 0.f));
   for (size_t j = 0; j < boxes.size(); j++) {
@@ -409,7 +409,7 @@ void add_tables(DevBlock& blk, ArmTables* t) {
 void trim_tables(ArmTables* t) {
   for (auto* v : {&t->sph32, &t->band32, &t->gbs, &t->pen_sph, &t->pen_box}) std::vector<float4>().swap(*v);
   std::vector<double>().swap(t->sph64);
-  std::vector<int4>().swap(t->pen_task);
+  std::vector<int2>().swap(t->pen_task);
 }
 
 }  // namespace

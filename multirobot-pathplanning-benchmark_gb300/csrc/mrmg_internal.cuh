@@ -117,7 +117,7 @@ struct PenDev {
   int real;              // spheres without the padding
   float reach;           // largest -d of any pair: two radii, or a radius and half a box's smallest extent
   const float4* sph;     // [S]  local xyz, radius
-  const int4* task;      // [NTK] first sphere, second sphere, the robot's first sphere, the next robot's first
+  const int2* task;      // [NTK] of the robot of spheres 2 t and 2 t + 1: its first sphere, the next robot's first
   const float4* box;     // [2B] centre xyz, half extents xyz
   int lk[kMaxRobots][kMaxLinks + 2];   // spheres of (robot r, frame k): [lk[r][k], lk[r][k+1])
 };

@@ -454,9 +454,9 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
   for (int base = 0, turn = 0; base < NTK; base += VW, turn ^= 1) {
     const int tk = turn ? base + VW - 1 - vw : base + vw;
     if (tk >= NTK) continue;
-    const int4 task = __ldg(&pd.task[tk]);   // first sphere, -, robot's first sphere, next robot's first
-    if (GRAD && !COST && (task.x < s_lo || task.x >= s_hi)) continue;   // another group's robot
-    const int i0 = task.x, i1 = i0 + 1;
+    const int2 task = __ldg(&pd.task[tk]);   // the robot's first sphere, the next robot's first
+    const int i0 = 2 * tk, i1 = i0 + 1;
+    if (GRAD && !COST && (i0 < s_lo || i0 >= s_hi)) continue;   // another group's robot
     auto side = [&](int i) {
       Side d;
       d.nx = bc2(-C[cen<SEG>(i, 0, wl)]);
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
     };
     const float2 none = bc2(MRMG_PEN_NONE);
     {   // the later robots' spheres
-      const int j0 = task.w / 2, j1 = S / 2, je = j0 + ((j1 - j0) & ~(HV - 1));
+      const int j0 = task.y / 2, j1 = S / 2, je = j0 + ((j1 - j0) & ~(HV - 1));
 #pragma unroll 4
       for (int j = j0; j < je; j += HV) {
         spheres(Flag<COST>(), j + half, br2[j + half]);
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(GRAD && SEG == 16 ? 384 : 512, GRAD && SEG == 
       flush_product<COST>(b);
     }
     if (GRAD) {   // the earlier robots' (the cost has counted them)
-      const int z = task.z / 2, ze = z & ~(HV - 1);
+      const int z = task.x / 2, ze = z & ~(HV - 1);
 #pragma unroll 4
       for (int j = 0; j < ze; j += HV) spheres(Flag<false>(), j + half, br2[j + half]);
       if (HV > 1 && ze < z) spheres(Flag<false>(), ze, half ? none : br2[ze]);
