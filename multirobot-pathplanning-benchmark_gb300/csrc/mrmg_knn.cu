@@ -1627,10 +1627,13 @@ constexpr int kNearWarps = 4;
 // bitmap, 56 us; 300 queries, whole call: 296 -> 228 us, with 11,600 results
 // each 4,910 -> 950 us.  4,000 queries on 40,000 nodes of one mode, 500 results
 // each: 147 us with a warp per query, 311 us with the look-ups per candidate and an
-// atomic per word, 190 us (the whole call 935, 962 and 827 us).  Six CTAs per SM: 8
-// spill 128 bytes a thread (879 us for that call), 7 851 us.
+// atomic per word, 175 us (the whole call 935, 962 and 827 us); a search per 32 words
+// 238 us.  Six CTAs per SM where rows are read whole (8 spill: 204 us, and 68 instead
+// of 59 us for the 2,001 queries), eight where they are not (4,000 queries in 6-D 101
+// us, six 112).
+__host__ __device__ constexpr int near_ctas(bool rows) { return rows ? 6 : 8; }
 template <bool ROWS>
-__global__ void __launch_bounds__(32 * kNearWarps, 6) near_exact_kernel(const double* __restrict__ qs, const float* __restrict__ qs32, long long Q,
+__global__ void __launch_bounds__(32 * kNearWarps, near_ctas(ROWS)) near_exact_kernel(const double* __restrict__ qs, const float* __restrict__ qs32, long long Q,
                                   const int* __restrict__ q_mode, const double* __restrict__ nodes,
                                   const float* __restrict__ nodes32, const long long* __restrict__ mode_beg,
                                   const long long* __restrict__ mode_end, SliceTab t,
@@ -1691,15 +1694,14 @@ __global__ void __launch_bounds__(32 * kNearWarps, 6) near_exact_kernel(const do
       __syncwarp();
       unsigned res = s_res[wib][lane];
       if (res != mk) bits[f] = res;
-      // the words' results counted: one atomic per query, by its first word's lane
-      const int rc = __popc(res);
-      int ri = rc;
+      if (__any_sync(MRMG_FULL, res != 0u)) {   // counted: one atomic per query, by its first word's lane
+        const int rc = __popc(res);
+        int ri = rc;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(MRMG_FULL, ri, o);
-        if (lane >= o) ri += y;
-      }
-      if (__shfl_sync(MRMG_FULL, ri, 31)) {
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(MRMG_FULL, ri, o);
+          if (lane >= o) ri += y;
+        }
         const long long before = __shfl_up_sync(MRMG_FULL, q, 1);
         const unsigned heads = __ballot_sync(MRMG_FULL, lane == 0 || q != before);
         const int head = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
@@ -2675,10 +2677,11 @@ cudaError_t near_query(NearState* ns, KnnStore* s, const double* d_qs, long long
   if (tc) {
     if (Wtot > 0) {
       // words per warp and turn: at least four turns of every warp
-      const long long turns = (Wtot + 31) / 32, warps = (long long)num_sms * 12 * kNearWarps;
+      const int ctas = num_sms * near_ctas(rows.n4 != 0);
+      const long long turns = (Wtot + 31) / 32, warps = (long long)ctas * kNearWarps;
       const int chunk = 32 * (int)std::max(1ll, std::min(16ll, turns / (4 * warps)));
       const long long blocks = (turns * 32 + (long long)kNearWarps * chunk - 1) / ((long long)kNearWarps * chunk);
-      (rows.n4 ? near_exact_kernel<true> : near_exact_kernel<false>)<<<(int)std::min<long long>(blocks, (long long)num_sms * 12),
+      (rows.n4 ? near_exact_kernel<true> : near_exact_kernel<false>)<<<(int)std::min<long long>(blocks, ctas),
                                                                         32 * kNearWarps, 0, st>>>(
           d_qs, d_q32, Q, d_qmode, nodes, s->nodes32, s->d_beg, s->d_end, t, metric, d_rp, d_woff, d_bits,
           (unsigned long long*)d_cnt, d_stage, rows, chunk);
