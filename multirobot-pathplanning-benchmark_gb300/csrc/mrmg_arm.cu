@@ -918,7 +918,7 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
   stage_tables(s, smem_arm, &t);
   if (!RESOLVE) {
     after_previous();
-    load_scan_rows(ctr, &s_rows);
+    if (list) load_scan_rows(ctr, &s_rows);
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(256, RESOLVE ? 1 : (GPL == 1 ? 4 : (GPL == 2 ?
   stage_tables(s, smem_arm, &t);
   if (!RESOLVE) {
     after_previous();
-    load_scan_rows(ctr, &s_rows);
+    if (listed) load_scan_rows(ctr, &s_rows);
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
