@@ -10,7 +10,7 @@
 // roots and maxima therefore run on the integer pipes (mrmg_exact.cuh), two FP64
 // operations per coordinate are left.  1,000 x 10,000 distances: euclidean in 4
 // coordinates 394 -> 145 us (the 7 FP64 operations alone 142 us; all 19 were 390),
-// in 28 1,850 -> 1,125 us, max over agents 2,400 -> 1,070 us, max 1,700 -> 570 us.
+// in 28 1,850 -> 1,125 us, max over agents 2,400 -> 1,060 us, max 1,700 -> 585 us.
 #include "mrmg_internal.cuh"
 
 namespace mrmg {

@@ -1627,9 +1627,9 @@ constexpr int kNearWarps = 4;
 // bitmap, 56 us; 300 queries, whole call: 296 -> 228 us, with 11,600 results
 // each 4,910 -> 950 us.  4,000 queries on 40,000 nodes of one mode, 500 results
 // each: 147 us with a warp per query, 311 us with the look-ups per candidate and an
-// atomic per word, 175 us (the whole call 935, 962 and 827 us); a search per 32 words
+// atomic per word, 176 us (the whole call 935, 962 and 827 us); a search per 32 words
 // 238 us.  Six CTAs per SM where rows are read whole (8 spill: 204 us, and 68 instead
-// of 59 us for the 2,001 queries), eight where they are not (4,000 queries in 6-D 101
+// of 58 us for the 2,001 queries), eight where they are not (4,000 queries in 6-D 90
 // us, six 112).
 __host__ __device__ constexpr int near_ctas(bool rows) { return rows ? 6 : 8; }
 template <bool ROWS>

@@ -305,8 +305,8 @@ __device__ __forceinline__ void acc2(float& h, float& l, float v) {
 // Bound: issue slots (cost: 15 warp instructions per 32 pairs, 83 % of them
 // used) and, with the gradient, the FMA and special-function pipes together
 // (18 instructions; 17 and 16 of 27 cycles per 32 pairs).  512 paths of 256
-// waypoints, four arms, 50 boxes: cost 1.55 -> 1.24 ms, gradient 3.63 -> 2.76
-// ms, both 4.03 -> 3.06 ms, against one log2 and one reciprocal per pair, two
+// waypoints, four arms, 50 boxes: cost 1.55 -> 1.22 ms, gradient 3.63 -> 2.76
+// ms, both 4.03 -> 3.03 ms, against one log2 and one reciprocal per pair, two
 // spheres per packed instruction and 32-waypoint gradient CTAs (one per SM).
 // The sphere loop unrolled by 1, 2, 4 or 8: cost 1.31, 1.31, 1.24, 1.23 ms, the
 // gradient unchanged; the box loop by 1 or 2: gradient 2.80, 2.76 ms, both 3.09,
