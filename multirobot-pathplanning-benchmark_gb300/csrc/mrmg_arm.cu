@@ -818,7 +818,7 @@ __device__ uint8_t eval_config(const ArmDev& s, const ArmSmem& t, float2* wcs, f
     }
     if (__any_sync(MRMG_FULL, umin <= s.pair_eps)) {
       bool coll = false;
-      if (umin <= 0.f) {
+      if (umin <= s.pair_eps) {
         const int ga = pr & 0xffff, gb = pr >> 16;
         for (int w = 0; w < SPG; w++) {
           const float4 bq = wsph[gb * SPG + w];

@@ -1,7 +1,7 @@
 """Large batches in which the scan stops because its rows do not collide:
 verdicts equal the oracle's for free batches (everything left), for batches that
 turn free or begin free (some rows ended, some listed, the rest left), around
-the size from which batches are scanned, with three rows per warp (ten robots),
+the size from which batches are scanned, with two and three rows per warp (sixteen and ten robots),
 for edges with and without their endpoints, and for serving steps that are
 gathered in parts."""
 import copy
@@ -74,6 +74,30 @@ def test_three_rows_per_warp(gpu, oracle, keep):
     q2 = q + np.float32(0.03)
     got = s.is_edge_collision_free_batch(q, q2, 0.01).cpu().numpy()
     assert np.array_equal(got, o.edges_free(q, q2, 0.01))
+
+
+def test_two_rows_per_warp(gpu, oracle):
+    """Sixteen six-joint arms, four groups of four far from one another."""
+    col, scenes = pkg("collision"), pkg("scenes")
+    one = scenes.make_arm_scene(0, n_boxes=20, n_links=6)
+    s = copy.deepcopy(one)
+    n = len(one.sphere_radius)
+    s.q_offset, s.q_dim = np.arange(16, dtype=np.int32) * 6, 96
+    s.base_kind, s.n_links = np.zeros(16, np.int32), np.full(16, 6, np.int32)
+    s.base_pose, s.dh = np.tile(one.base_pose, (4, 1)), np.tile(one.dh, (4, 1, 1))
+    s.base_pose[:, 9] += 20.0 * (np.arange(16) // 4)
+    s.sphere_robot = (np.tile(one.sphere_robot, 4) + 4 * (np.arange(4 * n) // n)).astype(np.int32)
+    s.sphere_link, s.sphere_local = np.tile(one.sphere_link, 4), np.tile(one.sphere_local, (4, 1))
+    s.sphere_radius, s.limits = np.tile(one.sphere_radius, 4), np.stack([np.full(96, -np.pi), np.full(96, np.pi)])
+    for keep in (20, 0):                                   # cluttered for the first group, then free of boxes
+        sc = _moved(s, keep)
+        q = scenes.uniform_configs(sc, 20_000, seed=4, dtype=np.float32)   # scanned from 16,384 rows
+        o = oracle.OracleScene(sc)
+        got = col.Gb300Scene(sc).is_collision_free_batch(torch.from_numpy(q).cuda()).cpu().numpy()
+        assert np.array_equal(got, o.configs_free(q))
+        q2 = q + np.float32(0.1)
+        got = col.Gb300Scene(sc).is_edge_collision_free_batch(q, q2, 0.05).cpu().numpy()
+        assert np.array_equal(got, o.edges_free(q, q2, 0.05))
 
 
 @pytest.mark.parametrize("keep", [0, 1])
