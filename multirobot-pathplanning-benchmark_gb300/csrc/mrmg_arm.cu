@@ -511,8 +511,10 @@ __device__ uint8_t eval_config(const ArmDev& s, const ArmSmem& t, float2* wcs, f
       gb[u][1] = p[1] + (R[3] * lb.x + R[4] * lb.y + R[5] * lb.z);
       gb[u][2] = p[2] + (R[6] * lb.x + R[7] * lb.y + R[8] * lb.z);
       // a robot outside the call's mask: its bound never reaches a box or
-      // another group, so none of its spheres is tested
-      gb[u][3] = ((s.robot_mask >> (gi & 0xff)) & 1u) ? lb.w : -1.f;
+      // another group, and no box reaches its spheres (a lane that re-tests one
+      // of its groups goes over all of them), so none of them is tested
+      const bool in = (s.robot_mask >> (gi & 0xff)) & 1u;
+      gb[u][3] = in ? lb.w : -1.f;
 #pragma unroll
       for (int v = 0; v < SPG; v++) {
         const float4 l = t.sph[g * SPG + v];
@@ -521,7 +523,7 @@ __device__ uint8_t eval_config(const ArmDev& s, const ArmSmem& t, float2* wcs, f
         float y = p[1] + (R[3] * l.x + R[4] * l.y + R[5] * l.z);
         float z = p[2] + (R[6] * l.x + R[7] * l.y + R[8] * l.z);
         if (bd.y < 0.f) { x = kFar * (float)(g + 1); y = x; z = 0.f; }   // padding slot
-        if constexpr (BOXES != BOX_BLOCKS) { cx[u][v] = x; cy[u][v] = y; cz[u][v] = z; rh[u][v] = bd.y; }
+        if constexpr (BOXES != BOX_BLOCKS) { cx[u][v] = x; cy[u][v] = y; cz[u][v] = z; rh[u][v] = in ? bd.y : -1.f; }
         wsph[g * SPG + v] = make_float4(x, y, z, bd.z);
       }
     } else {
